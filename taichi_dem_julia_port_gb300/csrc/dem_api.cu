@@ -375,6 +375,9 @@ int prepare_scene(const DemConfigC* cfg, const DemParticlesIn* pin, double cell_
         c0 += p.wn[c] * p.dmin[c];
     }
     p.f_wc0 = (float)c0;
+    const double mul = cfg->particle_contact_radius_multiplier;
+    p.f_r0_hi = (float)(std::max(mul, 1.0) * (1.0 + 0x1p-20));
+    p.f_r0_lo = (float)(mul * (1.0 - 0x1p-20));
     return DEM_OK;
 }
 

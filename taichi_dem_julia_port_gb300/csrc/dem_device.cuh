@@ -55,10 +55,12 @@ __device__ __forceinline__ float reach32(float x, float y, float z, float r) {
     const float M = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
     return (r * (1.0f + 0x1p-19f) + M * 0x1p-19f) * (1.0f + 0x1p-21f);
 }
-__device__ __forceinline__ bool maybe_touching32(float4 a, float4 b, float extra = 0.0f) {
+// `mul` >= 1 scales both reaches (r₀ = mul·r rounded: the bond initialisation).
+__device__ __forceinline__ bool maybe_touching32(float4 a, float4 b, float extra = 0.0f,
+                                                 float mul = 1.0f) {
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     const float s = dx * dx + dy * dy + dz * dz;
-    const float B = a.w + b.w + extra;  // extra: the neighbour-list skin
+    const float B = (a.w + b.w) * mul + extra;  // extra: the neighbour-list skin
     return !(s * (1.0f - 0x1p-17f) > B * B);
 }
 
@@ -168,6 +170,52 @@ __device__ __forceinline__ bool product_finite(double a, double b) {
     const int ea = (int)((__double_as_longlong(a) >> 52) & 0x7ff);
     const int eb = (int)((__double_as_longlong(b) >> 52) & 0x7ff);
     return ea != 0x7ff && eb != 0x7ff && ea + eb <= 0x7fd + 1023;
+}
+
+// ---- cells ----------------------------------------------------------------------
+// ceil(num / cell) with num / cell rounded as IEEE division (src/utils.jl:1).
+// q = num·(1/cell) is within 2^-51·|q| of the rounded quotient; when no
+// integer lies within 2^-49·|q| of q, both have the same ceiling.  Otherwise
+// (rare: q must sit within ~10^-15 relative of an integer) the quotient is
+// computed by the correctly rounded division.
+__device__ __forceinline__ int32_t cell_index(double num, double cell, double inv_cell) {
+    const double q = num * inv_cell;
+    const double d = fabs(q) * 0x1p-49;
+    const double lo = ceil(q - d), hi = ceil(q + d);
+    if (lo == hi && lo > -2147483648.0 && lo < 2147483647.0) return (int32_t)lo;
+    return ceil_i32(__ddiv_rn(num, cell));
+}
+// Cell ijk (1-based) and octant bits of a position for a given cell size
+// (`cell` and the center comparison of `neighbors`, src/utils.jl:1-16), with
+// an FP32 screen.  num = pos - dmin is formed exactly as the
+// reference forms it; q' = fl32(num)·fl32(1/cell) lies within 4·2^-24·|q| of
+// the exact quotient q = num/cell, and the reference's center
+// dmin + (ijk - 1/2)·cell within 2^-51·(|dmin|/cell + |q| + 1) of its exact
+// value (in cell units).  When the fraction of q' keeps a distance of
+// m = 2^-20·(|q'| + |dmin|/cell + 1) from 0, 1/2 and 1, the exact ceiling and
+// the exact octant side follow from q' alone; otherwise (and for NaN or huge
+// values, which fail the test) the exact FP64 computation decides.  (The centre
+// test only matters where the side is wanted.)
+// One coordinate: the cell index and, with want_side, whether the coordinate
+// lies above the cell's centre (*above; not computed otherwise).
+__device__ __forceinline__ int cell_component(double x, double dmin, double cell,
+                                              double inv_cell, float inv_cell32, float dmin_cells,
+                                              bool want_side, bool* above) {
+    const double num = __dsub_rn(x, dmin);
+    const float q = d2f(num) * inv_cell32;
+    const float fl = floorf(q);
+    const float frac = q - fl;
+    const float m = (fabsf(q) + dmin_cells + 1.0f) * 0x1p-20f;
+    if (frac > m && frac < 1.0f - m && (!want_side || fabsf(frac - 0.5f) > m)) {
+        if (want_side) *above = frac > 0.5f;
+        return (int)fl + 1;
+    }
+    const int ijk = cell_index(num, cell, inv_cell);
+    if (want_side) {
+        const double ctr = __dadd_rn(dmin, __dmul_rn(__dsub_rn((double)ijk, 0.5), cell));
+        *above = x > ctr;
+    }
+    return ijk;
 }
 
 // ---- Morton / bucket ---------------------------------------------------------

@@ -95,6 +95,9 @@ struct SceneParams {
     double hdt2;            // dt²/2
     double tol2_lo, tol2_x4;  // tolerance²·(1 - 2^-30) and 4·tolerance² (contact frame)
     float f_wn[3], f_wc0;   // FP32 wall normal and n·domain_min - wall_distance (wall screen)
+    // r₀/r (particle_contact_radius_multiplier) rounded up, at least 1, and
+    // rounded down (the distance screens of the bond initialisation)
+    float f_r0_hi, f_r0_lo;
 };
 
 // Material, surface and wall tables of a scene built with dem_create_tables

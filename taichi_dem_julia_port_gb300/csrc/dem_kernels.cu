@@ -180,49 +180,7 @@ __global__ void __launch_bounds__(kScanBlock)
 }
 
 // ---------------------------------------------------------------------------
-// ceil(num / cell) with num / cell rounded as IEEE division (src/utils.jl:1).
-// q = num·(1/cell) is within 2^-51·|q| of the rounded quotient; when no
-// integer lies within 2^-49·|q| of q, both have the same ceiling.  Otherwise
-// (rare: q must sit within ~10^-15 relative of an integer) the quotient is
-// computed by the correctly rounded division.
-__device__ __forceinline__ int32_t cell_index(double num, double cell, double inv_cell) {
-    const double q = num * inv_cell;
-    const double d = fabs(q) * 0x1p-49;
-    const double lo = ceil(q - d), hi = ceil(q + d);
-    if (lo == hi && lo > -2147483648.0 && lo < 2147483647.0) return (int32_t)lo;
-    return ceil_i32(__ddiv_rn(num, cell));
-}
-// Cell ijk (1-based) and octant bits of a position for a given cell size
-// (`cell` and the center comparison of `neighbors`, src/utils.jl:1-16), with
-// an FP32 screen.  num = pos - dmin is formed exactly as the
-// reference forms it; q' = fl32(num)·fl32(1/cell) lies within 4·2^-24·|q| of
-// the exact quotient q = num/cell, and the reference's center
-// dmin + (ijk - 1/2)·cell within 2^-51·(|dmin|/cell + |q| + 1) of its exact
-// value (in cell units).  When the fraction of q' keeps a distance of
-// m = 2^-20·(|q'| + |dmin|/cell + 1) from 0, 1/2 and 1, the exact ceiling and
-// the exact octant side follow from q' alone; otherwise (and for NaN or huge
-// values, which fail the test) the exact FP64 computation decides.
-// One coordinate: the cell index and, with want_side, whether the coordinate
-// lies above the cell's centre (*above; not computed otherwise).
-__device__ __forceinline__ int cell_component(double x, double dmin, double cell,
-                                              double inv_cell, float inv_cell32, float dmin_cells,
-                                              bool want_side, bool* above) {
-    const double num = __dsub_rn(x, dmin);
-    const float q = d2f(num) * inv_cell32;
-    const float fl = floorf(q);
-    const float frac = q - fl;
-    const float m = (fabsf(q) + dmin_cells + 1.0f) * 0x1p-20f;
-    if (frac > m && frac < 1.0f - m && fabsf(frac - 0.5f) > m) {
-        if (want_side) *above = frac > 0.5f;
-        return (int)fl + 1;
-    }
-    const int ijk = cell_index(num, cell, inv_cell);
-    if (want_side) {
-        const double ctr = __dadd_rn(dmin, __dmul_rn(__dsub_rn((double)ijk, 0.5), cell));
-        *above = x > ctr;
-    }
-    return ijk;
-}
+// Cell ijk (1-based) and octant bits of a position, screened (cell_component).
 __device__ __forceinline__ int4 cell_of_screened(const double pos[3], const double dmin[3],
                                                  double cell, double inv_cell, float inv_cell32,
                                                  float dmin_cells) {
@@ -695,9 +653,14 @@ __device__ __forceinline__ void detect_group(const DemDev& d, const DemParams& p
                 const int vs = atomicAdd(&sh.nvl, 1);
                 if (vs < p.kvl) vl[vs] = j;
             }
-            // bond initialisation tests r₀ (no FP32 pre-filter); otherwise a
-            // touching pair is near and passes the pre-filter
-            if (!init && (!near || !maybe_touching32(P32, qq[u]))) continue;
+            // a touching pair is near and passes the FP32 pre-filter; bond
+            // initialisation tests r₀, with the pre-filter's reaches scaled
+            // to it.  (Without a pre-filter of its own the initialisation
+            // took the exact FP64 test of every candidate: 370 us for
+            // 110,592 spheres.)
+            if (init ? !maybe_touching32(P32, qq[u], 0.0f, S.f_r0_hi)
+                     : (!near || !maybe_touching32(P32, qq[u])))
+                continue;
             bool found = false;
             if (cached) {
                 for (int t = 0; t < e1 - e0 && !found; ++t) found = sh.row[t] == j;
@@ -706,11 +669,16 @@ __device__ __forceinline__ void detect_group(const DemDev& d, const DemParams& p
                     found = (o.cj[e2] == j) && (o.fl[e2] & kActive);
             }
             if (found) continue;
-            const double4_32a P = d.spos[k];
-            const double4_32a Q = d.spos[qi[u]];
-            const double ri = init ? d.r0[i] : P.w;
-            const double rj = init ? d.r0[j] : Q.w;
-            if (!touching_rn(P.x, P.y, P.z, Q.x, Q.y, Q.z, ri, rj)) continue;
+            // pairs that certainly touch need no FP64 test (surely_touching32
+            // with the FP32 radii, scaled down to r₀ for the initialisation)
+            const float lo = init ? S.f_r0_lo : 1.0f;
+            if (!surely_touching32(P32, d.rm32[i].z * lo, qq[u], d.rm32[j].z * lo)) {
+                const double4_32a P = d.spos[k];
+                const double4_32a Q = d.spos[qi[u]];
+                const double ri = init ? d.r0[i] : P.w;
+                const double rj = init ? d.r0[j] : Q.w;
+                if (!touching_rn(P.x, P.y, P.z, Q.x, Q.y, Q.z, ri, rj)) continue;
+            }
             const int slot = atomicAdd(&sh.nnew, 1);
             if (slot < p.kstash) stash[slot] = j;
         }
