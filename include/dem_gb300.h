@@ -532,7 +532,7 @@ int dem_debug_step_enumeration(DemHandle* h, int64_t* pairs, uint64_t* checksum)
  * hash_table_size <= 1,024, two above): its work is O(n + H) whatever the
  * number of particles per bucket.
  *
- * The temporary memory is one 12.6 MB array inside the library, reserved on
+ * The temporary memory is one 9.4 MB array inside the library, reserved on
  * every GPU that loads it until the process exits, so n and hash_table_size
  * are each limited to 1,048,576 (larger values return DEM_ERR_CAPACITY
  * before any work is queued).  The first call on a device looks up that

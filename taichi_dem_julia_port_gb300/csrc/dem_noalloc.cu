@@ -18,9 +18,15 @@
 // occupancy: one bucket holding every particle costs the same as many small
 // ones.
 //
+// Three launches per pass, none of which waits on another block: the digit
+// counts of every chunk of 4,096 particles (the first pass counts while it
+// hashes), each digit's running sum over the chunks, and the scatter, which
+// scans the 1,024 digit totals itself.
+//
 // Limits: n <= 1,048,576 particles and hash_table_size <= 1,048,576 buckets;
-// the array is 12.6 MB (the first pass's keys and indices, the per-block
-// digit counts, and the tile sums of their scan).
+// the array is 9.4 MB (the first pass's keys and indices, the per-chunk
+// digit counts, and the digit totals).
+#include <cmath>
 #include <mutex>
 
 #include "dem_device.cuh"
@@ -30,25 +36,24 @@ namespace {
 
 constexpr long long kMaxN = 1 << 20;
 constexpr long long kMaxH = 1 << 20;
-constexpr int kBlock = 256;
-constexpr int kItems = 4;
+constexpr int kBlock = 512;
+constexpr int kWarps = kBlock / 32;
+constexpr int kItems = 8;
 constexpr int kChunk = kBlock * kItems;  // particles per block of a radix pass
 constexpr int kDigitBits = 10;
 constexpr int kBins = 1 << kDigitBits;
 constexpr long long kMaxBlocks = kMaxN / kChunk;
 constexpr long long kHistWords = kBins * kMaxBlocks;
-constexpr int kTile = 2048;  // counts per tile of the digit-count scan
-constexpr int kMaxTiles = (int)((kHistWords + kTile - 1) / kTile);
 constexpr size_t kKeysOff = 0;
 constexpr size_t kValsOff = kKeysOff + kMaxN;
 constexpr size_t kHistOff = kValsOff + kMaxN;
-constexpr size_t kTilesOff = kHistOff + kHistWords;
-constexpr size_t kWords = kTilesOff + kMaxTiles;
+constexpr size_t kTotalsOff = kHistOff + kHistWords;
+constexpr size_t kWords = kTotalsOff + kBins;
 constexpr int kMaxDevices = 64;
 
 // The scratch: the first pass's output keys (0-based buckets) and particle
-// indices, the digit counts of every block (digit-major, scanned in place
-// into each block's first slot per digit) and the per-tile sums of that scan.
+// indices, the digit counts of every chunk (digit-major, scanned in place over
+// the chunks) and the digits' totals.
 // Every word a call reads is written earlier in the same call, so nothing
 // needs clearing between calls.  Host code must not take this name as a
 // device address; it uses the address from cudaGetSymbolAddress (see
@@ -57,7 +62,9 @@ static __device__ __align__(256) uint32_t g_scratch[kWords];
 
 struct Geometry {
     double dmin[3];
-    double cell;
+    double cell, inv_cell;
+    float inv_cell32, dmin_cells;  // the FP32 screen of the cell (cell_component)
+    int screen;                    // 0: the cell size is beyond the screen's range
     uint32_t H;
     uint32_t mask;
 };
@@ -66,41 +73,92 @@ __device__ __forceinline__ uint32_t na_bucket(int x, int y, int z, const Geometr
     const uint32_t m = dem::morton1(x, y, z);
     return g.mask ? (m & g.mask) : (m % g.H);
 }
-
-// cell + hashcode (src/utils.jl:1-2): the reference's 1-based bucket
-__global__ void k_na_hash(const double* __restrict__ px, const double* __restrict__ py,
-                          const double* __restrict__ pz, int n, Geometry g, uint32_t* bucket_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double pos[3] = {px[i], py[i], pz[i]};
-    int ijk[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        ijk[c] = dem::ceil_i32(__ddiv_rn(__dsub_rn(pos[c], g.dmin[c]), g.cell));
-    bucket_out[i] = na_bucket(ijk[0], ijk[1], ijk[2], g) + 1u;
+__device__ __forceinline__ int na_cell(double x, int c, const Geometry& g) {
+    if (g.screen)
+        return dem::cell_component(x, g.dmin[c], g.cell, g.inv_cell, g.inv_cell32, g.dmin_cells,
+                                   false, nullptr);
+    return dem::ceil_i32(__ddiv_rn(__dsub_rn(x, g.dmin[c]), g.cell));
 }
 
-// Digit counts of one block's kChunk keys (key = in[k] - bias), written
-// digit-major: hist[digit * nblk + block].
-__global__ void k_na_digit_count(const uint32_t* __restrict__ keys, uint32_t bias, int n,
-                                 int shift, int nblk, uint32_t* __restrict__ hist) {
+// cell + hashcode (src/utils.jl:1-2) of one chunk, the reference's 1-based
+// buckets, with the first pass's digit counts (digit-major: hist[digit · nblk
+// + chunk]).  The three quotients per particle were the whole sort's largest
+// cost as FP64 divisions (1,000,000 particles: 74 us of 166 us; GB300 retires
+// one FP64 warp-instruction per 64 cycles and SM sub-partition); the FP32
+// screen of cell_component decides all but the cells' edges (9 us with the
+// counts).
+__global__ void __launch_bounds__(kBlock)
+    k_na_hash(const double* __restrict__ px, const double* __restrict__ py,
+              const double* __restrict__ pz, int n, Geometry g, int nblk, uint32_t* bucket_out,
+              uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kBins];
     for (int b = threadIdx.x; b < kBins; b += kBlock) h[b] = 0u;
     __syncthreads();
-    const long long base = (long long)blockIdx.x * kChunk;
+    const int base = blockIdx.x * kChunk + (int)threadIdx.x;
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-        const long long k = base + q * kBlock + threadIdx.x;
-        if (k < n) atomicAdd(&h[((keys[k] - bias) >> shift) & (kBins - 1)], 1u);
+        const int i = base + q * kBlock;
+        if (i < n) {
+            const int cx = na_cell(px[i], 0, g), cy = na_cell(py[i], 1, g), cz = na_cell(pz[i], 2, g);
+            const uint32_t b = na_bucket(cx, cy, cz, g);
+            bucket_out[i] = b + 1u;
+            atomicAdd(&h[b & (kBins - 1)], 1u);
+        }
     }
     __syncthreads();
     for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)b * nblk + blockIdx.x] = h[b];
 }
 
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t warp_sums[kBlock / 32];
+// Digit counts of one chunk's keys for a later pass.
+__global__ void __launch_bounds__(kBlock)
+    k_na_digit_count(const uint32_t* __restrict__ keys, int n, int shift, int nblk,
+                     uint32_t* __restrict__ hist) {
+    __shared__ uint32_t h[kBins];
+    for (int b = threadIdx.x; b < kBins; b += kBlock) h[b] = 0u;
+    __syncthreads();
+    const int base = blockIdx.x * kChunk + (int)threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int k = base + q * kBlock;
+        // equal digits of a warp are counted once: the keys come sorted by
+        // their low digit, so many neighbours share the high one
+        const uint32_t d = k < n ? (keys[k] >> shift) & (kBins - 1) : (uint32_t)kBins;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        if (k < n && (unsigned)(__ffs(peers) - 1) == (threadIdx.x & 31u))
+            atomicAdd(&h[d], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)b * nblk + blockIdx.x] = h[b];
+}
+
+// One warp per digit: its counts over the chunks become running sums, in
+// place, and its total.
+__global__ void k_na_digit_rows(uint32_t* hist, int nblk, uint32_t* totals) {
+    const unsigned lane = threadIdx.x & 31u;
+    const int d = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    if (d >= kBins) return;
+    uint32_t* row = hist + (size_t)d * nblk;
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < nblk; b0 += 32) {
+        const int b = b0 + (int)lane;
+        const uint32_t v = b < nblk ? row[b] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (unsigned)o) x += y;
+        }
+        if (b < nblk) row[b] = carry + x - v;
+        carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) totals[d] = carry;
+}
+
+// Exclusive scan of kBins values, two per thread (v: this thread's pair).
+static_assert(kBins == 2 * kBlock, "two digits per thread");
+__device__ __forceinline__ uint2 block_scan_bins(uint2 v, uint32_t* warp_sums) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t x = v;
+    uint32_t x = v.x + v.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -108,111 +166,105 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
     }
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kBlock / 32 ? warp_sums[lane] : 0u;
+    uint32_t pre = 0;
+    for (unsigned w = 0; w < warp; ++w) pre += warp_sums[w];
+    __syncthreads();
+    const uint32_t e = pre + x - (v.x + v.y);
+    return make_uint2(e, e + v.x);
+}
+
+// Stable scatter of one chunk's (key, index) pairs by the digit at `shift`.
+// Each warp ranks its own 256 consecutive elements, 32 per round
+// (__match_any_sync groups equal digits), in a digit table of its own; the
+// tables' running sums over the warps, in order, then place every element
+// after the earlier elements of its digit, so the order inside a digit is the
+// input order.  The chunk is put in digit order in shared memory and written
+// from there, runs of equal digits together.  (With one warp ranking 1,024
+// elements and every element written from its own thread the two scatters of
+// 1,000,000 particles took 26 and 13 us.)  idx_in == nullptr: the indices
+// are the positions.
+struct ScatterShared {
+    uint16_t cnt[kWarps][kBins];
+    uint32_t key[kChunk], idx[kChunk];
+    uint32_t dst[kBins];  // a digit's output position minus its position in the chunk
+    uint32_t warp_sums[kWarps];
+};
+__global__ void __launch_bounds__(kBlock)
+    k_na_digit_scatter(const uint32_t* __restrict__ keys, uint32_t bias,
+                       const uint32_t* __restrict__ idx_in, int n, int shift, int nblk,
+                       const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals,
+                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ idx_out) {
+    extern __shared__ unsigned char raw[];
+    ScatterShared& sh = *reinterpret_cast<ScatterShared*>(raw);
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const int base = blockIdx.x * kChunk;
+    const int m = min(kChunk, n - base);
+    uint32_t key[kItems], idx[kItems];
+    const int e0 = (int)warp * (kItems * 32) + (int)lane;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= (unsigned)o) w += y;
-        }
-        if (lane < kBlock / 32) warp_sums[lane] = w;
+    for (int r = 0; r < kItems; ++r) {
+        const int e = e0 + r * 32;
+        key[r] = e < m ? keys[base + e] - bias : 0u;
+        idx[r] = e < m ? (idx_in ? idx_in[base + e] : (uint32_t)(base + e)) : 0u;
     }
+    const int d0 = 2 * (int)threadIdx.x;
+    const uint2 tot = make_uint2(totals[d0], totals[d0 + 1]);
+    const uint2 row = make_uint2(hist[(size_t)d0 * nblk + blockIdx.x],
+                                 hist[(size_t)(d0 + 1) * nblk + blockIdx.x]);
+    uint32_t* zero = reinterpret_cast<uint32_t*>(&sh.cnt[0][0]);
+    for (int b = threadIdx.x; b < kWarps * kBins / 2; b += kBlock) zero[b] = 0u;
     __syncthreads();
-    *total = warp_sums[kBlock / 32 - 1];
-    const uint32_t r = (warp ? warp_sums[warp - 1] : 0u) + x - v;
-    __syncthreads();
-    return r;
-}
-
-// Exclusive scan of the digit counts, in place, in three passes without any
-// inter-block waiting: tile sums, one-block scan of the sums, apply.
-__global__ void k_na_tile_sums(const uint32_t* v, long long m, uint32_t* tiles) {
-    const long long base = (long long)blockIdx.x * kTile + threadIdx.x * (kTile / kBlock);
-    uint32_t s = 0;
-    for (int k = 0; k < kTile / kBlock; ++k)
-        if (base + k < m) s += v[base + k];
-    uint32_t total;
-    block_excl_scan(s, &total);
-    if (threadIdx.x == 0) tiles[blockIdx.x] = total;
-}
-
-__global__ void k_na_scan_tiles(uint32_t* tiles, int ntiles) {
-    uint32_t carry = 0;
-    for (int base = 0; base < ntiles; base += kBlock) {
-        const int t = base + threadIdx.x;
-        const uint32_t v = t < ntiles ? tiles[t] : 0u;
-        uint32_t total;
-        const uint32_t e = block_excl_scan(v, &total);
-        if (t < ntiles) tiles[t] = carry + e;
-        carry += total;
-    }
-}
-
-__global__ void k_na_apply(uint32_t* v, long long m, const uint32_t* tiles) {
-    const long long base = (long long)blockIdx.x * kTile + threadIdx.x * (kTile / kBlock);
-    uint32_t x[kTile / kBlock];
-    uint32_t s = 0;
-    for (int k = 0; k < kTile / kBlock; ++k) {
-        x[k] = base + k < m ? v[base + k] : 0u;
-        s += x[k];
-    }
-    uint32_t total;
-    uint32_t run = tiles[blockIdx.x] + block_excl_scan(s, &total);
-    for (int k = 0; k < kTile / kBlock; ++k) {
-        if (base + k < m) v[base + k] = run;
-        run += x[k];
-    }
-}
-
-// Stable scatter of one block's kChunk (key, index) pairs by the digit at
-// `shift`: an element's place is its block's first slot for that digit plus
-// the number of elements of the block before it with the same digit.  The
-// ranks are counted in element order by one warp, 32 elements per round
-// (__match_any_sync groups equal digits), so the order inside a digit is
-// the input order.  idx_in == nullptr: the indices are the positions.
-__global__ void k_na_digit_scatter(const uint32_t* __restrict__ keys, uint32_t bias,
-                                   const uint32_t* __restrict__ idx_in, int n, int shift, int nblk,
-                                   const uint32_t* __restrict__ first,
-                                   uint32_t* __restrict__ keys_out, uint32_t* __restrict__ idx_out) {
-    __shared__ uint32_t s_key[kChunk], s_idx[kChunk], s_rank[kChunk], s_cnt[kBins];
-    const long long base = (long long)blockIdx.x * kChunk;
-    const int m = (int)min((long long)kChunk, (long long)n - base);
-    for (int b = threadIdx.x; b < kBins; b += kBlock) s_cnt[b] = 0u;
+    uint32_t rank[kItems];  // within the warp's elements of the same digit
 #pragma unroll
-    for (int q = 0; q < kItems; ++q) {
-        const int e = q * kBlock + threadIdx.x;
-        if (e < m) {
-            s_key[e] = keys[base + e] - bias;
-            s_idx[e] = idx_in ? idx_in[base + e] : (uint32_t)(base + e);
-        }
+    for (int r = 0; r < kItems; ++r) {
+        const bool valid = e0 + r * 32 < m;
+        const uint32_t d = valid ? (key[r] >> shift) & (kBins - 1) : (uint32_t)kBins;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        uint32_t before = 0;
+        if (valid) before = sh.cnt[warp][d];
+        __syncwarp();
+        rank[r] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        if (valid && (unsigned)(__ffs(peers) - 1) == lane)
+            sh.cnt[warp][d] = (uint16_t)(before + (uint32_t)__popc(peers));
+        __syncwarp();
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const unsigned lane = threadIdx.x;
-        for (int r = 0; r < kChunk / 32; ++r) {
-            const int e = r * 32 + (int)lane;
-            const bool valid = e < m;
-            const uint32_t d = valid ? (s_key[e] >> shift) & (kBins - 1) : (uint32_t)kBins;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
-            uint32_t before = 0;
-            if (valid) before = s_cnt[d];
-            __syncwarp();
-            if (valid) {
-                s_rank[e] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-                if ((unsigned)(__ffs(peers) - 1) == lane) s_cnt[d] = before + (uint32_t)__popc(peers);
-            }
-            __syncwarp();
+    // the warps' counts of this thread's two digits become running sums
+    uint2 c = make_uint2(0u, 0u);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t u = reinterpret_cast<uint32_t*>(sh.cnt[w])[threadIdx.x];
+        reinterpret_cast<uint32_t*>(sh.cnt[w])[threadIdx.x] = c.x | (c.y << 16);
+        c.x += u & 0xffffu;
+        c.y += u >> 16;
+    }
+    const uint2 local = block_scan_bins(c, sh.warp_sums);    // first place in the chunk
+    const uint2 global = block_scan_bins(tot, sh.warp_sums);  // first place of the digit
+    // the chunk's first place of each digit joins the warps' running sums
+    // (at most kChunk - 1, so 16 bits hold it)
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w)
+        reinterpret_cast<uint32_t*>(sh.cnt[w])[threadIdx.x] += local.x | (local.y << 16);
+    sh.dst[d0] = global.x + row.x - local.x;
+    sh.dst[d0 + 1] = global.y + row.y - local.y;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+        if (e0 + r * 32 < m) {
+            const uint32_t at = sh.cnt[warp][(key[r] >> shift) & (kBins - 1)] + rank[r];
+            sh.key[at] = key[r];
+            sh.idx[at] = idx[r];
         }
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-        const int e = q * kBlock + threadIdx.x;
+        const int e = q * kBlock + (int)threadIdx.x;
         if (e < m) {
-            const uint32_t d = (s_key[e] >> shift) & (kBins - 1);
-            const uint32_t dst = first[(size_t)d * nblk + blockIdx.x] + s_rank[e];
-            idx_out[dst] = s_idx[e];
-            if (keys_out) keys_out[dst] = s_key[e];
+            const uint32_t k = sh.key[e];
+            const uint32_t dst = sh.dst[(k >> shift) & (kBins - 1)] + (uint32_t)e;
+            idx_out[dst] = sh.idx[e];
+            if (keys_out) keys_out[dst] = k;
         }
     }
 }
@@ -230,6 +282,12 @@ int scratch_on(int device, uint32_t** out) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_scratch) != cudaSuccess || !p) {
             cudaGetLastError();  // this call's own failure
+            return DEM_ERR_CUDA;
+        }
+        // the scatter's shared memory is above the default limit
+        if (cudaFuncSetAttribute(k_na_digit_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(ScatterShared)) != cudaSuccess) {
+            cudaGetLastError();
             return DEM_ERR_CUDA;
         }
         g_scratch_ptr[device] = static_cast<uint32_t*>(p);
@@ -264,37 +322,41 @@ extern "C" int dem_bucket_sort_noalloc(const double* px, const double* py, const
     uint32_t* keys_tmp = scratch + kKeysOff;
     uint32_t* idx_tmp = scratch + kValsOff;
     uint32_t* hist = scratch + kHistOff;
-    uint32_t* tiles = scratch + kTilesOff;
+    uint32_t* totals = scratch + kTotalsOff;
     Geometry g;
-    for (int c = 0; c < 3; ++c) g.dmin[c] = domain_min[c];  // host memory
+    double dm = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        g.dmin[c] = domain_min[c];  // host memory
+        dm = std::fmax(dm, std::fabs(g.dmin[c]));
+    }
     g.cell = cell_size;
+    g.inv_cell = 1.0 / cell_size;
+    g.inv_cell32 = (float)g.inv_cell;
+    g.dmin_cells = (float)(dm * g.inv_cell * 1.001);
+    g.screen = cell_size > 0x1p-100 && cell_size < 0x1p100;
     g.H = (uint32_t)hash_table_size;
     g.mask = (g.H & (g.H - 1)) == 0 ? g.H - 1 : 0u;
     const int nn = (int)n;
-    k_na_hash<<<(nn + kBlock - 1) / kBlock, kBlock, 0, s>>>(px, py, pz, nn, g, bucket);
-    if (!launched()) return DEM_ERR_CUDA;
     // buckets are 0 .. H-1 < 2^20: one 10-bit pass for H <= 1,024, else two
     const int passes = hash_table_size <= kBins ? 1 : 2;
     const int nblk = (nn + kChunk - 1) / kChunk;
-    const long long m = (long long)kBins * nblk;
-    const int ntiles = (int)((m + kTile - 1) / kTile);
+    k_na_hash<<<nblk, kBlock, 0, s>>>(px, py, pz, nn, g, nblk, bucket, hist);
+    if (!launched()) return DEM_ERR_CUDA;
     for (int pass = 0; pass < passes; ++pass) {
         const int shift = pass * kDigitBits;
         const bool last = pass == passes - 1;
         const uint32_t* kin = pass == 0 ? bucket : keys_tmp;
         const uint32_t bias = pass == 0 ? 1u : 0u;  // the outputs' buckets are 1-based
         const uint32_t* iin = pass == 0 ? nullptr : idx_tmp;
-        k_na_digit_count<<<nblk, kBlock, 0, s>>>(kin, bias, nn, shift, nblk, hist);
+        if (pass > 0) {
+            k_na_digit_count<<<nblk, kBlock, 0, s>>>(kin, nn, shift, nblk, hist);
+            if (!launched()) return DEM_ERR_CUDA;
+        }
+        k_na_digit_rows<<<kBins / 8, 256, 0, s>>>(hist, nblk, totals);
         if (!launched()) return DEM_ERR_CUDA;
-        k_na_tile_sums<<<ntiles, kBlock, 0, s>>>(hist, m, tiles);
-        if (!launched()) return DEM_ERR_CUDA;
-        k_na_scan_tiles<<<1, kBlock, 0, s>>>(tiles, ntiles);
-        if (!launched()) return DEM_ERR_CUDA;
-        k_na_apply<<<ntiles, kBlock, 0, s>>>(hist, m, tiles);
-        if (!launched()) return DEM_ERR_CUDA;
-        k_na_digit_scatter<<<nblk, kBlock, 0, s>>>(kin, bias, iin, nn, shift, nblk, hist,
-                                                   last ? nullptr : keys_tmp,
-                                                   last ? sorted : idx_tmp);
+        k_na_digit_scatter<<<nblk, kBlock, sizeof(ScatterShared), s>>>(
+            kin, bias, iin, nn, shift, nblk, hist, totals, last ? nullptr : keys_tmp,
+            last ? sorted : idx_tmp);
         if (!launched()) return DEM_ERR_CUDA;
     }
     return DEM_OK;
