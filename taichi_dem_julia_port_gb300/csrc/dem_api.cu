@@ -367,6 +367,8 @@ int prepare_scene(const DemConfigC* cfg, const DemParticlesIn* pin, double cell_
     p.f_tol4 = (float)(4.0 * p.tol * p.tol);
     p.f_tol1 = (float)(p.tol * p.tol * (1.0 - 0x1p-10));
     p.hdt2 = 0.5 * (p.dt * p.dt);
+    p.dt6 = 6.0 * p.dt;
+    p.f_tol8 = (float)(8.0 * p.tol * p.tol);
     p.tol2_lo = p.tol * p.tol * (1.0 - 0x1p-30);
     p.tol2_x4 = 4.0 * p.tol * p.tol;
     double c0 = -p.wd;
@@ -431,7 +433,8 @@ struct DemHandle {
     int ntiles_cells = 0;
     LaunchShape shape{};
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};  // one step, per contact-buffer parity
+    cudaGraphExec_t run[2] = {nullptr, nullptr};   // kRunSteps steps inside a longer call
     int graph_precision = -1;
     int enc = DEM_FP64;  // encoding of 𝐅ᵢ, 𝛕ᵢ, 𝛕ⱼ in the current contact buffer
     std::vector<void*> allocs;
@@ -440,19 +443,7 @@ struct DemHandle {
     int64_t xfer_n = 0;        // doubles
     int* err_host = nullptr;   // page-locked copy of the device error word
     int* err_dev = nullptr;    // its device address
-    // the exchanged step of dem_step_exchange as one graph per contact-buffer
-    // parity, for one set of caller buffers (key: their device addresses):
-    // the position upload, then the contact update while a second stream
-    // uploads velocities and spins, then forces and the integration (which
-    // reads orientations and wall shear from the caller and writes the state
-    // back into the caller's buffers)
-    static constexpr int kXKey = 14;
-    struct XGraph {
-        cudaGraphExec_t exec = nullptr;
-        const void* key[kXKey] = {};
-    } xg[2];
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    bool steps_ok = false;  // the steps' single launch (k_steps) fits the device
     // dem_step_profiled: the step's graph with an event before, between and
     // after its three kernels, per contact-buffer parity
     cudaGraphExec_t pg[2] = {nullptr, nullptr};
@@ -539,6 +530,8 @@ int allocate(DemHandle* h) {
         TRY(dalloc(h, &d.row_start[b], n));
         TRY(dalloc(h, &d.row_len[b], n));
     }
+    TRY(dalloc(h, &d.qmask, (n + 31) / 32));
+    CU(cudaMemsetAsync(d.qmask, 0xff, (n + 31) / 32 * sizeof(uint32_t), h->stream));
     TRY(dalloc(h, &d.stash, n * (size_t)h->p.kstash));
     TRY(dalloc(h, &d.keep, cap));
     TRY(dalloc(h, &d.tlist, cap));
@@ -571,15 +564,10 @@ void drop_graphs(DemHandle* h);
 
 void free_all(DemHandle* h) {
     drop_graphs(h);
-    if (h->fork_ev) cudaEventDestroy(h->fork_ev);
-    if (h->join_ev) cudaEventDestroy(h->join_ev);
     for (cudaEvent_t& e : h->pev) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
     }
-    if (h->side) cudaStreamDestroy(h->side);
-    h->fork_ev = h->join_ev = nullptr;
-    h->side = nullptr;
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -601,11 +589,16 @@ void free_all(DemHandle* h) {
 // Default launch shape: blocks of at most 256 threads, small enough that a
 // single scene's particles give every SM at least four blocks (a
 // 17,576-sphere scene in 256-thread blocks would leave half the SMs idle),
-// and its expected ~3 contacts per particle at least eight: the hardware
-// spreads many one-warp blocks more evenly over the SMs than fewer larger
-// ones (measured on that scene's 50,700 bonds: 32-thread force blocks
-// 46.9 us per step, 64-thread 48.0 us).  Arenas start at 256; the autotuner
-// refines.
+// and its expected ~3 contacts per particle at least eight.  Force blocks have
+// at most 64 threads: the FP64 force pass of a 103,823-sphere body takes
+// 82 us in blocks of 256, 70 us in blocks of 64, because the hardware spreads
+// small blocks more evenly over the SMs (the FP32 pass does not change).  An
+// arena's integrator, whose scenes differ in work per particle, takes blocks
+// of 128 (256 scenes: 151 -> 143 us).  Both kinds of handles default to the
+// FP32 force kernel with the register budget for four 256-thread blocks per
+// SM (64 registers, a few bytes of spills): with the compiler's choice (three
+// blocks) the 2,000,000-sphere bed's force pass measured 180 us instead of
+// 156 us, the 256 scenes' 186 us instead of 174 us.
 LaunchShape default_shape(const DemHandle* h) {
     auto block_for = [&](int64_t units, int per_sm) {
         int b = 256;
@@ -613,14 +606,9 @@ LaunchShape default_shape(const DemHandle* h) {
         return b;
     };
     const int64_t n = h->multi ? INT64_MAX / 16 : h->n_cap;
-    const int ib = block_for(n, 4), fb = block_for(3 * n, 8), cb = block_for(4 * n, 4);
-    // a single scene's FP32 force kernel with the register budget for four
-    // 256-thread blocks per SM (64 registers, a few bytes of spills): with
-    // the compiler's choice (74 registers, three blocks) the 2,000,000-sphere
-    // bed's force pass measured 215 us instead of 171 us.  The arena's keeps
-    // the compiler's choice (the autotuner tries both).
-    return LaunchShape{fb, h->sm_count * 16, cb, h->sm_count * 16, ib, 4, h->multi ? 0 : 4,
-                       0, 0, 0};
+    const int ib = h->multi ? 128 : block_for(n, 4), fb = std::min(block_for(3 * n, 8), 64);
+    const int cb = block_for(4 * n, 4);
+    return LaunchShape{fb, h->sm_count * 32, cb, h->sm_count * 16, ib, 4, 4, 0, 0, 0};
 }
 
 int init_handle(DemHandle* h) {
@@ -632,8 +620,11 @@ int init_handle(DemHandle* h) {
     h->shape = default_shape(h);
     h->p.dep = h->shape.dependent_launch;
     h->p.list_lanes = h->shape.list_lanes;
+    h->p.report = 1;
     return DEM_OK;
 }
+
+int mark_turned(DemHandle* h, int64_t p0, int64_t n);
 
 // Uploads a scene's particle arrays into slots [p0, p0 + n) and resets their
 // dynamic state (ω = 0, q = 1, wall shear = 0, last forces = 0).
@@ -665,6 +656,7 @@ int upload_scene(DemHandle* h, const SceneArrays& A, int64_t p0) {
     for (const auto& c : cols) CU(up(c.first, *c.second));
     k_scene_columns<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(d, p0, (int64_t)n);
     CU(cudaGetLastError());
+    TRY(mark_turned(h, p0, (int64_t)n));
     for (double* z : {d.wx, d.wy, d.wz, d.qx, d.qy, d.qz, d.wsx, d.wsy, d.wsz, d.fx, d.fy, d.fz,
                       d.tx, d.ty, d.tz})
         CU(cudaMemsetAsync(z + p0, 0, n * sizeof(double), h->stream));
@@ -713,6 +705,9 @@ int build_tables(const DemConfigC& cfg, const DemTables& t, int64_t n, MatTables
             P.sc = S.bond_compressive_strength;
             P.st = S.bond_tensile_strength;
             P.ss = S.bond_shear_strength;
+            P.f_sc = (float)P.sc;
+            P.f_st = (float)P.st;
+            P.f_ss = (float)P.ss;
         }
     for (int w = 0; w < M.nwall; ++w) {
         const DemWall& W = t.walls[w];
@@ -784,19 +779,32 @@ int flag_search(DemHandle* h, int s) {
     return DEM_OK;
 }
 
-void record_step(DemHandle* h, int cur) {
+// steps per graph inside a longer dem_step call of a single scene: a graph
+// launch costs about 2 us more than an edge inside a graph (even: the parity
+// of the contact buffers comes out as it went in)
+constexpr int kRunSteps = 8;
+void record_step(DemHandle* h, int cur, bool report) {
+    DemParams p = h->p;
+    p.report = report ? 1 : 0;
     const int nxt = cur ^ 1;
-    launch_search(h->d, h->p, cur, false, h->multi, false, h->shape, h->stream);
-    launch_force(h->d, h->p, nxt, h->multi, h->shape, h->stream);
-    launch_integrate(h->d, h->p, cur, h->multi, h->shape, h->stream);
+    launch_search(h->d, p, cur, false, h->multi, false, h->shape, h->stream);
+    launch_force(h->d, p, nxt, h->multi, h->shape, h->stream);
+    launch_integrate(h->d, p, cur, h->multi, h->shape, h->stream);
+}
+// Every quaternion bit of slots [p0, p0 + n) set (DemDev::qmask).
+int mark_turned(DemHandle* h, int64_t p0, int64_t n) {
+    if (n <= 0) return DEM_OK;
+    const size_t w0 = (size_t)p0 / 32, w1 = (size_t)(p0 + n - 1) / 32;
+    CU(cudaMemsetAsync(h->d.qmask + w0, 0xff, (w1 - w0 + 1) * sizeof(uint32_t), h->stream));
+    return DEM_OK;
 }
 
 void drop_graphs(DemHandle* h) {
     for (int b = 0; b < 2; ++b) {
         if (h->exec[b]) cudaGraphExecDestroy(h->exec[b]);
         h->exec[b] = nullptr;
-        if (h->xg[b].exec) cudaGraphExecDestroy(h->xg[b].exec);
-        h->xg[b].exec = nullptr;
+        if (h->run[b]) cudaGraphExecDestroy(h->run[b]);
+        h->run[b] = nullptr;
         if (h->pg[b]) cudaGraphExecDestroy(h->pg[b]);
         h->pg[b] = nullptr;
     }
@@ -817,6 +825,7 @@ int update_bounds(DemHandle* h) {
     const int n = (int)hi(h->pfree, h->n_cap, 32768);
     const uint32_t T = (uint32_t)hi(h->tfree, h->t_cap, 65536);
     if (n == h->p.n && T == h->p.T) return DEM_OK;
+    TRY(mark_turned(h, 0, h->n_cap));  // the integrator's layout may change with n
     CU(cudaStreamSynchronize(h->stream));
     h->p.n = n;
     h->p.T = T;
@@ -833,23 +842,51 @@ int update_bounds(DemHandle* h) {
     return DEM_OK;
 }
 
+// A graph of `steps` steps from contact-buffer parity `cur`.
+int capture_steps(DemHandle* h, int cur, int steps, bool report, cudaGraphExec_t* exec) {
+    cudaGraph_t g = nullptr;
+    CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    for (int s = 0; s < steps; ++s) record_step(h, (cur + s) & 1, report);
+    cudaError_t e = cudaGetLastError();
+    const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
+    if (e == cudaSuccess) e = ec;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+    if (g) cudaGraphDestroy(g);
+    CU(e);
+    return DEM_OK;
+}
+
 int build_graphs(DemHandle* h) {
     if (h->graph_precision == h->p.precision && h->exec[0]) return DEM_OK;
     drop_graphs(h);
-    for (int b = 0; b < 2; ++b) {
-        if (h->exec[b]) {
-            cudaGraphExecDestroy(h->exec[b]);
-            h->exec[b] = nullptr;
-        }
-        cudaGraph_t g = nullptr;
-        CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        record_step(h, b);
-        CU(cudaStreamEndCapture(h->stream, &g));
-        cudaError_t e = cudaGraphInstantiate(&h->exec[b], g, 0);
-        cudaGraphDestroy(g);
-        CU(e);
-    }
+    for (int b = 0; b < 2; ++b) TRY(capture_steps(h, b, 1, true, &h->exec[b]));
     h->graph_precision = h->p.precision;
+    return DEM_OK;
+}
+
+// Steps of single scenes of at most this many particles per SM run as one
+// cooperative launch (k_steps) unless the launch shape asks for a layout of
+// the separate kernels.
+constexpr int64_t kStepsPerSm = 256;
+bool steps_fit(const DemHandle* h) {
+    return h->steps_ok && h->p.n <= kStepsPerSm * h->sm_count && h->shape.list_lanes == 0 &&
+           h->shape.integrate_lanes == 0 && h->shape.dependent_launch == 0;
+}
+// nsteps steps by k_steps, at most kStepsPerLaunch in each launch (other
+// streams' work gets its turn between launches); the first reads io's input,
+// the last writes its output.
+constexpr int64_t kStepsPerLaunch = 64;
+int run_steps(DemHandle* h, int64_t nsteps, const StepIO& io) {
+    for (int64_t done = 0; done < nsteps;) {
+        const int k = (int)std::min<int64_t>(nsteps - done, kStepsPerLaunch);
+        StepIO part = io;
+        part.has_in = done == 0 ? io.has_in : 0;
+        part.has_out = done + k == nsteps ? io.has_out : 0;
+        CU(launch_steps(h->d, h->p, h->cur, k, done + k == nsteps, part, h->stream));
+        h->cur = (h->cur + k) & 1;
+        done += k;
+    }
+    h->steps += nsteps;
     return DEM_OK;
 }
 
@@ -1044,7 +1081,7 @@ bool host_readable(const void* p) {
 // `fb` 0 or 1, flags a full search when a particle left its skin.
 int exchange(DemHandle* h, int64_t p0, int64_t n, const int* k, double* const* host,
              double* const (*cols)[4], int nfields, bool to_cols, int* error = nullptr,
-             bool sync = true, int posf = -1, int fb = -1, const HostOut* arm = nullptr) {
+             bool sync = true, int posf = -1, int fb = -1) {
     if (error && !h->err_host) {
         CU(cudaMallocHost(&h->err_host, 64));
         h->err_dev = reinterpret_cast<int*>(device_view(h->err_host));
@@ -1088,10 +1125,7 @@ int exchange(DemHandle* h, int64_t p0, int64_t n, const int* k, double* const* h
                 if (staged[f])
                     CU(cudaMemcpyAsync(staged[f], src_host[f], sizeof(double) * x.k[f] * n,
                                        cudaMemcpyHostToDevice, h->stream));
-        if (arm && xpos >= 0) {
-            x.arm = 1;
-            x.hout = *arm;
-        }
+        if (to_cols) TRY(mark_turned(h, p0, n));
         if (xpos >= 0) launch_xfer_pos(x, (int)n, h->d, h->p, xpos, fb, h->stream);
         else launch_xfer(x, (int)n, (int)p0, to_cols, h->stream);
         CU(cudaGetLastError());
@@ -1369,6 +1403,12 @@ int create_single(const DemConfigC* cfg, const DemParticlesIn* pin, const DemTab
     int rc = init_handle(h);
     if (rc == DEM_OK) rc = upload_scene(h, A, 0);
     if (rc == DEM_OK && h->tab) rc = upload_tables(h, M, mid);
+    if (rc == DEM_OK && pin->n > 0 && pin->n <= kStepsPerSm * sms) {
+        h->steps_ok = steps_ready(h->p);
+        rc = dalloc(h, &h->d.wtouch, (size_t)pin->n);
+        if (rc == DEM_OK) rc = dalloc(h, &h->d.wchg, (size_t)pin->n);
+        if (rc == DEM_OK) rc = dalloc(h, &h->d.wforce, 6 * (size_t)h->nwall * (size_t)pin->n);
+    }
     if (rc == DEM_OK) rc = flag_search(h, 0);
     if (rc == DEM_OK) {
         launch_refresh_pos32(h->d, h->p, false, 0, h->n_cap, -1, h->stream);
@@ -1579,7 +1619,8 @@ int dem_set_launch_shape(DemHandle* h, const DemLaunchShape* sh) {
     h->p.dep = h->shape.dependent_launch;
     h->p.list_lanes = h->shape.list_lanes;
     drop_graphs(h);
-    return DEM_OK;
+    // layouts other than the one-thread integrator's keep no quaternion bits
+    return mark_turned(h, 0, h->n_cap);
 }
 
 int dem_get_launch_shape(DemHandle* h, DemLaunchShape* out) {
@@ -1644,8 +1685,19 @@ int dem_step(DemHandle* h, int64_t nsteps) {
         return DEM_OK;
     }
     TRY(ensure_encoding(h));
+    if (steps_fit(h)) return run_steps(h, nsteps, StepIO{});
     TRY(build_graphs(h));
     TRY(launch_inits(h));
+    // a single scene's long calls go kRunSteps steps per graph, the last steps
+    // one by one (they store what the caller can read after the call)
+    if (!h->multi) {
+        for (; nsteps > kRunSteps; nsteps -= kRunSteps) {
+            cudaGraphExec_t& run = h->run[h->cur];
+            if (!run) TRY(capture_steps(h, h->cur, kRunSteps, false, &run));
+            CU(cudaGraphLaunch(run, h->stream));
+            h->steps += kRunSteps;
+        }
+    }
     for (int64_t s = 0; s < nsteps; ++s) {
         CU(cudaGraphLaunch(h->exec[h->cur], h->stream));
         h->cur ^= 1;
@@ -1657,7 +1709,7 @@ int dem_step(DemHandle* h, int64_t nsteps) {
 
 int dem_step_timed(DemHandle* h, int64_t nsteps, float* ms) {
     if (!h || !ms) return DEM_ERR_INVALID;
-    TRY(build_graphs(h));
+    if (!steps_fit(h)) TRY(build_graphs(h));
     CU(cudaEventRecord(h->ev0, h->stream));
     TRY(dem_step(h, nsteps));
     CU(cudaEventRecord(h->ev1, h->stream));
@@ -1756,8 +1808,7 @@ int dem_get_particles(DemHandle* h, DemParticleState* out) {
     return dem_scene_get_particles(h, 0, out);
 }
 
-int set_particles(DemHandle* h, const DemParticleState* in, bool sync,
-                  const HostOut* arm = nullptr) {
+int set_particles(DemHandle* h, const DemParticleState* in, bool sync) {
     const SceneHost* S = scene_at(h, 0);
     if (!S || !in || h->multi) return DEM_ERR_INVALID;
     const int64_t n = S->sp.n;
@@ -1783,7 +1834,7 @@ int set_particles(DemHandle* h, const DemParticleState* in, bool sync,
     // new positions: the exchange kernel refreshes the FP32 positions; the
     // neighbour lists stay valid while every particle lies within skin/2 of
     // where they were built, else the next step searches in full
-    return exchange(h, 0, n, k, host, cols, 5, true, nullptr, sync, 0, h->cur, arm);
+    return exchange(h, 0, n, k, host, cols, 5, true, nullptr, sync, 0, h->cur);
 }
 
 int dem_set_particles(DemHandle* h, const DemParticleState* in) {
@@ -1794,84 +1845,21 @@ int dem_set_particles_async(DemHandle* h, const DemParticleState* in) {
     return set_particles(h, in, false);
 }
 
-// One exchanged step as a graph (DemHandle::XGraph): captured once per
-// contact-buffer parity and set of caller buffers, replayed afterwards.
-static int capture_exchange(DemHandle* h, int cur, double* pv, double* vv, double* ov, double* qv,
-                            double* wv, const HostOut& ho, cudaGraphExec_t* exec) {
-    if (!h->side) {
-        CU(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        CU(cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming));
-        CU(cudaEventCreateWithFlags(&h->join_ev, cudaEventDisableTiming));
-    }
-    const DemDev& d = h->d;
-    const int n = h->p.n;
-    XferSet xp{};  // positions: FP32 copies, skin test, arming
-    xp.rec[0] = pv;
-    xp.col[0][0] = d.px;
-    xp.col[0][1] = d.py;
-    xp.col[0][2] = d.pz;
-    xp.k[0] = 3;
-    xp.nf = 1;
-    xp.arm = 1;
-    xp.hout = ho;
-    // velocities, spins, orientations and the first wall's shear history,
-    // beside the contact update (which reads none of them)
-    XferSet xr{};
-    double* const rv[4] = {vv, ov, qv, wv};
-    double* const cv[4][4] = {{d.vx, d.vy, d.vz}, {d.wx, d.wy, d.wz}, {d.qw, d.qx, d.qy, d.qz},
-                              {d.wsx, d.wsy, d.wsz}};
-    const int kv[4] = {3, 3, 4, 3};
-    for (int f = 0; f < 4; ++f) {
-        if (!rv[f]) continue;
-        xr.rec[xr.nf] = rv[f];
-        for (int c = 0; c < kv[f]; ++c) xr.col[xr.nf][c] = cv[f][c];
-        xr.k[xr.nf] = kv[f];
-        ++xr.nf;
-    }
-    CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    auto ok = [&](cudaError_t r) {
-        if (e == cudaSuccess) e = r;
-        return e == cudaSuccess;
-    };
-    // the positions first, with the host link to themselves (the contact
-    // update waits for them); the rest from then on, beside the contact update
-    launch_xfer_pos(xp, n, d, h->p, 0, cur, h->stream);
-    ok(cudaGetLastError());
-    if (e == cudaSuccess && xr.nf && ok(cudaEventRecord(h->fork_ev, h->stream)) &&
-        ok(cudaStreamWaitEvent(h->side, h->fork_ev, 0))) {
-        launch_xfer(xr, n, 0, true, h->side);
-        if (ok(cudaGetLastError())) ok(cudaEventRecord(h->join_ev, h->side));
-    }
-    if (e == cudaSuccess) {
-        launch_search(d, h->p, cur, false, false, false, h->shape, h->stream);
-        if (ok(cudaGetLastError()) && xr.nf) ok(cudaStreamWaitEvent(h->stream, h->join_ev, 0));
-        if (e == cudaSuccess) {
-            launch_force(d, h->p, cur ^ 1, false, h->shape, h->stream);
-            launch_integrate(d, h->p, cur, false, h->shape, h->stream);
-            ok(cudaGetLastError());
-        }
-    }
-    cudaGraph_t g = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
-    if (e == cudaSuccess) e = ec;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
-    if (g) cudaGraphDestroy(g);
-    CU(e);
-    return DEM_OK;
-}
-
-// The fused exchange: the device addresses of the caller's output records
-// (every non-null field must be device-accessible: page-locked host or
-// device memory) and of the page-locked error word.
-constexpr int kNoHostOut = INT_MIN;  // the error word's sentinel: no fused exchange ran
-static bool fused_download(DemHandle* h, const DemParticleState* out, HostOut* ho) {
-    double* const f[kHostOutFields] = {out->pos,   out->vel,    out->omega,     out->quat,
-                                       out->force, out->moment, out->wall_shear};
-    for (int q = 0; q < kHostOutFields; ++q) {
-        ho->rec[q] = nullptr;
-        if (f[q] && !(ho->rec[q] = device_view(f[q]))) return false;
-    }
+// The exchange of dem_step_exchange inside the steps' launch: the device
+// addresses of the caller's records (every given field must be
+// device-accessible: page-locked host or device memory, and the positions
+// must be given) and of the page-locked error word.
+constexpr int kNoHostOut = INT_MIN;  // the error word's sentinel: not written
+static bool direct_exchange(DemHandle* h, const DemParticleState* in, int64_t nsteps,
+                            const DemParticleState* out, StepIO* io) {
+    if (!in || !in->pos || !out || nsteps <= 0 || !steps_fit(h)) return false;
+    const double* const fi[5] = {in->pos, in->vel, in->omega, in->quat, in->wall_shear};
+    double* const fo[kHostOutFields] = {out->pos,   out->vel,    out->omega,     out->quat,
+                                        out->force, out->moment, out->wall_shear};
+    for (int q = 0; q < 5; ++q)
+        if (fi[q] && !(io->in[q] = device_view(fi[q]))) return false;
+    for (int q = 0; q < kHostOutFields; ++q)
+        if (fo[q] && !(io->out.rec[q] = device_view(fo[q]))) return false;
     if (!h->err_host) {
         if (cudaMallocHost(&h->err_host, 64) != cudaSuccess) {
             cudaGetLastError();
@@ -1880,85 +1868,32 @@ static bool fused_download(DemHandle* h, const DemParticleState* out, HostOut* h
         }
         h->err_dev = reinterpret_cast<int*>(device_view(h->err_host));
     }
-    ho->err = h->err_dev;
-    ho->done = 0u;
-    return h->err_dev != nullptr;
+    if (!h->err_dev) return false;
+    io->out.err = h->err_dev;
+    // a one-step exchange in place: values the step leaves unchanged are in
+    // `out` already (the step's input of that field came from there)
+    const double* const same[kHostOutFields] = {io->in[0], io->in[1], io->in[2], io->in[3],
+                                                nullptr,   nullptr,   io->in[4]};
+    if (nsteps == 1)
+        for (int q = 0; q < kHostOutFields; ++q)
+            if (same[q] && same[q] == io->out.rec[q]) io->out.same |= 1u << q;
+    io->has_in = io->has_out = 1;
+    return true;
 }
 
 int dem_step_exchange(DemHandle* h, const DemParticleState* in, int64_t nsteps,
                       DemParticleState* out) {
     if (!h || nsteps < 0 || h->multi) return DEM_ERR_INVALID;
-    HostOut ho{};
-    const SceneHost* S = scene_at(h, 0);
-    // the split integrator (the step graph's layout for this scene) writes
-    // the state into `out` while it runs, instead of a separate read after
-    // the step.  The upload before the step carries only the positions: in
-    // the graph of a single step the other fields are uploaded on a second
-    // stream beside the contact update; otherwise velocities and spins go
-    // with the positions, and the integrator of the first step reads the
-    // orientations and the first wall's shear history from `in` itself.
-    if (in && in->pos && out && nsteps > 0 && nsteps <= INT_MAX && S && S->sp.n > 0 &&
-        split_integrator(h->shape, h->p.n, h->p.sms) && fused_download(h, out, &ho)) {
-        *reinterpret_cast<volatile int*>(h->err_host) = kNoHostOut;
-        ho.steps_left = ho.steps_total = (int)nsteps;
-        double* const pv = device_view(in->pos);
-        double* const vv = in->vel ? device_view(in->vel) : nullptr;
-        double* const ov = in->omega ? device_view(in->omega) : nullptr;
-        double* const qv = in->quat ? device_view(in->quat) : nullptr;
-        double* const wv = in->wall_shear ? device_view(in->wall_shear) : nullptr;
-        // a one-step exchange in place: values the step leaves unchanged are
-        // in `out` already (the step's input of that field came from there)
-        const double* const inv[kHostOutFields] = {pv, vv, ov, qv, nullptr, nullptr, wv};
-        ho.same = 0u;
-        if (nsteps == 1)
-            for (int q = 0; q < kHostOutFields; ++q)
-                if (inv[q] && inv[q] == ho.rec[q]) ho.same |= 1u << q;
-        ho.qin = qv;
-        ho.wsin = wv;
-        int rc = DEM_OK;
-        if (nsteps == 1 && pv && (!in->vel || vv) && (!in->omega || ov) && (!in->quat || qv) &&
-            (!in->wall_shear || wv)) {
-            ho.qin = ho.wsin = nullptr;  // uploaded beside the contact update
-            rc = ensure_encoding(h);
-            if (rc == DEM_OK) rc = build_graphs(h);
-            const void* key[DemHandle::kXKey] = {pv, vv, ov, qv, wv, ho.err,
-                                                 reinterpret_cast<const void*>((uintptr_t)ho.same)};
-            for (int q = 0; q < kHostOutFields; ++q) key[7 + q] = ho.rec[q];
-            DemHandle::XGraph& X = h->xg[h->cur];
-            if (rc == DEM_OK && (!X.exec || std::memcmp(X.key, key, sizeof(key)) != 0)) {
-                if (X.exec) cudaGraphExecDestroy(X.exec);
-                X.exec = nullptr;
-                rc = capture_exchange(h, h->cur, pv, vv, ov, qv, wv, ho, &X.exec);
-                if (rc == DEM_OK) std::memcpy(X.key, key, sizeof(key));
-            }
-            if (rc == DEM_OK) {
-                if (cudaGraphLaunch(X.exec, h->stream) == cudaSuccess) {
-                    h->cur ^= 1;
-                    h->steps += 1;
-                } else {
-                    rc = DEM_ERR_CUDA;
-                }
-            }
-        } else {
-            DemParticleState up = *in;
-            if (ho.qin) up.quat = nullptr;
-            if (ho.wsin) up.wall_shear = nullptr;
-            rc = set_particles(h, &up, false, &ho);
-            if (rc == DEM_OK) rc = dem_step(h, nsteps);
-        }
-        if (rc != DEM_OK) {  // disarm before any later step can see it
-            cudaMemsetAsync(&h->d.ctr->hout, 0, sizeof(HostOut), h->stream);
-            cudaStreamSynchronize(h->stream);
-            return rc;
-        }
+    StepIO io{};
+    if (direct_exchange(h, in, nsteps, out, &io)) {
+        volatile int* word = h->err_host;
+        *word = kNoHostOut;
+        TRY(ensure_encoding(h));
+        TRY(run_steps(h, nsteps, io));
         CU(cudaStreamSynchronize(h->stream));
-        const int err = *reinterpret_cast<volatile int*>(h->err_host);
-        if (err != kNoHostOut) {
-            ++h->exchanges_direct;
-            return error_code(err);
-        }
-        // not expected (the split layout writes the records): the usual read
-        return dem_get_particles(h, out);
+        ++h->exchanges_direct;
+        if (*word != kNoHostOut) return error_code(*word);
+        return device_error(h);  // not expected: a barrier of the steps gave up
     }
     if (in) TRY(set_particles(h, in, false));
     TRY(dem_step(h, nsteps));
@@ -2079,10 +2014,9 @@ int dem_set_contacts(DemHandle* h, const DemContacts* in, int64_t nc) {
         CU(cudaMemcpyAsync(h->d.row_len[h->cur], rl.data(), (size_t)n * 4,
                            cudaMemcpyHostToDevice, h->stream));
     }
-    // the uploaded buffer's bond count is not kept: the force pass reads the
-    // type-ordered list of the buffer a step's rows are placed in
     RowCounter alloc[2] = {{0u, 0u}, {0u, 0u}};
     alloc[h->cur].rows = (unsigned)nc;
+    for (int64_t t = 0; t < nc; ++t) alloc[h->cur].bonds += (fl[t] & kBonded) ? 1u : 0u;
     CU(cudaMemcpyAsync(h->d.ctr->alloc, alloc, sizeof(alloc), cudaMemcpyHostToDevice,
                        h->stream));
     CU(cudaStreamSynchronize(h->stream));

@@ -36,11 +36,28 @@ __device__ __forceinline__ double norm_rn(double x, double y, double z) {
 }
 
 // `norm(𝐤ᵢ - 𝐤ⱼ) < rᵢ + rⱼ` exactly as the reference evaluates it
-// (src/kernels.jl:72, 103).
+// (src/kernels.jl:72, 103).  With R = fl(rᵢ + rⱼ), the evaluated norm lies
+// within 2^-51 of the exact one (relative), and s, the squared distance by
+// FMAs, within 2^-51 of its square: when s and R² (both with exponent fields
+// well inside the normal range) differ by more than 16 units in the last
+// place, at least 2^-49, their order is the answer, in 8 FP64 instructions
+// instead of about 26 with the square root.  The bit patterns of
+// non-negative binary64 values are ordered as the values are.
+static __device__ __noinline__ bool touching_root(double dx, double dy, double dz, double R) {
+    return norm_rn(dx, dy, dz) < R;
+}
 __device__ __forceinline__ bool touching_rn(double xi, double yi, double zi, double xj, double yj,
                                             double zj, double ri, double rj) {
-    double l = norm_rn(__dsub_rn(xi, xj), __dsub_rn(yi, yj), __dsub_rn(zi, zj));
-    return l < __dadd_rn(ri, rj);
+    const double dx = __dsub_rn(xi, xj), dy = __dsub_rn(yi, yj), dz = __dsub_rn(zi, zj);
+    const double R = __dadd_rn(ri, rj);
+    const double s = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx))), R2 = __dmul_rn(R, R);
+    const long long sb = __double_as_longlong(s), rb = __double_as_longlong(R2);
+    const bool ordinary = (unsigned)((sb >> 52) - 100) < 1800u && (unsigned)((rb >> 52) - 100) < 1800u;
+    if (ordinary && __double2hiint(R) >= 0) {
+        if (sb < rb - 16) return true;
+        if (sb > rb + 16) return false;
+    }
+    return touching_root(dx, dy, dz, R);
 }
 
 // Conservative FP32 rejection: returns false only when the FP64 test above is
@@ -130,6 +147,13 @@ __device__ __forceinline__ double rcp_nr(double x) {
     return fma(y, e, y);
 }
 
+// 1/x for any x: rcp_nr inside the normal FP32 range, the division outside it.
+static __device__ __noinline__ double rcp_div(double x) { return 1.0 / x; }
+__device__ __forceinline__ double rcp_range(double x) {
+    const unsigned e = (unsigned)(__double_as_longlong(x) >> 52) - (1023u - 125u);
+    return e < 250u ? rcp_nr(x) : rcp_div(x);  // sign clear, 2^-125 <= x < 2^125
+}
+
 // x·0.5 exactly, without the FP64 pipe: a normal x whose exponent field is at
 // least 2 loses one from it, a zero is returned as it is; subnormal,
 // smallest-normal, infinite and NaN inputs take the FP64 multiply (out of
@@ -141,6 +165,15 @@ __device__ __forceinline__ double half_exact(double x) {
     if (e - 2u < 0x7fdu) return __longlong_as_double(b - (1ll << 52));  // e in [2, 0x7fe]
     if ((b & 0x7fffffffffffffffll) == 0) return x;
     return half_hw(x);
+}
+
+// x·2 exactly, the same way: exponent fields up to 0x7fd gain one.
+static __device__ __noinline__ double twice_hw(double x) { return x + x; }
+__device__ __forceinline__ double twice_exact(double x) {
+    const long long b = __double_as_longlong(x);
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    if (e - 1u < 0x7fdu) return __longlong_as_double(b + (1ll << 52));  // e in [1, 0x7fd]
+    return twice_hw(x);
 }
 
 // Bit tests on the IEEE 754 binary64 layout (integer pipe): v is not -0; v
@@ -159,6 +192,9 @@ __device__ __forceinline__ bool finite_not_negzero(double v) {
 // with a clear sign bit the IEEE order is the order of their bit patterns,
 // and a NaN of either sign compares as an unsigned pattern above every
 // finite positive b, so it compares false as in IEEE.
+__device__ __forceinline__ bool positive_bits(double a) {  // a > 0
+    return (unsigned long long)__double_as_longlong(a) - 1ull < 0x7ff0000000000000ull;
+}
 __device__ __forceinline__ bool nonzero_bits(double a) {
     return (__double_as_longlong(a) & 0x7fffffffffffffffll) != 0;
 }

@@ -92,12 +92,13 @@ struct SceneParams {
     // neighbour-list skin (0: a full search every step) and half of it in FP32
     double skin;
     float f_skin, f_half_skin;
-    double hdt2;            // dt²/2
+    double hdt2, dt6;       // dt²/2, 6·dt
     double tol2_lo, tol2_x4;  // tolerance²·(1 - 2^-30) and 4·tolerance² (contact frame)
     float f_wn[3], f_wc0;   // FP32 wall normal and n·domain_min - wall_distance (wall screen)
     // r₀/r (particle_contact_radius_multiplier) rounded up, at least 1, and
     // rounded down (the distance screens of the bond initialisation)
     float f_r0_hi, f_r0_lo;
+    float f_tol8;  // 8·tolerance² (the FP64 frame's FP32 screen)
 };
 
 // Material, surface and wall tables of a scene built with dem_create_tables
@@ -112,6 +113,7 @@ constexpr int kMaxWalls = 8;
 struct PairConst {
     double mu, Ys, Gs, cgn, cgt;              // Hertz-Mindlin: μ, Y*, G*, γ coefficients
     double ratio, E, nu, inv1pnu, sc, st, ss;  // EBPM: ρ, E, ν, 1/(1+ν), σc, σt, σs
+    float f_sc, f_st, f_ss;                    // FP32 strengths (the breakage screen)
 };
 struct WallConst {
     double wn[3], wd;
@@ -138,32 +140,27 @@ struct alignas(8) RowCounter {
     unsigned int rows, bonds;
 };
 
-// The fused exchange of dem_step_exchange: the upload arms it, and the
-// integrator of the last of `steps_left` steps writes the particle state
-// straight into the caller's device-accessible page-locked records (the
-// DemParticleState fields in their order: pos, vel, omega, quat, force,
-// moment, wall_shear; nullptr: not written) and then the device error word
-// into `err`.  With `qin` / `wsin` set, the upload left the orientations /
-// the first wall's shear history out and the integrator of the first step
-// (steps_left == steps_total) reads them from these records instead.  Every
-// integrator launch of an armed handle counts its blocks in `done`; the last
-// block out decrements `steps_left`, so the arming lasts exactly steps_total
-// launches.  An integrator that cannot use the records (one thread per
-// particle: the host then uploads every field) only counts, and `err` keeps
-// the host's sentinel, so the host reads the state the usual way.
+// The state exchange of a dem_step_exchange call that runs inside the steps'
+// launch (k_steps), in the caller's device-accessible memory (page-locked host
+// or device): the input records of the first step (pos, vel, omega, quat, the
+// first wall's shear history; nullptr: kept, the positions always given) and
+// the output records of the last one (the DemParticleState fields in their
+// order: pos, vel, omega, quat, force, moment, wall_shear; nullptr: not
+// written) with the device error word.
 constexpr int kHostOutFields = 7;
 constexpr int kHostOutRows = 22;  // 3+3+3+4+3+3+3 values per particle
 struct HostOut {
     double* rec[kHostOutFields];
-    const double* qin;   // orientations (4n), or nullptr: uploaded
-    const double* wsin;  // first wall's shear history (3n), or nullptr: uploaded
     int* err;
-    int steps_left, steps_total;
-    unsigned int done;
     // bit f: record f is the same memory as the step's input of that field
     // (a one-step exchange in place), so values the step left bit for bit
     // unchanged are already there and are not written again
     unsigned int same;
+};
+struct StepIO {
+    const double* in[5];
+    HostOut out;
+    int has_in, has_out;
 };
 
 struct DevCounters {
@@ -173,12 +170,11 @@ struct DevCounters {
     unsigned int pad;
     RowCounter alloc[2];            // contacts placed in each contact buffer
     unsigned long long tickets[2];  // tile tickets of the scan sites (never reset)
-    unsigned int bar_count, bar_gen;  // grid barrier of the fused search (arrivals, generation)
+    unsigned int bar, bar_pad;        // grid barrier of the cooperative kernels (grid_sync)
     unsigned int hashed[2];           // particles hashed by the step reading buffer cur
     // inspection of the fused pair search (DemParams::debug_enum): candidate
     // pairs (i, j > i) it visited and the wrapping sum of enum_mix(i, j)
     unsigned long long enum_pairs, enum_hash;
-    HostOut hout;  // the fused download (zero: not armed)
 };
 
 // scan sites: each has its own ticket counter and tile-state array
@@ -190,6 +186,11 @@ struct DemDev {
     // particles
     double *px, *py, *pz, *vx, *vy, *vz, *wx, *wy, *wz;
     double *qw, *qx, *qy, *qz;
+    // one bit per slot: the one-thread integrator's step has a quaternion to
+    // look at (clear: zero spin and the identity orientation, which stay as
+    // they are).  Set by the integrator where a spin appears, and for every
+    // slot by whatever else writes spins or orientations.
+    uint32_t* qmask;
     double *m, *inv_m, *r, *r0, *inv_inertia;
     double *b_invA, *b_rbI;        // bond section constants for rb = ρ·r (1/A, rb/I)
     double *b_EA, *b_EI, *b_phic;  // E·A, E·I and 20/3·(1+ν)·rb² for rb = ρ·r
@@ -198,6 +199,11 @@ struct DemDev {
     double *fx, *fy, *fz, *tx, *ty, *tz;  // totals of the last step
     double *wsx, *wsy, *wsz;              // wall shear history: wall w of slot i at
                                           // [w * DemParams::wstride + i]
+    // k_steps: per slot, the touching walls (bit mask) with their forces and
+    // moments (row 6·wall + component, wstride slots per row), and which
+    // components of the first wall's shear history the step changed
+    uint8_t *wtouch, *wchg;
+    double* wforce;
     const MatTables* mt;                  // tables of a dem_create_tables handle, else null
     const uint8_t* mid;                   // its grains' material indices, else null
     int32_t* scene_of;                    // arena: scene of each slot (-1 free); null otherwise
@@ -262,6 +268,8 @@ struct DemParams {
     int tab;        // 1: a single scene with material / wall tables (DemDev::mt, mid)
     int list_lanes; // neighbour-list update: 0 auto, 1 or 4 lanes per particle
     int wstride;    // slots per wall-shear column
+    int report;     // 1: a step stores what only its caller reads (contact points, Hertz
+                    // forces, force and moment totals); 0: a later step of the call does
     SceneParams s0; // the scene of a single-scene handle
 };
 
@@ -287,6 +295,13 @@ inline bool split_integrator(const LaunchShape& sh, long long n, int sms) {
     return sh.integrate_lanes == 4 || (sh.integrate_lanes == 0 && n <= (long long)sms * 256);
 }
 
+// The list update of a single scene: one lane per particle (k_list1) when the
+// shape asks for it, or by default when the particles outnumber half of the
+// contact update's threads (four 256-thread blocks per SM).
+__host__ __device__ inline bool narrow_list(long long n, int sms, int list_lanes) {
+    return list_lanes == 1 || (list_lanes == 0 && n > (long long)sms * 512);
+}
+
 // ---- launchers (dem_kernels.cu) --------------------------------------------
 // All launches go to `s`.  `cur` selects the contact buffer that holds the
 // state at the start of the step; the step writes buffer cur^1.  `multi`
@@ -302,6 +317,13 @@ void launch_broadphase(const DemDev& d, const DemParams& p, int cur, bool multi,
 // particle searches (bond initialisation).
 void launch_search(const DemDev& d, const DemParams& p, int cur, bool init, bool multi, bool all,
                    const LaunchShape& sh, cudaStream_t s);
+// nsteps whole steps of a single scene in one cooperative launch, with the
+// exchange of `io` (k_steps); `report`: the last step stores the contact
+// points, Hertz forces and particle totals that a caller can read; steps_ready sets the kernels up on the current
+// device and says whether that launch fits it
+bool steps_ready(const DemParams& p);
+cudaError_t launch_steps(const DemDev& d, const DemParams& p, int cur, int nsteps, bool report,
+                         const StepIO& io, cudaStream_t s);
 void launch_force(const DemDev& d, const DemParams& p, int nxt, bool multi, const LaunchShape& sh,
                   cudaStream_t s);
 void launch_integrate(const DemDev& d, const DemParams& p, int cur, bool multi,
@@ -336,8 +358,6 @@ struct XferSet {
     int nf;
     const int* err_src;  // with err_dst (device-accessible): the kernel copies
     int* err_dst;        // the device error word (nullptr: no copy)
-    int arm;             // an upload with positions: also arms the fused download
-    HostOut hout;
 };
 void launch_xfer(const XferSet& x, int n, int p0, bool to_cols, cudaStream_t s);
 // the upload of a single-scene handle whose field `posf` holds positions:

@@ -27,6 +27,7 @@
 // All of it is captured once in a CUDA graph per contact-buffer parity (three
 // launches per step).  The standalone broad-phase kernels (k_hash,
 // k_scan_excl, k_scatter, k_canon) serve the cp_list inspection entry point.
+#include <algorithm>
 #include <type_traits>
 
 #include "dem_device.cuh"
@@ -35,10 +36,11 @@ namespace dem {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kListBlocks = 6;  // k_list1: resident blocks per SM its registers allow
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
-constexpr unsigned long long kSpinLimit = 1ull << 24;
+constexpr unsigned long long kSpinLimit = 1ull << 22;
 constexpr double kPi = 3.141592653589793;  // Julia's π rounded to binary64
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
@@ -59,6 +61,49 @@ __device__ __forceinline__ const SceneParams& scene_rec(const DemDev& d, const D
 // or it initialises bonds, or the caller hashes everything.)
 __device__ __forceinline__ bool full_search(const DemDev& d, int cur, int sc, int mode, int all) {
     return all || mode == kModeInit || d.sflags[cur][sc] != 0u;
+}
+
+// The threads of a block that work through a phase of the contact update
+// together: threads [0, nt) of the block (whole warps), their barrier `bar`
+// and a shared word that is set once a grid barrier gives up.
+struct Team {
+    int nt, bar;
+    int* fail;
+    __device__ __forceinline__ void sync() const {
+        asm volatile("barrier.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory");
+    }
+};
+
+// Grid barrier over the teams of all blocks of a cooperative launch (every
+// block is resident, so it cannot wait on one that has not started).  Block 0
+// arrives with 2^31 - (blocks - 1), the others with 1: each full round of
+// arrivals flips the word's top bit and leaves the others as they were, so
+// the word needs no reset and any grid size can use it next.  The wait is
+// bounded: when it gives up it raises kErrTimeout and returns false to every
+// thread of the team.  The release / acquire pair on the one word orders the
+// blocks' writes and drops what the SM's L1 held.  Measured with 152 blocks:
+// 1.05 us; with separate count and generation words, full fences and
+// nanosleep between polls 2.07 us.
+__device__ __forceinline__ bool grid_sync(DevCounters* c, const Team& tm,
+                                          unsigned long long spin_limit = kSpinLimit) {
+    tm.sync();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<unsigned int, cuda::thread_scope_device> word(c->bar);
+        const unsigned int add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u;
+        const unsigned int old = word.fetch_add(add, cuda::memory_order_acq_rel);
+        if ((((old + add) ^ old) & 0x80000000u) == 0u) {  // not the last to arrive
+            unsigned long long it = 0;
+            while (((word.load(cuda::memory_order_acquire) ^ old) & 0x80000000u) == 0u) {
+                if (++it > spin_limit) {
+                    raise_error(c, kErrTimeout);
+                    *tm.fail = 1;
+                    break;
+                }
+            }
+        }
+    }
+    tm.sync();
+    return *tm.fail == 0;
 }
 
 // particles placed in the bucket-sorted arrays this step
@@ -391,13 +436,6 @@ __device__ __forceinline__ int place_rows(const DemDev& d, const DemParams& p, i
         len = 0;
     }
     return start;
-}
-
-__device__ __forceinline__ void add_incoming_entry(const DemDev& d, const DemParams& p, int j,
-                                                   int pos, int i) {
-    const int slot = atomicAdd(&d.in_cnt[j], 1);
-    if (slot < p.kin) d.in_list[(size_t)j * p.kin + slot] = make_int2(pos, i);
-    else raise_error(d.ctr, kErrCapacity);
 }
 
 // Writes the row of job `r` at [start, start + r.len) of buffer cur^1 (L
@@ -925,58 +963,79 @@ __device__ __forceinline__ void list_particle(const DemDev& d, const DemParams& 
     job.nb = nbond;
 }
 
+// A Hertz contact's touching test and a list partner's, FP32 screens first
+// (maybe_touching32, surely_touching32), the exact FP64 test where neither
+// decides.
+__device__ __forceinline__ bool touches(const DemDev& d, int i, int j, float4 Pi, float4 Pj) {
+    if (!maybe_touching32(Pi, Pj)) return false;
+    return surely_touching32(Pi, d.rm32[i].z, Pj, d.rm32[j].z) ||
+           touching_rn(d.px[i], d.py[i], d.pz[i], d.px[j], d.py[j], d.pz[j], d.r[i], d.r[j]);
+}
+
+// What the FP32 screens leave open, out of line (rare; inlined, it took the
+// narrow layout's registers): does the Hertz contact (i, j) survive, and does
+// the list partner j touch.
+template <bool MULTI>
+static __device__ __noinline__ bool survives_exact(const DemDev& d, const DemParams& p, int i,
+                                                   int j) {
+    return touching_rn(d.px[i], d.py[i], d.pz[i], d.px[j], d.py[j], d.pz[j], d.r[i], d.r[j]) ||
+           !in_cp_list<MULTI>(d, scene_rec<MULTI>(d, p, slot_scene<MULTI>(d, i)), i, j);
+}
+static __device__ __noinline__ bool touches_exact(const DemDev& d, int i, int j) {
+    return touching_rn(d.px[i], d.py[i], d.pz[i], d.px[j], d.py[j], d.pz[j], d.r[i], d.r[j]);
+}
+
 // The list update of one particle by one lane (the narrow layout): the same
 // decisions as list_particle, with the row and the list walked by the lane
-// itself (no shared row cache: a row's few entries are re-read from L1).
-// Clearly touching pairs are accepted by an FP32 screen before the exact
-// FP64 test (surely_touching32).  (The four-lane path keeps the FP64 test
-// alone: on the 17,576-sphere cube the screen made its contact update 1.8 us
-// faster and the force pass 2.8 us slower, because the FP64 position loads it
-// saves were warming L2 for the force pass.)
+// itself.  Survival goes into a bit mask (rows of up to 64 entries; longer
+// ones also use the keep flags), the row is written by emit_row1.
+constexpr int kNarrowRow = 64;
 template <bool MULTI>
 __device__ __forceinline__ void list_particle1(const DemDev& d, const DemParams& p, int cur, int i,
-                                               int e0, int e1, int nv, bool frozen, RowJob& job) {
+                                               int e0, int e1, int nv, bool frozen, RowJob& job,
+                                               unsigned long long& keepm) {
     const ContactSoA o = d.c[cur];
+    const int32_t* vl = d.vl + (size_t)i * p.kvl;
+    // the first entry, the first list partner and the particle's own FP32
+    // position are loaded together (most rows and lists hold one)
+    uint32_t fl0 = e0 < e1 ? o.fl[e0] : 0u;
+    int j0 = e0 < e1 ? o.cj[e0] : -1;
+    int v0 = nv > 0 ? vl[0] : -1;
+    const float4 Pi = d.pos32[i];
     int nkeep = 0, ended = 0, nbond = 0;
+    keepm = 0ull;
     for (int e = e0; e < e1; ++e) {
-        const uint32_t fl = o.fl[e];
+        const uint32_t fl = e == e0 ? fl0 : o.fl[e];
         int keep;
         if (!(fl & kActive)) {
             keep = 0;
         } else if (frozen || (fl & kBonded)) {
             keep = 1;
         } else {
-            const int j = o.cj[e];
-            const bool valid =
-                surely_touching32(d.pos32[i], d.rm32[i].z, d.pos32[j], d.rm32[j].z) ||
-                touching_rn(d.px[i], d.py[i], d.pz[i], d.px[j], d.py[j], d.pz[j], d.r[i],
-                            d.r[j]);
-            keep = (valid ||
-                    !in_cp_list<MULTI>(d, scene_rec<MULTI>(d, p, slot_scene<MULTI>(d, i)), i, j))
+            const int j = e == e0 ? j0 : o.cj[e];
+            keep = (surely_touching32(Pi, d.rm32[i].z, d.pos32[j], d.rm32[j].z) ||
+                    survives_exact<MULTI>(d, p, i, j))
                        ? 1
                        : 0;
             ended += 1 - keep;
         }
-        d.keep[e] = (uint8_t)keep;
+        if (e - e0 < kNarrowRow) keepm |= (unsigned long long)keep << (e - e0);
+        else d.keep[e] = (uint8_t)keep;
         nkeep += keep;
         nbond += (keep && (fl & kBonded)) ? 1 : 0;
     }
     int32_t* stash = d.stash + (size_t)i * p.kstash;
     int nnew = 0;
     if (!frozen) {
-        const float4 Pi = d.pos32[i];
-        const int32_t* vl = d.vl + (size_t)i * p.kvl;
         for (int v = 0; v < nv; ++v) {
-            const int j = vl[v];
-            bool found = false;
-            for (int e = e0; e < e1 && !found; ++e)
+            const int j = v == 0 ? v0 : vl[v];
+            bool found = (fl0 & kActive) && j == j0;
+            for (int e = e0 + 1; e < e1 && !found; ++e)
                 found = (o.cj[e] == j) && (o.fl[e] & kActive);
             if (found) continue;
             const float4 Pj = d.pos32[j];
             if (!maybe_touching32(Pi, Pj)) continue;
-            if (!surely_touching32(Pi, d.rm32[i].z, Pj, d.rm32[j].z) &&
-                !touching_rn(d.px[i], d.py[i], d.pz[i], d.px[j], d.py[j], d.pz[j], d.r[i],
-                             d.r[j]))
+            if (!surely_touching32(Pi, d.rm32[i].z, Pj, d.rm32[j].z) && !touches_exact(d, i, j))
                 continue;
             if (nnew < p.kstash) stash[nnew] = j;
             ++nnew;
@@ -1009,6 +1068,63 @@ __device__ __forceinline__ void list_particle1(const DemDev& d, const DemParams&
     job.nb = nbond;
 }
 
+// One contact entry of a next row (see finish_row): `before` the row entries
+// before it, nbb the bonds among them; from: its slot in buffer cur, -1 a new
+// contact.  tl: the type-ordered list is in use.
+__device__ __forceinline__ void write_entry(const DemDev& d, const DemParams& p, int cur, int i,
+                                            int j, uint32_t fl, int from, bool stepping, int start,
+                                            int bstart, int before, int nbb, bool tl) {
+    const ContactSoA& o = d.c[cur];
+    const ContactSoA& w = d.c[cur ^ 1];
+    const int pos = start + before;
+    w.ci[pos] = i;
+    w.cj[pos] = j;
+    w.fl[pos] = fl;
+    w.src[pos] = stepping ? from : -1;
+    if (!stepping)
+        for (int f = 0; f < 15; ++f) w.f[f][pos] = from >= 0 ? o.f[f][from] : 0.0;
+    if (tl) {
+        const long long k = (fl & kBonded) ? (long long)bstart + nbb
+                                           : (long long)p.cap - 1 - (start - bstart + before - nbb);
+        if (k >= 0 && k < (long long)p.cap) d.tlist[k] = pos;
+    }
+}
+
+// One lane's row: the merge, by j, of the surviving entries and the new
+// partners in one walk.
+__device__ __forceinline__ void write_row1(const DemDev& d, const DemParams& p, int cur,
+                                           const RowJob& r, unsigned long long keepm, int start,
+                                           int bstart, int len, bool tl) {
+    d.row_start[cur ^ 1][r.i] = start;
+    d.row_len[cur ^ 1][r.i] = len;
+    if (len == 0) return;
+    const ContactSoA& o = d.c[cur];
+    const int32_t* st = d.stash + (size_t)r.i * p.kstash;
+    const bool stepping = r.mode == kModeStep;
+    int at = 0, nbb = 0, u = 0;
+    for (int e = r.e0; e < r.e1; ++e) {
+        const int k = e - r.e0;
+        if (!(k < kNarrowRow ? (int)((keepm >> k) & 1ull) : (int)d.keep[e])) continue;
+        const int j = o.cj[e];
+        const uint32_t fl = o.fl[e];
+        for (; u < r.nnew && st[u] < j; ++u, ++at)
+            write_entry(d, p, cur, r.i, st[u], kActive, -1, stepping, start, bstart, at, nbb, tl);
+        write_entry(d, p, cur, r.i, j, fl, e, stepping, start, bstart, at, nbb, tl);
+        ++at;
+        nbb += (fl & kBonded) ? 1 : 0;
+    }
+    for (; u < r.nnew; ++u, ++at)
+        write_entry(d, p, cur, r.i, st[u], kActive, -1, stepping, start, bstart, at, nbb, tl);
+}
+
+// Places and writes the rows of a warp's 32 particles, one lane each (every
+// lane of the warp calls it).
+__device__ __forceinline__ void emit_row1(const DemDev& d, const DemParams& p, int cur, bool active,
+                                          const RowJob& r, unsigned long long keepm, bool tl) {
+    int len = active ? r.len : 0, bstart = 0;
+    const int start = place_rows<1>(d, p, cur ^ 1, len, active ? r.nb : 0, &bstart);
+    if (active) write_row1(d, p, cur, r, keepm, start, bstart, len, tl);
+}
 // The neighbour-list update with one lane per particle: in large scenes with
 // few contacts and list partners per particle (a compacted bed, a pour) four
 // lanes per particle leave most lanes idle and too few particles in flight
@@ -1020,9 +1136,10 @@ __device__ __forceinline__ void list_particle1(const DemDev& d, const DemParams&
 // consecutive blocks on the same SM, so chunks by block would leave SMs idle
 // whenever the particles do not fill the grid.
 template <bool MULTI>
-__device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemParams& p, int cur) {
+__device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemParams& p, int cur,
+                                                  int nt, bool tl) {
     const int wslot = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
-    for (long long t0 = 0; t0 < p.n; t0 += (long long)gridDim.x * kThreads) {
+    for (long long t0 = 0; t0 < p.n; t0 += (long long)gridDim.x * nt) {
         const int i0 = (int)(t0 + 32LL * wslot);
         const int i = i0 + (int)lane_id();
         bool act = i < p.n, frz = false;
@@ -1032,6 +1149,7 @@ __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemPara
             frz = (path >> 2) == kModeFrozen;
         }
         RowJob job{};
+        unsigned long long keepm = 0ull;
         if (act) {
             const int e0 = d.row_start[cur][i];
             const int e1 = e0 + d.row_len[cur][i];
@@ -1041,11 +1159,121 @@ __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemPara
                 d.row_len[cur ^ 1][i] = 0;
                 act = false;
             } else {
-                list_particle1<MULTI>(d, p, cur, i, e0, e1, nv, frz, job);
+                list_particle1<MULTI>(d, p, cur, i, e0, e1, nv, frz, job, keepm);
             }
         }
-        emit_rows<1>(d, p, cur, act, job, 0);
+        emit_row1(d, p, cur, act, job, keepm, tl);
     }
+}
+
+// The list update of a warp's eight particles, four lanes each, whose rows and
+// lists all hold at most four entries (the common case: a bonded lattice, a
+// bed): lane k of a group takes row entry k and list partner k, the decisions
+// are exchanged by ballots, and a row is placed and written from registers.
+// Same decisions and rows as list_particle and emit_rows, which walk rows of
+// any length through shared memory, survival flags in memory and warp scans:
+// about 14 dependent memory round trips and 600 instructions of a chain that
+// needs 5 (row bounds; entries and list; partners' positions; the placing
+// atomic; the row's stores).
+template <bool MULTI>
+__device__ __forceinline__ void list_quads(const DemDev& d, const DemParams& p, int cur, int i,
+                                           bool act, bool frozen, int e0, int len, int nv,
+                                           bool tl) {
+    const unsigned full = 0xffffffffu;
+    const int gl = (int)lane_id() & 3, gbase = (int)lane_id() & ~3;
+    const ContactSoA& o = d.c[cur];
+    const int e = e0 + gl;
+    const bool has = gl < len;
+    const uint32_t fl = has ? o.fl[e] : 0u;
+    const int cj = has ? o.cj[e] : -1;
+    const int vj = gl < nv ? d.vl[(size_t)i * p.kvl + gl] : -1;
+    const bool alive = (fl & kActive) != 0u, bond = alive && (fl & kBonded);
+    const int row = alive ? cj : -1;
+    bool found = vj < 0;  // a partner already in the row (a bond, a Hertz contact)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) found |= __shfl_sync(full, row, gbase + k) == vj;
+    const bool hertz = alive && !bond && !frozen;
+    bool touch = false, fresh = false;
+    if (hertz || !found) {
+        const float4 Pi = d.pos32[i];
+        const float ri = d.rm32[i].z;
+        float4 Pc = Pi, Pv = Pi;
+        float rc = ri;
+        if (hertz) {
+            Pc = d.pos32[cj];
+            rc = d.rm32[cj].z;
+        }
+        if (!found) Pv = d.pos32[vj];
+        if (hertz)
+            touch = surely_touching32(Pi, ri, Pc, rc) || touches(d, i, cj, Pi, Pc);
+        if (!found) fresh = touches(d, i, vj, Pi, Pv);
+    }
+    // a Hertz contact that no longer touches ends iff the pair is in the
+    // cp_list: the group's lanes share each such test
+    bool keep = alive && (bond || frozen || touch), ended = false;
+    for (unsigned pend = __ballot_sync(full, hertz && !touch); pend; pend &= pend - 1) {
+        const int src = __ffs(pend) - 1;
+        if ((src & ~3) == gbase) {
+            const unsigned gmask = 0xfu << gbase;
+            const int j = __shfl_sync(gmask, cj, src);
+            const bool in = in_cp_list_group(
+                d, scene_rec<MULTI>(d, p, slot_scene<MULTI>(d, i)), i, j, gl, gmask);
+            if ((int)lane_id() == src) {
+                keep = !in;
+                ended = in;
+            }
+        }
+        __syncwarp();
+    }
+    const unsigned K = __ballot_sync(full, keep), N = __ballot_sync(full, fresh);
+    const unsigned B = __ballot_sync(full, keep && bond), E = __ballot_sync(full, ended);
+    const unsigned gK = (K >> gbase) & 0xfu, gN = (N >> gbase) & 0xfu, gB = (B >> gbase) & 0xfu;
+    if (gl == 0 && ((N | E) >> gbase) & 0xfu) {
+        const int sc = slot_scene<MULTI>(d, i);
+        const unsigned gE = (E >> gbase) & 0xfu;
+        if (gE) atomicAdd(&d.sctr[sc].ended, (unsigned long long)__popc(gE));
+        if (gN) atomicAdd(&d.sctr[sc].created, (unsigned long long)__popc(gN));
+    }
+    // the rows' places (place_rows, from the ballots)
+    const unsigned below = (1u << gbase) - 1u;
+    unsigned long long base = 0ull;
+    if (lane_id() == 0 && (K | N))
+        base = atomicAdd(reinterpret_cast<unsigned long long*>(&d.ctr->alloc[cur ^ 1]),
+                         (unsigned long long)(__popc(K) + __popc(N)) |
+                             ((unsigned long long)__popc(B) << 32));
+    // entries before this lane's in its row: survivors of smaller j (row
+    // order), new partners of smaller j
+    const unsigned lt = (1u << gl) - 1u;
+    int kbefore = __popc(gK & lt), kbonds = __popc(gB & lt);  // of this lane's row entry
+    int nbefore = 0, nbonds = 0;                              // of its new partner
+    if (N) {
+        const int kj = keep ? cj : -1, nj = fresh ? vj : 0x7fffffff;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int a = __shfl_sync(full, kj, gbase + k), b = __shfl_sync(full, nj, gbase + k);
+            kbefore += b < cj ? 1 : 0;
+            nbefore += (a >= 0 && a < vj ? 1 : 0) + (b < vj ? 1 : 0);
+            nbonds += (a >= 0 && a < vj && ((gB >> k) & 1u)) ? 1 : 0;
+        }
+    }
+    base = __shfl_sync(full, base, 0);
+    int start = (int)((unsigned)base + __popc(K & below) + __popc(N & below));
+    const int bstart = (int)((unsigned)(base >> 32) + __popc(B & below));
+    int rlen = __popc(gK) + __popc(gN);
+    if (rlen > 0 && (long long)start + rlen > (long long)p.cap) {
+        if (gl == 0) raise_error(d.ctr, kErrCapacity);
+        rlen = 0;
+    }
+    if (rlen == 0) start = 0;
+    if (act && gl == 0) {
+        d.row_start[cur ^ 1][i] = start;
+        d.row_len[cur ^ 1][i] = rlen;
+    }
+    if (rlen == 0) return;
+    if (keep)
+        write_entry(d, p, cur, i, cj, fl, e, !frozen, start, bstart, kbefore, kbonds, tl);
+    if (fresh)
+        write_entry(d, p, cur, i, vj, kActive, -1, !frozen, start, bstart, nbefore, nbonds, tl);
 }
 
 // The neighbour-list update (a12, a13, a21 for scenes whose lists are valid):
@@ -1061,12 +1289,19 @@ __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemPara
 // 0.581 ms per step).
 template <bool MULTI>
 __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, int cur,
-                                           ListShared* sh) {
+                                           ListShared* sh, int nt) {
+    // contacts in the current buffer: fixed while this kernel runs (rows are
+    // placed in the other buffer), so every thread takes the same branch
+    const unsigned ncur = __ldcg(&d.ctr->alloc[cur].rows);
+    // without bonds in the current buffer the next one has none (they only
+    // come from the bond initialisation), and the force pass of one type of
+    // contacts reads no type-ordered list
+    const bool tl = MULTI || __ldcg(&d.ctr->alloc[cur].bonds) != 0u;
     // one lane per particle when chosen, or by default when the particles
     // outnumber half the launch's threads
-    if (p.list_lanes == 1 ||
-        (p.list_lanes == 0 && 2LL * p.n > (long long)gridDim.x * kThreads)) {
-        list_phase_narrow<MULTI>(d, p, cur);
+    if (MULTI && (p.list_lanes == 1 ||
+                  (p.list_lanes == 0 && 2LL * p.n > (long long)gridDim.x * nt))) {
+        list_phase_narrow<MULTI>(d, p, cur, nt, tl);
         return;
     }
     const int lane = threadIdx.x & (kVLanes - 1);
@@ -1074,13 +1309,10 @@ __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, 
     const unsigned gmask = 0xfu << (lane_id() & ~3u);
     // a warp's eight groups move together (their rows are placed per warp)
     const int gwarp = (int)(threadIdx.x >> 5) * (32 / kVLanes);
-    // contacts in the current buffer: fixed while this kernel runs (rows are
-    // placed in the other buffer), so every thread takes the same branch
-    const long long ncur = (long long)__ldcg(&d.ctr->alloc[cur].rows);
-    if (p.n > gridDim.x * (kThreads / kVLanes) && 4 * ncur < (long long)p.n) {
+    if (p.n > (int)gridDim.x * (nt / kVLanes) && 4ll * ncur < (long long)p.n) {
         const int gw = g - gwarp;  // the group within the warp, 0..7
-        for (int base = blockIdx.x * kThreads + (int)(threadIdx.x & ~31u); base < p.n;
-             base += gridDim.x * kThreads) {
+        for (int base = blockIdx.x * nt + (int)(threadIdx.x & ~31u); base < p.n;
+             base += gridDim.x * nt) {
             const int ip = base + (int)lane_id();
             bool act = ip < p.n, frz = false;
             if (MULTI && act) {
@@ -1128,7 +1360,7 @@ __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, 
     const int per = (int)((((long long)p.n + gridDim.x - 1) / gridDim.x + 7) & ~7LL);
     const int lo = blockIdx.x * per;
     const int hi = min(lo + per, p.n);
-    for (int i0 = lo + gwarp; i0 < hi; i0 += kThreads / kVLanes) {
+    for (int i0 = lo + gwarp; i0 < hi; i0 += nt / kVLanes) {
         const int i = i0 + (g - gwarp);
         // which particles test their lists: the path byte the search wrote (arena)
         bool active = i < hi;
@@ -1144,16 +1376,18 @@ __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, 
             e0 = d.row_start[cur][i];
             e1 = e0 + d.row_len[cur][i];
             nv = frozen ? 0 : d.vl_len[i];
-            // no contact and no list partner: an empty next row, decided at once
-            if (e1 == e0 && nv == 0) {
-                job.i = i;
-                job.mode = frozen ? kModeFrozen : kModeStep;
-                job.e0 = job.e1 = e0;
-                active = false;
-                if (lane == 0) {
-                    d.row_start[cur ^ 1][i] = 0;
-                    d.row_len[cur ^ 1][i] = 0;
-                }
+        }
+        if (p.kstash >= kVLanes &&
+            __all_sync(0xffffffffu, e1 - e0 <= kVLanes && nv <= kVLanes)) {
+            list_quads<MULTI>(d, p, cur, i, active, frozen, e0, e1 - e0, nv, tl);
+            continue;
+        }
+        // no contact and no list partner: an empty next row, decided at once
+        if (active && e1 == e0 && nv == 0) {
+            active = false;
+            if (lane == 0) {
+                d.row_start[cur ^ 1][i] = 0;
+                d.row_len[cur ^ 1][i] = 0;
             }
         }
         if (active) list_particle<MULTI>(d, p, cur, sh, g, lane, gmask, i, e0, e1, nv, frozen, job);
@@ -1173,44 +1407,16 @@ __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, 
 // each slot's path), runs the list update of its list scenes, and ends there
 // when nothing was hashed.
 
-// Grid barrier: arrival counter and generation word; a block waits for the
-// generation to move on, with a bounded wait that raises kErrTimeout.
-__device__ __forceinline__ void grid_sync(DevCounters* c,
-                                          unsigned long long spin_limit = kSpinLimit) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* gen = &c->bar_gen;
-        const unsigned int g = *gen;
-        __threadfence();
-        if (atomicAdd(&c->bar_count, 1u) == gridDim.x - 1) {
-            atomicExch(&c->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&c->bar_gen, 1u);
-        } else {
-            for (unsigned long long it = 0; *gen == g; ++it) {
-                if (it > spin_limit) {
-                    raise_error(c, kErrTimeout);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-// Block-wide sum of one value per thread (kThreads threads).
-__device__ __forceinline__ unsigned long long block_sum(unsigned long long v,
-                                                        unsigned long long* red) {
+// Sum of one value per thread of the team.
+__device__ __forceinline__ unsigned long long team_sum(unsigned long long v, const Team& tm,
+                                                       unsigned long long* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane_id() == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
+    tm.sync();
     unsigned long long t = 0;
-#pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    __syncthreads();
+    for (int w = 0; w < tm.nt / 32; ++w) t += red[w];
+    tm.sync();
     return t;
 }
 
@@ -1218,32 +1424,33 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v,
 // buckets up to this step's largest, as the standalone scan), in tiles of
 // kScanTile: tile sums, a barrier, then each tile's prefix from the sums.
 // Ends with a barrier.
-constexpr int kFusedItems = kScanTile / kThreads;
-__device__ void scan_phase(const DemDev& d, const DemParams& p, unsigned long long* red) {
+__device__ bool scan_phase(const DemDev& d, const DemParams& p, const Team& tm,
+                           unsigned long long* red) {
     // (values written by other blocks earlier in this launch are read past L1)
     const long long lim = (long long)__ldcg(&d.ctr->bmax) + 1;
     const long long count = lim < (long long)p.T ? lim : (long long)p.T;
     const int ntiles = (int)((count + kScanTile - 1) / kScanTile);
+    const int items = (kScanTile + tm.nt - 1) / tm.nt;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * kFusedItems;
+        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * items;
+        const long long end = min(min(base + items, (long long)(t + 1) * kScanTile), count);
         unsigned long long v = 0;
 #pragma unroll 8
-        for (int k = 0; k < kFusedItems; ++k)
-            if (base + k < count) v += d.cell_count[base + k];
-        const unsigned long long tot = block_sum(v, red);
+        for (long long k = base; k < end; ++k) v += d.cell_count[k];
+        const unsigned long long tot = team_sum(v, tm, red);
         if (threadIdx.x == 0) d.tile_sums[t] = (uint32_t)tot;
     }
-    grid_sync(d.ctr);
+    if (!grid_sync(d.ctr, tm)) return false;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         unsigned long long pre = 0;
-        for (int u = threadIdx.x; u < t; u += kThreads) pre += __ldcg(&d.tile_sums[u]);
-        pre = block_sum(pre, red);
-        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * kFusedItems;
+        for (int u = threadIdx.x; u < t; u += tm.nt) pre += __ldcg(&d.tile_sums[u]);
+        pre = team_sum(pre, tm, red);
+        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * items;
+        const long long end = min(min(base + items, (long long)(t + 1) * kScanTile), count);
         unsigned long long mine = 0;
 #pragma unroll 8
-        for (int k = 0; k < kFusedItems; ++k)
-            if (base + k < count) mine += d.cell_count[base + k];
-        // exclusive prefix of `mine` across the block
+        for (long long k = base; k < end; ++k) mine += d.cell_count[k];
+        // exclusive prefix of `mine` across the team
         unsigned long long x = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1251,36 +1458,31 @@ __device__ void scan_phase(const DemDev& d, const DemParams& p, unsigned long lo
             if (lane_id() >= (unsigned)o) x += y;
         }
         if (lane_id() == 31) red[threadIdx.x >> 5] = x;
-        __syncthreads();
+        tm.sync();
         unsigned long long wpre = 0;
         for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) wpre += red[w];
-        __syncthreads();
+        tm.sync();
         unsigned long long run = pre + wpre + x - mine;
 #pragma unroll 8
-        for (int k = 0; k < kFusedItems; ++k) {
-            if (base + k < count) {
-                d.cell_start[base + k] = (uint32_t)run;
-                run += d.cell_count[base + k];
-            }
+        for (long long k = base; k < end; ++k) {
+            d.cell_start[k] = (uint32_t)run;
+            run += d.cell_count[k];
         }
-        if (t == ntiles - 1 && threadIdx.x == kThreads - 1) d.cell_start[count] = (uint32_t)run;
+        if (t == ntiles - 1 && (int)threadIdx.x == tm.nt - 1) d.cell_start[count] = (uint32_t)run;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr->cell_limit = (unsigned int)count;
-    grid_sync(d.ctr);
+    return grid_sync(d.ctr, tm);
 }
 
-template <bool INIT, bool MULTI, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB) k_search(DemDev d, DemParams p, int cur, int all) {
-    __shared__ DetectShared sh[kThreads / kLanes];
-    __shared__ ListShared lsh[kThreads / kVLanes];
-    __shared__ unsigned long long red[kThreads / 32];
-    dep_begin();
-    if (!MULTI && !(all || INIT || d.sflags[cur][0] != 0u)) {
-        list_phase<false>(d, p, cur, lsh);  // the scene tests its neighbour lists
-        return;
-    }
-    const int stride = gridDim.x * kThreads;
-    const int wbase = blockIdx.x * kThreads + (int)(threadIdx.x & ~31u);
+// The full pair search of the scenes that run it this step, with the list
+// update of the others, by every block's team (sh holds nt / kLanes,
+// lsh nt / kVLanes and red nt / 32 entries).  False once a barrier gave up.
+template <bool INIT, bool MULTI>
+__device__ __forceinline__ bool search_phases(const DemDev& d, const DemParams& p, int cur, int all,
+                                              const Team& tm, DetectShared* sh, ListShared* lsh,
+                                              unsigned long long* red) {
+    const int stride = gridDim.x * tm.nt;
+    const int wbase = blockIdx.x * tm.nt + (int)(threadIdx.x & ~31u);
     if (MULTI && blockIdx.x == 0 && threadIdx.x == 0) d.ctr->hashed[cur ^ 1] = 0u;
     // hash (`cell`, `hashcode`, `neighbors`, `count_particles!`)
     for (int i0 = wbase; i0 < p.n; i0 += stride) {
@@ -1290,31 +1492,31 @@ __global__ void __launch_bounds__(kThreads, MINB) k_search(DemDev d, DemParams p
         if (i < p.n) hash_particle<MULTI>(d, p, cur, all, i, act, b);
         hash_count(d, act, b, MULTI ? &d.ctr->hashed[cur] : nullptr);
     }
-    grid_sync(d.ctr);
+    if (!grid_sync(d.ctr, tm)) return false;
     // the scenes that test their neighbour lists (path bytes written above):
     // independent of the search below (other particles and rows)
-    if (MULTI && !INIT) list_phase<true>(d, p, cur, lsh);
-    if (MULTI && *(volatile unsigned int*)&d.ctr->hashed[cur] == 0u) return;
+    if (MULTI && !INIT) list_phase<true>(d, p, cur, lsh, tm.nt);
+    if (MULTI && *(volatile unsigned int*)&d.ctr->hashed[cur] == 0u) return true;
     // `accumulate!` of the bucket counts
-    scan_phase(d, p, red);
+    if (!scan_phase(d, p, tm, red)) return false;
     // `get_particle_id!`
     for (int i0 = wbase; i0 < p.n; i0 += stride) scatter_warp(d, p, i0 + (int)lane_id());
-    grid_sync(d.ctr);
+    if (!grid_sync(d.ctr, tm)) return false;
     // canonical order; this step's bucket maximum is no longer read
     const uint32_t lim = __ldcg(&d.ctr->cell_limit);
     const int count = (int)__ldcg(&d.cell_start[lim]);
     if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr->bmax = 0u;
-    for (int k = blockIdx.x * kThreads + (int)threadIdx.x; k < count; k += stride)
+    for (int k = blockIdx.x * tm.nt + (int)threadIdx.x; k < count; k += stride)
         canon_slot<MULTI>(d, p, cur, k);
-    grid_sync(d.ctr);
+    if (!grid_sync(d.ctr, tm)) return false;
     // cp_list enumeration with update_contacts! / init_bonds!, then the next
     // rows; a warp's four groups move together (the rows are placed per warp)
     const int lane = threadIdx.x & (kLanes - 1);
     const int g = threadIdx.x / kLanes;
     const unsigned gmask = 0xffu << (lane_id() & ~7u);
     const int gwarp = (int)(threadIdx.x >> 5) * (32 / kLanes);  // the warp's first group
-    for (int k0 = blockIdx.x * (kThreads / kLanes) + gwarp; k0 < count;
-         k0 += gridDim.x * (kThreads / kLanes)) {
+    for (int k0 = blockIdx.x * (tm.nt / kLanes) + gwarp; k0 < count;
+         k0 += gridDim.x * (tm.nt / kLanes)) {
         const int k = k0 + (g - gwarp);
         RowJob job{};
         const bool active = k < count;
@@ -1322,6 +1524,139 @@ __global__ void __launch_bounds__(kThreads, MINB) k_search(DemDev d, DemParams p
         emit_rows<kLanes>(d, p, cur, active, job, lane);
         __syncwarp();
     }
+    return true;
+}
+
+template <bool INIT, bool MULTI, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB)
+    k_search(const __grid_constant__ DemDev d, const __grid_constant__ DemParams p, int cur, int all) {
+    __shared__ DetectShared sh[kThreads / kLanes];
+    __shared__ ListShared lsh[kThreads / kVLanes];
+    __shared__ unsigned long long red[kThreads / 32];
+    __shared__ int fail;
+    dep_begin();
+    if (!MULTI && !(all || INIT || d.sflags[cur][0] != 0u)) {
+        // the scene tests its neighbour lists (k_list1 has, if it was launched)
+        if (!narrow_list(p.n, p.sms, p.list_lanes)) list_phase<false>(d, p, cur, lsh, kThreads);
+        return;
+    }
+    if (threadIdx.x == 0) fail = 0;  // the first barrier orders this before any read of it
+    search_phases<INIT, MULTI>(d, p, cur, all, Team{kThreads, 0, &fail}, sh, lsh, red);
+}
+
+// 𝐪 + Δ𝐪 with Δ𝐪 = ½ 𝛚 ⊗ 𝐪 (no dt, as the reference), the ½ folded into
+// 𝛚, as explicit FMA chains.  With 𝛚 = (+0, +0, +0) each fma(a, +0, c)
+// (a finite) returns c unless c is -0, so for a finite 𝐪 without a -0
+// component the chains return 𝐪 itself: a particle that does not spin
+// skips them, with identical results.  The normalisation always runs.
+// A spinless particle with the identity orientation (1, +0, +0, +0)
+// keeps it: |𝐪|² = 1 exactly, rsqrt(1) = 1 (checked by
+// dem_selftest_conversions) and 𝐪·1 = 𝐪, so nothing is computed or stored
+// (false is returned).
+__device__ __forceinline__ bool update_quaternion(const DemDev& d, int i, double wx, double wy,
+                                                  double wz, double qw, double qx, double qy,
+                                                  double qz) {
+    double nw = qw, nx = qx, ny = qy, nz = qz;
+    const bool spinless = (__double_as_longlong(wx) | __double_as_longlong(wy) |
+                           __double_as_longlong(wz)) == 0ll;
+    const bool identity = spinless && __double_as_longlong(qw) == 0x3ff0000000000000ll &&
+                          (__double_as_longlong(qx) | __double_as_longlong(qy) |
+                           __double_as_longlong(qz)) == 0ll;
+    if (identity) return false;
+    if (!(spinless && finite_not_negzero(qw) && finite_not_negzero(qx) &&
+          finite_not_negzero(qy) && finite_not_negzero(qz))) {
+        const double hx = half_exact(wx), hy = half_exact(wy), hz = half_exact(wz);
+        nw = __fma_rn(-qz, hz, __fma_rn(-qy, hy, __fma_rn(-qx, hx, qw)));
+        nx = __fma_rn(-qz, hy, __fma_rn(qy, hz, __fma_rn(qw, hx, qx)));
+        ny = __fma_rn(qz, hx, __fma_rn(qx, hz, __fma_rn(qw, hy, qy)));
+        nz = __fma_rn(-qy, hx, __fma_rn(qx, hy, __fma_rn(qw, hz, qz)));
+    }
+    const double inq = rsqrt(__fma_rn(nz, nz, __fma_rn(ny, ny, __fma_rn(nx, nx, nw * nw))));
+    d.qw[i] = nw * inq;
+    d.qx[i] = nx * inq;
+    d.qy[i] = ny * inq;
+    d.qz[i] = nz * inq;
+    return true;
+}
+// The quaternions of a warp's 32 particles (slot i on lane i mod 32), reading
+// only those whose bit of d.qmask is set (DemDev); clears the bits of those
+// that turn out to have nothing to update.
+__device__ __forceinline__ void quaternion_warp(const DemDev& d, int i, bool exists) {
+    const uint32_t word = exists ? d.qmask[i >> 5] : 0u;
+    bool more = false;
+    if ((word >> lane_id()) & 1u)
+        more = update_quaternion(d, i, d.wx[i], d.wy[i], d.wz[i], d.qw[i], d.qx[i], d.qy[i], d.qz[i]);
+    const uint32_t left = __ballot_sync(0xffffffffu, more);
+    if (lane_id() == 0 && left != word) d.qmask[i >> 5] = left;
+}
+
+// The list update of a single scene with one lane per particle, in a launch of
+// its own before k_search (which then only runs for a scene that searches).
+// A block places its 256 particles' rows with one atomic: with one per warp,
+// the 62,500 same-address atomics of 2,000,000 particles took longer than
+// everything else.  It also updates the particles' quaternions, which depend on
+// the step's starting spins only: the list update waits for memory and leaves
+// the FP64 pipe idle, and in the integrator, which keeps that pipe more than
+// half busy, the update was 28 of a particle's 48 FP64 instructions.
+__global__ void __launch_bounds__(kThreads, kListBlocks)
+    k_list1(const __grid_constant__ DemDev d, const __grid_constant__ DemParams p, int cur,
+            int quat) {
+    __shared__ unsigned long long s_tot[kThreads / 32];  // a warp's rows | bonds << 32
+    __shared__ unsigned long long s_base;
+    dep_begin();
+    const int i = blockIdx.x * kThreads + (int)threadIdx.x;
+    bool act = i < p.n;
+    if (quat) quaternion_warp(d, i, act);
+    if (d.sflags[cur][0] != 0u) return;
+    const bool tl = __ldcg(&d.ctr->alloc[cur].bonds) != 0u;
+    RowJob job{};
+    unsigned long long keepm = 0ull;
+    if (act) {
+        const int e0 = d.row_start[cur][i];
+        const int e1 = e0 + d.row_len[cur][i];
+        const int nv = d.vl_len[i];
+        if (e1 == e0 && nv == 0) {  // no contact and no list partner: an empty row
+            d.row_start[cur ^ 1][i] = 0;
+            d.row_len[cur ^ 1][i] = 0;
+            act = false;
+        } else {
+            list_particle1<false>(d, p, cur, i, e0, e1, nv, false, job, keepm);
+        }
+    }
+    const int len = act ? job.len : 0, nb = act ? job.nb : 0;
+    if (__syncthreads_or(act ? 1 : 0) == 0) return;
+    // the lengths of 32 rows and their bonds, scanned together in one word
+    // (a row has at most the capacity, below 2^31, entries)
+    unsigned long long x = (unsigned long long)(unsigned)len | ((unsigned long long)(unsigned)nb << 32);
+    const unsigned long long mine = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane_id() >= (unsigned)o) x += y;
+    }
+    const int w = (int)(threadIdx.x >> 5);
+    if (lane_id() == 31) s_tot[w] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long t = 0;
+#pragma unroll
+        for (int k = 0; k < kThreads / 32; ++k) {
+            const unsigned long long v = s_tot[k];
+            s_tot[k] = t;
+            t += v;
+        }
+        s_base = t ? atomicAdd(reinterpret_cast<unsigned long long*>(&d.ctr->alloc[cur ^ 1]), t) : 0ull;
+    }
+    __syncthreads();
+    if (!act) return;
+    const unsigned long long at = s_base + s_tot[w] + x - mine;
+    int start = (int)(unsigned)at, rlen = len;
+    if (rlen > 0 && (long long)start + rlen > (long long)p.cap) {
+        raise_error(d.ctr, kErrCapacity);
+        rlen = 0;
+    }
+    if (rlen == 0) start = 0;
+    write_row1(d, p, cur, job, keepm, start, (int)(unsigned)(at >> 32), rlen, tl);
 }
 
 // End of a step (run by k_integrate): the rebuild flags of this step are
@@ -1400,17 +1735,25 @@ static __device__ __noinline__ Frame frame_exact_from(double dx, double dy, doub
 }
 __device__ __forceinline__ Frame contact_frame(double dx, double dy, double dz, double ax,
                                                double ay, double az, const SceneParams& S) {
+    Frame F;
+    F.a1 = ax;
+    F.a2 = ay;
+    F.a3 = az;
+    F.neg3 = false;
+    // f = (1 - a₁)/s² = 1/(1 + a₁), since s² = 1 - a₁²: three FP64
+    // instructions fewer, and well conditioned away from a₁ = -1.  That the
+    // degenerate branch is far (s² well above 4·tolerance²) is seen in FP32.
+    const float y = d2f(ay), z = d2f(az);
+    if (y * y + z * z > S.f_tol8 && d2f(ax) > -0.5f) {
+        F.f = rcp_nr(1.0 + ax);  // in (0.5, 2]
+        return F;
+    }
     const double s2 = ay * ay + az * az;
     // s² >= +0 (a sum of squares) and the tolerances are positive: compared
     // as bit patterns, off the FP64 pipe
     if (less_nonneg(s2, S.tol2_lo)) return frame_degenerate(ax);
     if (less_nonneg(s2, S.tol2_x4)) return frame_exact_from(dx, dy, dz, S.tol);
-    Frame F;
-    F.a1 = ax;
-    F.a2 = ay;
-    F.a3 = az;
-    F.f = (1.0 - ax) * rcp_nr(s2);  // (1 - a₁)/s²
-    F.neg3 = false;
+    F.f = (1.0 - ax) * rcp_range(s2);
     return F;
 }
 template <typename T>
@@ -1472,13 +1815,6 @@ __device__ __forceinline__ bool bond_breaks(const Vec3<double>& F, const Vec3<do
                                             const SceneParams& p) {
     return bond_breaks(F, ti, tj, invA, rbI, p.b_sc, p.b_st, p.b_ss);
 }
-// The breakage test of a bond between grains of a table scene (no FP32 screen).
-static __device__ __noinline__ bool bond_breaks_tab(const Vec3<double>& F, const Vec3<double>& ti,
-                                                    const Vec3<double>& tj, double invA,
-                                                    double rbI, const PairConst& pc) {
-    return bond_breaks(F, ti, tj, invA, rbI, pc.sc, pc.st, pc.ss);
-}
-
 // Breakage decision of bond_breaks behind an FP32 screen.  The three stresses
 // σc = fa + rb/I·sqrt(amax), σt = -fa - rb/I·sqrt(amin) and
 // σs = |τᵢ₁|·rb/2/I + 4/3/A·sqrt(F₂²+F₃²) are evaluated in FP32 from the FP64
@@ -1501,14 +1837,13 @@ static __device__ __noinline__ bool bond_breaks_pairs(const float2 (&F)[3], cons
 }
 
 __device__ __forceinline__ bool stress_clear(const Vec3<float>& Ff, const Vec3<float>& tif,
-                                             const Vec3<float>& tjf, float iA, float rb,
-                                             const SceneParams& p) {
+                                             const Vec3<float>& tjf, float iA, float rb, float sc,
+                                             float st, float ss) {
     const float ai = tif.y * tif.y + tif.z * tif.z, aj = tjf.y * tjf.y + tjf.z * tjf.z;
     const float fa = Ff.x * iA;
     const float smax = rb * sqrtf(fmaxf(ai, aj)), smin = rb * sqrtf(fminf(ai, aj));
     const float s1 = fabsf(tif.x) * 0.5f * rb;
     const float s2 = (4.0f / 3.0f) * iA * sqrtf(Ff.y * Ff.y + Ff.z * Ff.z);
-    const float sc = p.f_sc, st = p.f_st, ss = p.f_ss;
     const float afa = fabsf(fa);
     return (fa + smax + (afa + smax + fabsf(sc)) * 0x1p-16f < sc) &&
            (-fa - smin + (afa + smin + fabsf(st)) * 0x1p-16f < st) &&
@@ -1519,7 +1854,7 @@ __device__ __forceinline__ bool bond_breaks_screened(const float2 (&F)[3], const
                                                      const Vec3<float>& tif, const Vec3<float>& tjf,
                                                      float iA, float rb, const DemDev& d, int small,
                                                      const SceneParams& p) {
-    if (stress_clear(Ff, tif, tjf, iA, rb, p)) return false;
+    if (stress_clear(Ff, tif, tjf, iA, rb, p.f_sc, p.f_st, p.f_ss)) return false;
     return bond_breaks_pairs(F, ti, tj, d.b_invA[small], d.b_rbI[small], p);
 }
 // The FP64 force mode's breakage decision behind the same FP32 screen.
@@ -1529,13 +1864,33 @@ static __device__ __noinline__ bool bond_breaks_d(const Vec3<double>& F, const V
     return bond_breaks(F, ti, tj, invA, rbI, p);
 }
 __device__ __forceinline__ bool bond_breaks_fp64(const Vec3<double>& F, const Vec3<double>& ti,
-                                                 const Vec3<double>& tj, const DemDev& d,
-                                                 int small, const SceneParams& p) {
+                                                 const Vec3<double>& tj, float iA, float rb,
+                                                 const DemDev& d, int small,
+                                                 const SceneParams& p) {
     const Vec3<float> Ff{d2f(F.x), d2f(F.y), d2f(F.z)};
     const Vec3<float> tif{d2f(ti.x), d2f(ti.y), d2f(ti.z)};
     const Vec3<float> tjf{d2f(tj.x), d2f(tj.y), d2f(tj.z)};
-    if (stress_clear(Ff, tif, tjf, d.bk32[small].w, d.rm32[small].x, p)) return false;
+    if (stress_clear(Ff, tif, tjf, iA, rb, p.f_sc, p.f_st, p.f_ss)) return false;
     return bond_breaks_d(F, ti, tj, d.b_invA[small], d.b_rbI[small], p);
+}
+
+// The breakage test of a bond between grains of a table scene behind the FP32
+// screen: the section's two FP64 divisions and the FP64 test run only for a
+// bond near one of its strengths.
+static __device__ __noinline__ bool bond_breaks_tab_d(const Vec3<double>& F, const Vec3<double>& ti,
+                                                      const Vec3<double>& tj, double A, double I,
+                                                      double rb, const PairConst& pc) {
+    return bond_breaks(F, ti, tj, __ddiv_rn(1.0, A), __ddiv_rn(rb, I), pc.sc, pc.st, pc.ss);
+}
+__device__ __forceinline__ bool bond_breaks_tab(const Vec3<double>& F, const Vec3<double>& ti,
+                                                const Vec3<double>& tj, float iA, float rbI,
+                                                double A, double I, double rb,
+                                                const PairConst& pc) {
+    const Vec3<float> Ff{d2f(F.x), d2f(F.y), d2f(F.z)};
+    const Vec3<float> tif{d2f(ti.x), d2f(ti.y), d2f(ti.z)};
+    const Vec3<float> tjf{d2f(tj.x), d2f(tj.y), d2f(tj.z)};
+    if (stress_clear(Ff, tif, tjf, iA, rbI, pc.f_sc, pc.f_st, pc.f_ss)) return false;
+    return bond_breaks_tab_d(F, ti, tj, A, I, rb, pc);
 }
 
 // FP32 hi/lo pair accumulator (hi + lo carries about 48 bits): (hi, lo) + x
@@ -1603,7 +1958,8 @@ __device__ __forceinline__ Vec3<float> rot_t32(const Frame32& R, Vec3<float> v) 
 // overlap's relative error at FP32 rounding even though L is FP32.
 __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
                                         const ContactSoA& w, const ContactSoA& o, int sidx, int c,
-                                        uint32_t fl, int i, int j, int sc, size_t cap) {
+                                        uint32_t fl, int i, int j, int sc, size_t cap,
+                                        bool report) {
     const double kix = d.px[i], kiy = d.py[i], kiz = d.pz[i];
     const double dxd = d.px[j] - kix, dyd = d.py[j] - kiy, dzd = d.pz[j] - kiz;
     const float dx = d2f(dxd), dy = d2f(dyd), dz = d2f(dzd);
@@ -1665,7 +2021,8 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
             fig = rot_t32(R, {-Ff.x, -Ff.y, -Ff.z});
             mi = rot_t32(R, {-tif.x, -tif.y, -tif.z});
             mj = rot_t32(R, {-tjf.x, -tjf.y, -tjf.z});
-            st3(w.f, CK, c, {kix + 0.5 * dxd, kiy + 0.5 * dyd, kiz + 0.5 * dzd});
+            if (report)
+                st3(w.f, CK, c, {kix + 0.5 * dxd, kiy + 0.5 * dyd, kiz + 0.5 * dzd});
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 pair_col(w, CF + q)[c] = Fp[q];
@@ -1684,7 +2041,7 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
         if (num > 0.0) atomicAdd(&d.sctr[sc].warn_gap, 1ull);
         const float ext = rmi.z - fabsf(gap);
         const Vec3<float> kri{ax * ext, ay * ext, az * ext};
-        st3(w.f, CK, c, {kix + f2d(kri.x), kiy + f2d(kri.y), kiz + f2d(kri.z)});
+        if (report) st3(w.f, CK, c, {kix + f2d(kri.x), kiy + f2d(kri.y), kiz + f2d(kri.z)});
         const Vec3<float> krj{kri.x - dx, kri.y - dy, kri.z - dz};
         const Vec3<float> wi{d2f(d.wx[i]), d2f(d.wy[i]), d2f(d.wz[i])};
         const Vec3<float> wj{d2f(d.wx[j]), d2f(d.wy[j]), d2f(d.wz[j])};
@@ -1724,9 +2081,11 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
         fig = rot_t32(R, {-F1, -F2, -F3});
         mi = cross3<float>(kri, fig);
         mj = cross3<float>(krj, {-fig.x, -fig.y, -fig.z});
-        pair_col(w, CF + 0)[c] = make_float2(F1, 0.0f);
-        pair_col(w, CF + 1)[c] = make_float2(F2, 0.0f);
-        pair_col(w, CF + 2)[c] = make_float2(F3, 0.0f);
+        if (report) {
+            pair_col(w, CF + 0)[c] = make_float2(F1, 0.0f);
+            pair_col(w, CF + 1)[c] = make_float2(F2, 0.0f);
+            pair_col(w, CF + 2)[c] = make_float2(F3, 0.0f);
+        }
         st3(w.f, CS, c, s);
     }
     float* cb = d.contrib32;
@@ -1741,172 +2100,214 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
     cb[8 * cap + c] = mj.z;
 }
 
-// `resolve_collision!` for one active contact (src/kernels.jl:136-313).  T is
-// the arithmetic type of the force model: double (DEM_FP64) or float
-// (DEM_FP32_FORCE).  Relative quantities (overlap, relative displacement and
-// rotation increments, relative velocity) are always formed in FP64 and then
-// cast; the accumulated bond force/torques, the shear displacement 𝐬 and the
-// bond-breakage test stay FP64 in both modes.
+// `resolve_collision!` for one active contact (src/kernels.jl:136-313): T =
+// double (DEM_FP64), or float (DEM_FP32_FORCE, force32).
 //
 // EBPM in sum/difference form: with 𝚫 = 𝐝ᵢ - 𝐝ⱼ = 𝐑(𝐯ᵢ - 𝐯ⱼ)dt,
 // 𝛉ₛ = 𝐑(𝛚ᵢ + 𝛚ⱼ)dt and 𝛉_d = 𝐑(𝛚ᵢ - 𝛚ⱼ)dt, the reference's increments
 // k₅𝛉ᵢ + k₆𝛉ⱼ and k₆𝛉ᵢ + k₅𝛉ⱼ are k₊𝛉ₛ ± k₋𝛉_d with k₊ = (k₅+k₆)/2 =
 // 3EI/L/(1+ϕ) and k₋ = (k₅-k₆)/2 = EI/L; dt is folded into the stiffnesses.
-// One contact, one thread: FP64 mode (T = double) or the FP32 force mode's
-// Hertz and bond paths (T = float, via force32).
+// One contact, one thread.  Each law loads everything it needs first, the
+// carried state and the bond section too, so that their latency runs beside
+// the frame's FP64 chain instead of after it.  What an FP64 thread spends is
+// FP64 instructions (64 cycles each on its SM sub-partition), so the forms
+// with the fewest are taken: 105 per bond (116 with the frame's f from s² and
+// the stiffnesses by way of ϕ), about 110 per Hertz contact (151 with
+// divisions by kₜ and |𝐅ₜ| and for R*, m*).
 // TAB: a scene with material and wall tables (FP64 only): the pair's
 // constants come from surfaces[midᵢ, midⱼ] and materials midᵢ, midⱼ, and the
 // bond section of rb = ρ·min(rᵢ, rⱼ) is formed here from that surface.
+__device__ __forceinline__ Frame pair_frame(Vec3<double> D, double L2, double invL,
+                                            const SceneParams& SP) {
+    return contact_frame(D.x, D.y, D.z, D.x * invL, D.y * invL, D.z * invL, SP);
+}
+__device__ __forceinline__ Vec3<double> sub3(Vec3<double> a, Vec3<double> b) {
+    return {a.x - b.x, a.y - b.y, a.z - b.z};
+}
+struct PairOut {
+    Vec3<double> F, mi, mj;  // force on i, moments on i and j
+};
+// EBPM (src/kernels.jl:170-239)
+template <bool TAB>
+__device__ __forceinline__ PairOut bond_one(const DemDev& d, const SceneParams& SP,
+                                            const ContactSoA& w, const ContactSoA& o, int sidx,
+                                            int c, int i, int j, int sc, const PairConst* pc,
+                                            bool report) {
+    const double ri = d.r[i], rj = d.r[j];
+    const Vec3<double> dk{d.px[j] - d.px[i], d.py[j] - d.py[i], d.pz[j] - d.pz[i]};
+    const Vec3<double> dv{d.vx[i] - d.vx[j], d.vy[i] - d.vy[j], d.vz[i] - d.vz[j]};
+    const Vec3<double> wi{d.wx[i], d.wy[i], d.wz[i]}, wj{d.wx[j], d.wy[j], d.wz[j]};
+    Vec3<double> Fi{0.0, 0.0, 0.0}, ti = Fi, tj = Fi;
+    if (sidx >= 0) {
+        Fi = ld3(o.f, CF, sidx);
+        ti = ld3(o.f, CTI, sidx);
+        tj = ld3(o.f, CTJ, sidx);
+    }
+    const int small = !less_nonneg(rj, ri) ? i : j;  // rb = ρ·min(rᵢ, rⱼ); radii > 0
+    // bond section (src/kernels.jl:178-184): per particle for the scene's one
+    // surface, per pair from the surface table
+    double b_phic, b_EI, b_EA, b_1pnu, b_A = 0.0, b_I = 0.0, b_rb = 0.0;
+    float f_invA, f_rbI;
+    if constexpr (TAB) {
+        const double rb = __dmul_rn(pc->ratio, small == i ? ri : rj);
+        const double rb2 = __dmul_rn(rb, rb);
+        b_A = __dmul_rn(rb2, kPi);
+        b_I = __dmul_rn(__dmul_rn(rb2, rb2), kPi / 4.0);
+        b_EA = __dmul_rn(pc->E, b_A);
+        b_EI = __dmul_rn(pc->E, b_I);
+        b_phic = __dmul_rn(__dmul_rn(20.0 / 3.0, __dadd_rn(1.0, pc->nu)), rb2);
+        b_1pnu = pc->inv1pnu;
+        b_rb = rb;
+        // FP32 section for the breakage screen, within a few roundings
+        const float fr = d2f(rb), fA = fr * fr * (float)kPi;
+        f_invA = 1.0f / fA;
+        f_rbI = 4.0f / (fA * fr);
+    } else {
+        b_phic = d.b_phic[small];
+        b_EI = d.b_EI[small];
+        b_EA = d.b_EA[small];
+        b_1pnu = SP.b_inv1pnu;
+        f_invA = d.bk32[small].w;
+        f_rbI = d.rm32[small].x;
+    }
+    const double L2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
+    const double invL = rsqrt(L2);
+    const Frame R = pair_frame(dk, L2, invL, SP);
+    const Vec3<double> D = rot<double>(R, dv);
+    const Vec3<double> Sv = rot<double>(R, {wi.x + wj.x, wi.y + wj.y, wi.z + wj.z});
+    const Vec3<double> Q = rot<double>(R, sub3(wi, wj));
+    // with ϕ = c/L² the factor 1/(L²(1 + ϕ)) is 1/(L² + c), so
+    // k₃dt = 6EI·dt/(L² + c), k₂dt = 2k₃dt/L, k₊dt = k₃dt·L/2 and
+    // k₋dt = EI·dt/L
+    const double idt = invL * SP.dt;
+    const double km = b_EI * idt;
+    const double k1 = b_EA * idt;
+    const double k3 = (b_EI * SP.dt6) * rcp_range(L2 + b_phic);
+    const double k2 = twice_exact(k3 * invL);
+    const double k4 = km * b_1pnu;
+    const double kp = half_exact(k3) * (L2 * invL);
+    const double ay_ = kp * Sv.y - k3 * D.z, az_ = kp * Sv.z + k3 * D.y;
+    const double dtix = k4 * Q.x;
+    Fi = {Fi.x + k1 * D.x, Fi.y + (k2 * D.y + k3 * Sv.z), Fi.z + (k2 * D.z - k3 * Sv.y)};
+    ti = {ti.x + dtix, ti.y + (ay_ + km * Q.y), ti.z + (az_ + km * Q.z)};
+    tj = {tj.x - dtix, tj.y + (ay_ - km * Q.y), tj.z + (az_ - km * Q.z)};
+    // breakage test, FP64 (src/kernels.jl:208-222)
+    bool broken;
+    if constexpr (TAB) broken = bond_breaks_tab(Fi, ti, tj, f_invA, f_rbI, b_A, b_I, b_rb, *pc);
+    else broken = bond_breaks_fp64(Fi, ti, tj, f_invA, f_rbI, d, small, SP);
+    if (broken) {
+        w.fl[c] = 0u;  // contact_active and contact_bonded bits cleared
+        atomicAdd(&d.sctr[sc].broken, 1ull);
+        return {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    }
+    st3(w.f, CF, c, Fi);
+    st3(w.f, CTI, c, ti);
+    st3(w.f, CTJ, c, tj);  // a bond's 𝐬 stays zero and is not stored
+    if (report)
+        st3(w.f, CK, c, {half_exact(d.px[i] + d.px[j]), half_exact(d.py[i] + d.py[j]),
+                         half_exact(d.pz[i] + d.pz[j])});
+    return {rot_t<double>(R, {-Fi.x, -Fi.y, -Fi.z}), rot_t<double>(R, {-ti.x, -ti.y, -ti.z}),
+            rot_t<double>(R, {-tj.x, -tj.y, -tj.z})};
+}
+// |𝐅ₜ| >= μF1 as the reference compares it
+static __device__ __noinline__ bool slides_exact(double n2, double muF1) { return sqrt(n2) >= muF1; }
+// The tangential force of a Hertz contact, with a particle or a wall
+// (src/kernels.jl:288-296, 398-408): F2, F3 in the contact frame, and the shear
+// history (0, sy, sz) of a sliding contact scaled back to μF1 = kₜ|𝐬|, which
+// is 𝐅ₜ/kₜ without the divisions.  The test |𝐅ₜ| >= μF1 is taken on the
+// squares (on the roots where those are zero, tiny or not finite).
+__device__ __forceinline__ void tangential(double sx, double& sy, double& sz, double kt, double gt,
+                                           double vcy, double vcz, double muF1, double& F2,
+                                           double& F3) {
+    const double Fx = -kt * sx, Fy = -kt * sy, Fz = -kt * sz;
+    const double n2 = Fx * Fx + Fy * Fy + Fz * Fz, m2 = muF1 * muF1;
+    // n2 and m2 are >= +0 or NaN; both ordinary (an exponent field in
+    // [64, 0x7fe]): compared as bit patterns, off the FP64 pipe
+    const unsigned en = (unsigned)__double2hiint(n2) - 0x04000000u;
+    const unsigned em = (unsigned)__double2hiint(m2) - 0x04000000u;
+    bool slide;
+    if (en < 0x7bf00000u && em < 0x7bf00000u)
+        slide = !less_nonneg(n2, m2) || __double2hiint(muF1) < 0;
+    else slide = slides_exact(n2, muF1);
+    if (slide) {
+        const double ratio = muF1 * rsqrt(n2);
+        F2 = ratio * Fy;
+        F3 = ratio * Fz;
+        sy *= -ratio;
+        sz *= -ratio;
+    } else {
+        F2 = Fy - gt * vcy;
+        F3 = Fz - gt * vcz;
+    }
+}
+// Hertz-Mindlin (src/kernels.jl:240-313)
+template <bool TAB>
+__device__ __forceinline__ PairOut hertz_one(const DemDev& d, const SceneParams& SP,
+                                             const ContactSoA& w, const ContactSoA& o, int sidx,
+                                             int c, int i, int j, int sc, const PairConst* pc,
+                                             bool report) {
+    const double ri = d.r[i], rj = d.r[j];
+    const Vec3<double> dk{d.px[j] - d.px[i], d.py[j] - d.py[i], d.pz[j] - d.pz[i]};
+    const Vec3<double> dv0{d.vx[j] - d.vx[i], d.vy[j] - d.vy[i], d.vz[j] - d.vz[i]};
+    const Vec3<double> wi{d.wx[i], d.wy[i], d.wz[i]}, wj{d.wx[j], d.wy[j], d.wz[j]};
+    Vec3<double> s{0.0, 0.0, 0.0};
+    if (sidx >= 0) s = ld3(o.f, CS, sidx);
+    const double mi = d.m[i], mj = d.m[j];
+    const double L2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
+    const double invL = rsqrt(L2);
+    const double L = L2 * invL;
+    const Frame R = pair_frame(dk, L2, invL, SP);
+    const double gap = L - ri - rj;
+    if (positive_bits(gap)) atomicAdd(&d.sctr[sc].warn_gap, 1ull);
+    const double dn = fabs(gap), ext = (ri - dn) * invL;
+    const Vec3<double> kri{dk.x * ext, dk.y * ext, dk.z * ext};
+    if (report) st3(w.f, CK, c, {d.px[i] + kri.x, d.py[i] + kri.y, d.pz[i] + kri.z});
+    const Vec3<double> krj = sub3(kri, dk);
+    const Vec3<double> wci = cross3<double>(wi, kri), wcj = cross3<double>(wj, krj);
+    const Vec3<double> vc = rot<double>(R, {dv0.x + (wcj.x - wci.x), dv0.y + (wcj.y - wci.y),
+                                            dv0.z + (wcj.z - wci.z)});
+    const double sq = sqrt(ri * rj * rcp_range(ri + rj) * dn);  // √(R*·|gap|)
+    const double pYs = TAB ? pc->Ys : SP.pp_Ys, pGs = TAB ? pc->Gs : SP.pp_Gs;
+    const double pcgn = TAB ? pc->cgn : SP.pp_cgn, pcgt = TAB ? pc->cgt : SP.pp_cgt;
+    const double kn = (4.0 / 3.0 * pYs) * sq, kt = (8.0 * pGs) * sq;
+    const double root = sqrt(mi * mj * rcp_range(mi + mj) * sq);  // √(m*·√(R*·|gap|))
+    const double gn = pcgn * root, gt = pcgt * root;
+    if (__double2hiint(gn) < 0 || __double2hiint(gt) < 0) {
+        const int neg = (gn < 0.0) + (gt < 0.0);
+        if (neg) atomicAdd(&d.sctr[sc].warn_damp, (unsigned long long)neg);
+    }
+    // (0·vc.x adds nothing to the normal component unless it is not finite)
+    s = {(__double2hiint(vc.x) & 0x7ff00000) != 0x7ff00000 ? s.x : s.x + vc.x * 0.0, s.y + vc.y * SP.dt, s.z + vc.z * SP.dt};
+    const double F1 = -kn * gap - gn * vc.x;
+    double F2, F3;
+    tangential(s.x, s.y, s.z, kt, gt, vc.y, vc.z, (TAB ? pc->mu : SP.pp_mu) * F1, F2, F3);
+    st3(w.f, CS, c, s);
+    if (report) st3(w.f, CF, c, {F1, F2, F3});
+    const Vec3<double> F = rot_t<double>(R, {-F1, -F2, -F3});
+    return {F, cross3<double>(kri, F), cross3<double>(krj, {-F.x, -F.y, -F.z})};
+}
 template <typename T, bool TAB = false>
 __device__ __forceinline__ void contact_one(const DemDev& d, const SceneParams& SP,
-                                            const ContactSoA& w, const ContactSoA& o, int c,
-                                            uint32_t fl, int i, int j, int sc, size_t cap) {
-    const int sidx = w.src[c];  // carried state in the other buffer (-1: new, zero)
+                                            const ContactSoA& w, const ContactSoA& o, int sidx,
+                                            int c, uint32_t fl, int i, int j, int sc, size_t cap,
+                                            bool report) {
     if constexpr (std::is_same<T, float>::value) {
-        force32(d, SP, w, o, sidx, c, fl, i, j, sc, cap);
+        force32(d, SP, w, o, sidx, c, fl, i, j, sc, cap, report);
         return;
     }
     const PairConst* pc = nullptr;
     if constexpr (TAB) pc = &d.mt->pair[d.mid[i] * d.mt->nmat + d.mid[j]];
-    const double dt = SP.dt;
-    const Vec3<double> ki{d.px[i], d.py[i], d.pz[i]}, kj{d.px[j], d.py[j], d.pz[j]};
-    const double ri = d.r[i], rj = d.r[j];
-    const Vec3<double> vi{d.vx[i], d.vy[i], d.vz[i]}, vj{d.vx[j], d.vy[j], d.vz[j]};
-    const Vec3<double> wi{d.wx[i], d.wy[i], d.wz[i]}, wj{d.wx[j], d.wy[j], d.wz[j]};
-    const double dx = kj.x - ki.x, dy = kj.y - ki.y, dz = kj.z - ki.z;
-    const double L2 = dx * dx + dy * dy + dz * dz;
-    const double invL = rsqrt(L2);
-    const double L = L2 * invL;
-    const double ax = dx * invL, ay = dy * invL, az = dz * invL;
-    const Frame R = contact_frame(dx, dy, dz, ax, ay, az, SP);
-    Vec3<T> fig, mi, mj;
-    if (fl & kBonded) {
-        // EBPM (src/kernels.jl:170-239)
-        const Vec3<double> Dd = rot<double>(R, {vi.x - vj.x, vi.y - vj.y, vi.z - vj.z});
-        const Vec3<double> Ts = rot<double>(R, {wi.x + wj.x, wi.y + wj.y, wi.z + wj.z});
-        const Vec3<double> Td = rot<double>(R, {wi.x - wj.x, wi.y - wj.y, wi.z - wj.z});
-        const Vec3<T> D = from_d<T>(Dd), Sv = from_d<T>(Ts), Q = from_d<T>(Td);
-        const int small = !less_nonneg(rj, ri) ? i : j;  // rb = ρ·min(rᵢ, rⱼ); radii > 0
-        // bond section (src/kernels.jl:178-184): per particle for the scene's
-        // one surface, per pair from the surface table
-        double b_phic, b_EI, b_EA, b_1pnu, b_invA = 0.0, b_rbI = 0.0;
-        if constexpr (TAB) {
-            const double rb = __dmul_rn(pc->ratio, d.r[small]);
-            const double rb2 = __dmul_rn(rb, rb);
-            const double Ab = __dmul_rn(rb2, kPi);
-            const double Ib = __dmul_rn(__dmul_rn(rb2, rb2), kPi / 4.0);
-            b_EA = __dmul_rn(pc->E, Ab);
-            b_EI = __dmul_rn(pc->E, Ib);
-            b_phic = __dmul_rn(__dmul_rn(20.0 / 3.0, __dadd_rn(1.0, pc->nu)), rb2);
-            b_1pnu = pc->inv1pnu;
-            b_invA = __ddiv_rn(1.0, Ab);
-            b_rbI = __ddiv_rn(rb, Ib);
-        } else {
-            b_phic = d.b_phic[small];
-            b_EI = d.b_EI[small];
-            b_EA = d.b_EA[small];
-            b_1pnu = SP.b_inv1pnu;
-        }
-        const T tinvL = (T)invL, tdt = (T)dt;
-        const T phi = (T)b_phic * tinvL * tinvL;
-        const T iphi = rcp_nr((T)1.0 + phi);  // 1/(1 + ϕ)
-        const T EILdt = (T)b_EI * tinvL * tdt;  // EI/L·dt
-        const T k1 = (T)b_EA * tinvL * tdt;
-        const T k3 = (T)6.0 * EILdt * tinvL * iphi;
-        const T k2 = (T)2.0 * k3 * tinvL;
-        const T k4 = EILdt * (T)b_1pnu;
-        const T kp = (T)3.0 * EILdt * iphi;
-        const T km = EILdt;
-        const T dFx = k1 * D.x, dFy = k2 * D.y + k3 * Sv.z, dFz = k2 * D.z - k3 * Sv.y;
-        const T ay_ = -k3 * D.z + kp * Sv.y, az_ = k3 * D.y + kp * Sv.z;
-        const T dtix = k4 * Q.x, dtiy = ay_ + km * Q.y, dtiz = az_ + km * Q.z;
-        const T dtjx = -k4 * Q.x, dtjy = ay_ - km * Q.y, dtjz = az_ - km * Q.z;
-        const Vec3<double> z3{0.0, 0.0, 0.0};
-        Vec3<double> Fi = sidx >= 0 ? ld3(o.f, CF, sidx) : z3;
-        Vec3<double> ti = sidx >= 0 ? ld3(o.f, CTI, sidx) : z3;
-        Vec3<double> tj = sidx >= 0 ? ld3(o.f, CTJ, sidx) : z3;
-        Fi = {Fi.x + (double)dFx, Fi.y + (double)dFy, Fi.z + (double)dFz};
-        ti = {ti.x + (double)dtix, ti.y + (double)dtiy, ti.z + (double)dtiz};
-        tj = {tj.x + (double)dtjx, tj.y + (double)dtjy, tj.z + (double)dtjz};
-        // breakage test, FP64 (src/kernels.jl:208-222)
-        bool broken;
-        if constexpr (TAB) broken = bond_breaks_tab(Fi, ti, tj, b_invA, b_rbI, *pc);
-        else broken = bond_breaks_fp64(Fi, ti, tj, d, small, SP);
-        if (broken) {
-            w.fl[c] = 0u;  // contact_active and contact_bonded bits cleared
-            atomicAdd(&d.sctr[sc].broken, 1ull);
-            fig = {(T)0, (T)0, (T)0};
-            mi = fig;
-            mj = fig;
-        } else {
-            fig = from_d<T>(rot_t<double>(R, {-Fi.x, -Fi.y, -Fi.z}));
-            mi = from_d<T>(rot_t<double>(R, {-ti.x, -ti.y, -ti.z}));
-            mj = from_d<T>(rot_t<double>(R, {-tj.x, -tj.y, -tj.z}));
-            st3(w.f, CK, c, {half_exact(ki.x + kj.x), half_exact(ki.y + kj.y),
-                             half_exact(ki.z + kj.z)});
-            st3(w.f, CF, c, Fi);
-            st3(w.f, CTI, c, ti);
-            st3(w.f, CTJ, c, tj);  // a bond's 𝐬 stays zero and is not stored
-        }
-    } else {
-        // Hertz-Mindlin (src/kernels.jl:240-313)
-        const double gap = L - ri - rj;
-        if (gap > 0) atomicAdd(&d.sctr[sc].warn_gap, 1ull);
-        const double ext = ri - fabs(gap);
-        st3(w.f, CK, c, {ki.x + ax * ext, ki.y + ay * ext, ki.z + az * ext});
-        const Vec3<T> kri{(T)(ax * ext), (T)(ay * ext), (T)(az * ext)};
-        const Vec3<T> krj{kri.x - (T)dx, kri.y - (T)dy, kri.z - (T)dz};
-        const Vec3<T> wci = cross3<T>(from_d<T>(wi), kri);
-        const Vec3<T> wcj = cross3<T>(from_d<T>(wj), krj);
-        const Vec3<T> dv{(T)(vj.x - vi.x) + (wcj.x - wci.x), (T)(vj.y - vi.y) + (wcj.y - wci.y),
-                         (T)(vj.z - vi.z) + (wcj.z - wci.z)};
-        const Vec3<T> vc = rot<T>(R, dv);
-        const T tri = (T)ri, trj = (T)rj, tmi = (T)d.m[i], tmj = (T)d.m[j];
-        const T Rs = tri * trj / (tri + trj);
-        const T ms = tmi * tmj / (tmi + tmj);
-        const T tgap = (T)gap;
-        const T sq = sqrt(Rs * (T)fabs(gap));
-        const double pYs = TAB ? pc->Ys : SP.pp_Ys, pGs = TAB ? pc->Gs : SP.pp_Gs;
-        const double pcgn = TAB ? pc->cgn : SP.pp_cgn, pcgt = TAB ? pc->cgt : SP.pp_cgt;
-        const double pmu = TAB ? pc->mu : SP.pp_mu;
-        const T kn = (T)(4.0 / 3.0 * pYs) * sq;
-        const T kt = (T)(8.0 * pGs) * sq;
-        const T root = sqrt(ms * sq);
-        const T gn = (T)pcgn * root;
-        const T gt = (T)pcgt * root;
-        if (gn < (T)0 || gt < (T)0)
-            atomicAdd(&d.sctr[sc].warn_damp, (unsigned long long)((gn < (T)0) + (gt < (T)0)));
-        Vec3<double> s = sidx >= 0 ? ld3(o.f, CS, sidx) : Vec3<double>{0.0, 0.0, 0.0};
-        s = {s.x + (double)vc.x * 0.0, s.y + (double)vc.y * dt, s.z + (double)vc.z * dt};
-        const T F1 = -kn * tgap - gn * vc.x;
-        const Vec3<T> Ft{-kt * (T)s.x, -kt * (T)s.y, -kt * (T)s.z};
-        const T nFt = sqrt(Ft.x * Ft.x + Ft.y * Ft.y + Ft.z * Ft.z);
-        const T muF1 = (T)pmu * F1;
-        T F2, F3;
-        if (nFt >= muF1) {
-            const T ratio = muF1 / nFt;
-            F2 = ratio * Ft.y;
-            F3 = ratio * Ft.z;
-            s = {s.x, (double)(F2 / kt), (double)(F3 / kt)};
-        } else {
-            F2 = Ft.y - gt * vc.y;
-            F3 = Ft.z - gt * vc.z;
-        }
-        fig = rot_t<T>(R, {-F1, -F2, -F3});
-        mi = cross3<T>(kri, fig);
-        mj = cross3<T>(krj, {-fig.x, -fig.y, -fig.z});
-        st3(w.f, CF, c, {(double)F1, (double)F2, (double)F3});
-        st3(w.f, CS, c, s);
-    }
-    d.contrib[0 * cap + c] = (double)fig.x;
-    d.contrib[1 * cap + c] = (double)fig.y;
-    d.contrib[2 * cap + c] = (double)fig.z;
-    d.contrib[3 * cap + c] = (double)mi.x;
-    d.contrib[4 * cap + c] = (double)mi.y;
-    d.contrib[5 * cap + c] = (double)mi.z;
-    d.contrib[6 * cap + c] = (double)mj.x;
-    d.contrib[7 * cap + c] = (double)mj.y;
-    d.contrib[8 * cap + c] = (double)mj.z;
+    const PairOut f = (fl & kBonded) ? bond_one<TAB>(d, SP, w, o, sidx, c, i, j, sc, pc, report)
+                                     : hertz_one<TAB>(d, SP, w, o, sidx, c, i, j, sc, pc, report);
+    d.contrib[0 * cap + c] = f.F.x;
+    d.contrib[1 * cap + c] = f.F.y;
+    d.contrib[2 * cap + c] = f.F.z;
+    d.contrib[3 * cap + c] = f.mi.x;
+    d.contrib[4 * cap + c] = f.mi.y;
+    d.contrib[5 * cap + c] = f.mi.z;
+    d.contrib[6 * cap + c] = f.mj.x;
+    d.contrib[7 * cap + c] = f.mj.y;
+    d.contrib[8 * cap + c] = f.mj.z;
 }
 
 // With bonds and other contacts both present, threads take the contacts in
@@ -1917,8 +2318,17 @@ __device__ __forceinline__ void contact_one(const DemDev& d, const SceneParams& 
 // whatever the number of active lanes.  With one type only, thread t takes
 // contact t (no list read).  The list entry of a thread's next contact is
 // read one iteration ahead, so that its latency overlaps the current one.
-template <typename T, bool MULTI, bool TAB = false>
-__device__ __forceinline__ void force_body(const DemDev& d, const DemParams& p, int nxt) {
+// This thread takes items t0, t0 + stride, ... (t0 and stride keep a warp's
+// lanes consecutive).
+// `report`: the contacts' points and the Hertz contacts' forces are stored (a
+// step whose contacts nobody can read before the next step leaves them out).
+// LATE: the incoming-list entry is written after the force, so that a warp on
+// its own does not wait for the atomic's slot (k_steps); with many warps in
+// flight the earlier write is the faster one (256 scenes, 1.3 M contacts:
+// force pass 213 us, late 254 us).  Returns the number of items.
+template <typename T, bool MULTI, bool TAB, bool LATE>
+__device__ __forceinline__ int force_body(const DemDev& d, const DemParams& p, int nxt, int t0,
+                                          int stride, bool report) {
     const RowCounter a = d.ctr->alloc[nxt];
     const int C = min((int)a.rows, p.cap);
     const int NB = min((int)a.bonds, C);
@@ -1927,9 +2337,8 @@ __device__ __forceinline__ void force_body(const DemDev& d, const DemParams& p, 
     const int total = mixed ? NBw + (C - NB) : C;
     const ContactSoA w = d.c[nxt];
     const ContactSoA o = d.c[nxt ^ 1];
-    const int stride = gridDim.x * blockDim.x;
     const size_t cap = (size_t)p.cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
+    for (int t = t0; t < total; t += stride) {
         int c = t;
         if (mixed) {
             if (t >= NB && t < NBw) continue;  // padding up to the warp boundary
@@ -1938,31 +2347,43 @@ __device__ __forceinline__ void force_body(const DemDev& d, const DemParams& p, 
         }
         const uint32_t fl = w.fl[c];
         const int i = w.ci[c], j = w.cj[c];
+        const int sidx = w.src[c];  // carried state in the other buffer (-1: new, zero)
         const int sc = slot_scene<MULTI>(d, i);
         if (MULTI && (sc < 0 || d.sp[sc].mode != kModeStep)) continue;
         // the contact in its partner's incoming list (the integrator's gather
         // sorts the list by owner, so the order of registration is free)
-        add_incoming_entry(d, p, j, c, i);
-        contact_one<T, TAB>(d, scene_rec<MULTI>(d, p, sc), w, o, c, fl, i, j, sc, cap);
+        const int slot = atomicAdd(&d.in_cnt[j], 1);
+        auto enlist = [&]() {
+            if (slot < p.kin) d.in_list[(size_t)j * p.kin + slot] = make_int2(c, i);
+            else raise_error(d.ctr, kErrCapacity);
+        };
+        if (!LATE) enlist();
+        contact_one<T, TAB>(d, scene_rec<MULTI>(d, p, sc), w, o, sidx, c, fl, i, j, sc, cap,
+                            report);
+        if (LATE) enlist();
     }
+    return total;
 }
 
 // The force pass with the compiler's register choice, and with a budget for
 // four 256-thread blocks per SM (an autotuner choice for the FP32 mode).
 template <typename T, bool MULTI>
-__global__ void __launch_bounds__(kThreads) k_force(DemDev d, DemParams p, int nxt) {
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 3) k_force(DemDev d, DemParams p, int nxt) {
     dep_begin(p.dep == 2);
-    force_body<T, MULTI>(d, p, nxt);
+    force_body<T, MULTI, false, false>(d, p, nxt, blockIdx.x * blockDim.x + threadIdx.x,
+                                 gridDim.x * blockDim.x, p.report != 0);
 }
 template <typename T, bool MULTI>
 __global__ void __launch_bounds__(kThreads, 4) k_force4(DemDev d, DemParams p, int nxt) {
     dep_begin(p.dep == 2);
-    force_body<T, MULTI>(d, p, nxt);
+    force_body<T, MULTI, false, false>(d, p, nxt, blockIdx.x * blockDim.x + threadIdx.x,
+                                 gridDim.x * blockDim.x, p.report != 0);
 }
 // a single scene with material and wall tables (FP64)
-__global__ void __launch_bounds__(kThreads) k_force_tab(DemDev d, DemParams p, int nxt) {
+__global__ void __launch_bounds__(kThreads, 2) k_force_tab(DemDev d, DemParams p, int nxt) {
     dep_begin(p.dep == 2);
-    force_body<double, false, true>(d, p, nxt);
+    force_body<double, false, true, false>(d, p, nxt, blockIdx.x * blockDim.x + threadIdx.x,
+                                 gridDim.x * blockDim.x, p.report != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -2151,10 +2572,13 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
                                    __dmul_rn(z, W.wn[2]));
     const double L = __dsub_rn(dotkn, W.wd);
     if (fabs(L) < r) {
+        // touching, so gap = |L| - r < 0 and |gap| = r - |L|: the contact
+        // point -L/|L|·(|L| + |gap|/2)·n is -sign(L)·(|L| + r)/2·n
         const double gap = fabs(L) - r;
-        const double dn = fabs(gap);
-        const double lsc = (fabs(L) + dn / 2.0) / fabs(L);
-        const double kix = -L * W.wn[0] * lsc, kiy = -L * W.wn[1] * lsc, kiz = -L * W.wn[2] * lsc;
+        const double dn = -gap;
+        const double h = 0.5 * (fabs(L) + r);
+        const double hs = L > 0.0 ? -h : (L < 0.0 ? h : CUDART_NAN);  // L/|L| of a centre on the wall
+        const double kix = hs * W.wn[0], kiy = hs * W.wn[1], kiz = hs * W.wn[2];
         const double vcix = wy * kiz - wz * kiy + vx, vciy = wz * kix - wx * kiz + vy,
                      vciz = wx * kiy - wy * kix + vz;
         const double* Rw = W.wR;
@@ -2167,23 +2591,14 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
         const double root = sqrt(m * sq);
         const double gn = W.cgn * root;
         const double gt = W.cgt * root;
-        if (count && gn < 0) atomicAdd(&d.sctr[sc].warn_damp, 1ull);
-        if (count && gt < 0) atomicAdd(&d.sctr[sc].warn_damp, 1ull);
+        if (count && (__double2hiint(gn) < 0 || __double2hiint(gt) < 0)) {
+            const int neg = (gn < 0.0) + (gt < 0.0);
+            if (neg) atomicAdd(&d.sctr[sc].warn_damp, (unsigned long long)neg);
+        }
         double sx = *wsx + vcx * 0.0, sy = *wsy + vcy * dt, sz = *wsz + vcz * dt;
         const double F1 = -kn * gap - gn * vcx;
-        const double Ftx = -kt * sx, Fty = -kt * sy, Ftz = -kt * sz;
-        const double nFt = sqrt(Ftx * Ftx + Fty * Fty + Ftz * Ftz);
         double F2, F3;
-        if (nFt >= W.mu * F1) {
-            const double ratio = W.mu * F1 / nFt;
-            F2 = ratio * Fty;
-            F3 = ratio * Ftz;
-            sy = F2 / kt;
-            sz = F3 / kt;
-        } else {
-            F2 = Fty - gt * vcy;
-            F3 = Ftz - gt * vcz;
-        }
+        tangential(sx, sy, sz, kt, gt, vcy, vcz, W.mu * F1, F2, F3);
         const double* Ri = W.wRinv;
         const double gx = -(Ri[0] * F1 + Ri[1] * F2 + Ri[2] * F3);
         const double gy = -(Ri[3] * F1 + Ri[4] * F2 + Ri[5] * F3);
@@ -2222,40 +2637,12 @@ __device__ __forceinline__ void wall_contact(const DemDev& d, int sc, const Wall
     }
 }
 
-// The fused download of an exchanged step (HostOut): the armed step count
-// as this launch sees it (0 for arena kernels and unarmed handles; every
-// block of a launch reads the same value, since it changes only after all
-// of them have counted themselves out).
-template <bool MULTI>
-__device__ __forceinline__ int host_out_left(const DemDev& d) {
-    if constexpr (MULTI) return 0;
-    else return __ldcg(&d.ctr->hout.steps_left);
-}
-// One thread per block, after the block's records are written (`wrote`) or
-// at any point (an integrator that writes none): the last block of the
-// launch disarms one step and, after the last armed step's records, copies
-// the device error word (no integrator raises one) to the host.
-__device__ __forceinline__ void host_out_count(const DemDev& d, int left, bool wrote) {
-    HostOut& H = d.ctr->hout;
-    __threadfence();
-    if (atomicAdd(&H.done, 1u) != gridDim.x - 1) return;
-    __threadfence();
-    if (left == 1 && wrote) *H.err = __ldcg(&d.ctr->error);
-    H.done = 0u;
-    H.steps_left = left - 1;
-}
-
-template <bool MULTI, bool F32, bool TAB = false>
+// QUAT: with the quaternions (otherwise k_list1 has updated them)
+template <bool MULTI, bool F32, bool TAB, bool QUAT>
 __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams& p, int cur) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nxt = cur ^ 1;
     if (i == 0) d.ctr->alloc[cur] = RowCounter{0u, 0u};  // the free buffer is next step's target
-    // an armed handle's step: this layout writes no records (the host reads
-    // the state the usual way), it only counts the launch
-    if (!MULTI && threadIdx.x == 0) {
-        const int left = host_out_left<MULTI>(d);
-        if (left > 0) host_out_count(d, left, false);
-    }
     // the end-of-step rebuild-flag work of every scene (see scene_flags_one):
     // it only ORs into the next flags, as the particles' skin test does
     for (int s = i; s < p.ns; s += gridDim.x * blockDim.x) scene_flags_one<MULTI>(d, p, cur, s);
@@ -2274,40 +2661,17 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     const double wx = d.wx[i], wy = d.wy[i], wz = d.wz[i];
     const double r = d.r[i], m = d.m[i];
     const double invm = d.inv_m[i], ii = d.inv_inertia[i];
-    const double qw = d.qw[i], qx = d.qx[i], qy = d.qy[i], qz = d.qz[i];
+    const uint32_t qword = d.qmask[i >> 5];
+    const bool turned = QUAT && ((qword >> lane_id()) & 1u);
+    double q4[4] = {0.0, 0.0, 0.0, 0.0};
+    if (turned) {
+        q4[0] = d.qw[i];
+        q4[1] = d.qx[i];
+        q4[2] = d.qy[i];
+        q4[3] = d.qz[i];
+    }
     const float4 p32 = d.pos32[i], xr = d.xref[i];
     const float r32 = d.rm32[i].z;
-    // 𝐪 + Δ𝐪 with Δ𝐪 = ½ 𝛚 ⊗ 𝐪 (no dt, as the reference), the ½ folded into
-    // 𝛚, as explicit FMA chains.  With 𝛚 = (+0, +0, +0) each fma(a, +0, c)
-    // (a finite) returns c unless c is -0, so for a finite 𝐪 without a -0
-    // component the chains return 𝐪 itself: a particle that does not spin
-    // skips them, with identical results.  The normalisation always runs.
-    // A spinless particle with the identity orientation (1, +0, +0, +0)
-    // keeps it: |𝐪|² = 1 exactly, rsqrt(1) = 1 (checked by
-    // dem_selftest_conversions) and 𝐪·1 = 𝐪, so nothing is computed or stored.
-    auto update_quaternion = [&]() {
-        double nw = qw, nx = qx, ny = qy, nz = qz;
-        const bool spinless = (__double_as_longlong(wx) | __double_as_longlong(wy) |
-                               __double_as_longlong(wz)) == 0ll;
-        const bool identity = spinless && __double_as_longlong(qw) == 0x3ff0000000000000ll &&
-                              (__double_as_longlong(qx) | __double_as_longlong(qy) |
-                               __double_as_longlong(qz)) == 0ll;
-        if (!identity) {
-            if (!(spinless && finite_not_negzero(qw) && finite_not_negzero(qx) &&
-                  finite_not_negzero(qy) && finite_not_negzero(qz))) {
-                const double hx = half_exact(wx), hy = half_exact(wy), hz = half_exact(wz);
-                nw = __fma_rn(-qz, hz, __fma_rn(-qy, hy, __fma_rn(-qx, hx, qw)));
-                nx = __fma_rn(-qz, hy, __fma_rn(qy, hz, __fma_rn(qw, hx, qx)));
-                ny = __fma_rn(qz, hx, __fma_rn(qx, hz, __fma_rn(qw, hy, qy)));
-                nz = __fma_rn(-qy, hx, __fma_rn(qx, hy, __fma_rn(qw, hz, qz)));
-            }
-            const double inq = rsqrt(__fma_rn(nz, nz, __fma_rn(ny, ny, __fma_rn(nx, nx, nw * nw))));
-            d.qw[i] = nw * inq;
-            d.qx[i] = nx * inq;
-            d.qy[i] = ny * inq;
-            d.qz[i] = nz * inq;
-        }
-    };
     double F[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
     if constexpr (F32) {
         float Ff[3] = {0.0f, 0.0f, 0.0f}, Mf[3] = {0.0f, 0.0f, 0.0f};
@@ -2386,7 +2750,7 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     d.vx[i] = vx + ax * dt;
     d.vy[i] = vy + ay * dt;
     d.vz[i] = vz + az * dt;
-    update_quaternion();
+    bool spin = turned && update_quaternion(d, i, wx, wy, wz, q4[0], q4[1], q4[2], q4[3]);
     // 𝛚 + 𝐌·I⁻¹dt: with 𝐌 = (+0, +0, +0) and a finite I⁻¹dt, fma(+0, I⁻¹dt, w)
     // is w unless w is -0, so a torque-free particle keeps its stored spin
     const bool torque_free = (__double_as_longlong(M[0]) | __double_as_longlong(M[1]) |
@@ -2394,16 +2758,31 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     if (!(torque_free && product_finite(ii, dt) && not_negzero(wx) && not_negzero(wy) &&
           not_negzero(wz))) {
         const double iidt = ii * dt;
-        d.wx[i] = __fma_rn(M[0], iidt, wx);
-        d.wy[i] = __fma_rn(M[1], iidt, wy);
-        d.wz[i] = __fma_rn(M[2], iidt, wz);
+        const double w0 = __fma_rn(M[0], iidt, wx), w1 = __fma_rn(M[1], iidt, wy),
+                     w2 = __fma_rn(M[2], iidt, wz);
+        d.wx[i] = w0;
+        d.wy[i] = w1;
+        d.wz[i] = w2;
+        spin |= (__double_as_longlong(w0) | __double_as_longlong(w1) | __double_as_longlong(w2)) != 0ll;
+    } else {
+        spin |= (__double_as_longlong(wx) | __double_as_longlong(wy) | __double_as_longlong(wz)) != 0ll;
     }
-    d.fx[i] = F[0];
-    d.fy[i] = F[1];
-    d.fz[i] = F[2];
-    d.tx[i] = M[0];
-    d.ty[i] = M[1];
-    d.tz[i] = M[2];
+    {
+        // the quaternion bits of the warp's slots: cleared where nothing was
+        // updated (QUAT), set where a spin will turn the particle
+        const unsigned am = __activemask();
+        const unsigned on = __ballot_sync(am, spin), looked = __ballot_sync(am, QUAT);
+        const uint32_t next = (qword & ~looked) | on;
+        if (lane_id() == (unsigned)(__ffs(am) - 1) && next != qword) d.qmask[i >> 5] = next;
+    }
+    if (p.report) {  // nobody can read the totals of a step inside a call
+        d.fx[i] = F[0];
+        d.fy[i] = F[1];
+        d.fz[i] = F[2];
+        d.tx[i] = M[0];
+        d.ty[i] = M[1];
+        d.tz[i] = M[2];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2462,17 +2841,20 @@ __device__ __forceinline__ void gather_component(const DemDev& d, const DemParam
 #pragma unroll
     for (int u = 0; u < 4; ++u) v4[u] = u < nin ? il[u] : make_int2(0, 0x7fffffff);
     const int c1 = min(c0 + len, p.cap);
-    int c = c0;
-    for (; c + 1 < c1; c += 2) {
-        const T a0 = cf[c], a1 = cmi[c], b0 = cf[c + 1], b1 = cmi[c + 1];
-        F += a0;
-        M += a1;
-        F += b0;
-        M += b1;
-    }
-    if (c < c1) {
-        F += cf[c];
-        M += cmi[c];
+    for (int c = c0; c < c1; c += 4) {  // four entries' loads at a time
+        T a[4], m[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c + u < c1) {
+                a[u] = cf[c + u];
+                m[u] = cmi[c + u];
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c + u < c1) {
+                F += a[u];
+                M += m[u];
+            }
     }
     if (nin <= 4) {
         add_incoming_component<T, 4>(cf, cmj, v4, nin, F, M);
@@ -2500,41 +2882,95 @@ __device__ __forceinline__ void gather_component(const DemDev& d, const DemParam
     }
 }
 
-template <bool MULTI, bool F32, bool TAB = false>
-__device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams& p, int cur) {
-    constexpr int NW = TAB ? kMaxWalls : 1;
-    __shared__ double s_wall[NW][6][32];  // each wall's force and moment on each particle
-    __shared__ uint8_t s_touch[NW][32];
-    __shared__ float s_pos[3][32];        // the new FP32 position components
-    // an armed single-scene step: the new state of the block's particles, as
-    // rows of the output records (HostOut), and the first armed step's
-    // orientations and first-wall shear histories read from the caller's
-    __shared__ double s_out[MULTI ? 1 : kHostOutRows][32];
-    __shared__ uint8_t s_chg[MULTI ? 1 : kHostOutRows][32];  // value differs from the input
-    __shared__ double s_in[MULTI ? 1 : 7][32];
-    // 0, 1, 2: component; 3: walls and quaternion.  The roles rotate with
-    // the block's round over the SMs: warp w of a block runs on SM
-    // sub-partition w, and blocks are placed one per SM in turn (blocks b,
-    // b + sms, b + 2·sms, ... share an SM), so rotating by b / sms gives the
-    // blocks on one SM different sub-partitions for their wall and
-    // quaternion warp, the one with the most FP64 instructions (a rotation by
-    // b mod 4 would not: the SM count, 152, is a multiple of 4)
-    const int q = ((int)(threadIdx.x >> 5) - (int)((blockIdx.x / (unsigned)max(p.sms, 1)) & 3u) -
-                   1) & 3;
-    const int l = (int)lane_id();
-    const int i = blockIdx.x * 32 + l;
-    const int nxt = cur ^ 1;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int left = host_out_left<MULTI>(d);
-    const bool out = !MULTI && left == 1;  // this launch writes the caller's records
-    const double* qin = nullptr;           // this launch reads these from the caller's
-    const double* wsin = nullptr;
-    if (!MULTI && left > 0 && left == __ldcg(&d.ctr->hout.steps_total)) {
-        qin = d.ctr->hout.qin;
-        wsin = d.ctr->hout.wsin;
+// resolve_wall! of wall wl for particle i of scene sc (wall_force)
+template <bool TAB>
+__device__ __forceinline__ bool particle_wall(const DemDev& d, const DemParams& p,
+                                              const SceneParams& S, int i, int sc, int wl, double wx,
+                                              double wy, double wz, double g[3], double mw[3]) {
+    size_t o = i;
+    WallK K;
+    if constexpr (TAB) {
+        const MatTables& T = *d.mt;
+        const int a = d.mid[i];
+        const WallConst& W = T.wall[wl];
+        K = WallK{W.wn, W.wd, W.wR, W.wRinv, W.f_wn, W.f_wc0, W.mu[a], W.Ys[a], W.Gs[a],
+                  W.cgn[a], W.cgt[a]};
+        o = (size_t)wl * p.wstride + i;
+    } else {
+        K = WallK{S.wn, S.wd, S.wR, S.wRinv, S.f_wn, S.f_wc0, S.pw_mu, S.pw_Ys, S.pw_Gs,
+                  S.pw_cgn, S.pw_cgt};
     }
-    if (t == 0) d.ctr->alloc[cur] = RowCounter{0u, 0u};  // the free buffer is next step's target
-    for (int s2 = t; s2 < p.ns; s2 += gridDim.x * blockDim.x) scene_flags_one<MULTI>(d, p, cur, s2);
+    return wall_force(d, sc, K, S.dt, d.pos32[i], d.rm32[i].z, d.px[i], d.py[i], d.pz[i], d.vx[i],
+                      d.vy[i], d.vz[i], wx, wy, wz, d.r[i], d.m[i], d.wsx + o, d.wsy + o,
+                      d.wsz + o, g, mw, true);
+}
+
+// k_steps: the walls of the 32 particles [32u, 32u + 32) by one warp, in the
+// force phase (the walls depend on the step's starting state only, and the
+// warps that have no contacts to compute are free then; a wall contact's
+// chain, about 90 FP64 instructions, was the longest of the integration).
+// Leaves the touching walls as a bit mask, their forces and moments, and
+// which components of the first wall's shear history changed.
+template <bool TAB>
+__device__ __forceinline__ void wall_items(const DemDev& d, const DemParams& p, int u) {
+    const int i = u * 32 + (int)lane_id();
+    if (i >= p.n) return;
+    const SceneParams& S = p.s0;
+    const int nwall = TAB ? d.mt->nwall : (S.has_wall ? 1 : 0);
+    const double wx = d.wx[i], wy = d.wy[i], wz = d.wz[i];
+    unsigned touch = 0u, chg = 0u;
+    for (int wl = 0; wl < nwall; ++wl) {
+        const double before[3] = {d.wsx[i], d.wsy[i], d.wsz[i]};
+        double g[3], mw[3];
+        if (particle_wall<TAB>(d, p, S, i, 0, wl, wx, wy, wz, g, mw)) {
+            touch |= 1u << wl;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                d.wforce[(size_t)(6 * wl + c) * p.wstride + i] = g[c];
+                d.wforce[(size_t)(6 * wl + 3 + c) * p.wstride + i] = mw[c];
+            }
+        }
+        if (wl == 0) {
+            const double after[3] = {d.wsx[i], d.wsy[i], d.wsz[i]};
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                chg |= __double_as_longlong(after[c]) != __double_as_longlong(before[c]) ? 1u << c : 0u;
+        }
+    }
+    d.wtouch[i] = (uint8_t)touch;
+    d.wchg[i] = (uint8_t)chg;
+}
+
+// Shared memory of one group of four warps.  FUSED (k_steps): with the staging
+// of the exchange's output, and without the walls' forces, which wall_items
+// has left in memory.
+template <bool TAB, bool FUSED>
+struct SplitShared {
+    static constexpr int NW = FUSED ? 1 : (TAB ? kMaxWalls : 1);
+    double wall[FUSED ? 1 : NW][FUSED ? 1 : 6][32];  // each wall's force and moment on each particle
+    double out[FUSED ? kHostOutRows : 1][32];   // the new state, as rows of the output records
+    float pos[3][32];                           // the new FP32 position components
+    uint8_t touch[NW][32];
+    uint8_t chg[FUSED ? kHostOutRows : 1][32];  // value differs from the step's input
+};
+// The particles [32u, 32u + 32) by four warps: q is the calling warp's role
+// (0, 1, 2: component; 3: walls and quaternion), tq its thread's index among
+// the four warps, which meet at block barrier `bar`.  FUSED: the walls' forces
+// come from wall_items; H (may be null): this step also writes the new state
+// into the caller's records; `report`: the force and moment totals are stored
+// (a step whose totals nobody can read before the next one leaves them out).
+template <bool MULTI, bool F32, bool TAB, bool FUSED>
+__device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams& p, int cur, int u,
+                                                int q, int tq, int bar,
+                                                SplitShared<TAB, FUSED>& sh, const HostOut* H,
+                                                bool report) {
+    auto meet = [bar]() {
+        asm volatile("barrier.sync %0, %1;" ::"r"(bar), "r"(kSplitThreads) : "memory");
+    };
+    const int l = (int)lane_id();
+    const int i = u * 32 + l;
+    const int nxt = cur ^ 1;
+    const bool out = FUSED && H != nullptr;
     // every thread reaches both barriers; `live`: a particle of a stepping scene
     const bool exists = i < p.n;
     int sc = 0;
@@ -2555,6 +2991,8 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             m = d.m[i];
             invm = d.inv_m[i];
             ii = d.inv_inertia[i];
+            uint8_t tch = 0;
+            if constexpr (FUSED) tch = d.wtouch[i];
             if constexpr (F32) {
                 float Ff = 0.0f, Mf = 0.0f;
                 gather_component<float>(d, p, i, row0, rlen, nin, q, Ff, Mf);
@@ -2563,21 +3001,14 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             } else {
                 gather_component<double>(d, p, i, row0, rlen, nin, q, Fq, Mq);
             }
-        }
-    }
-    if constexpr (!MULTI) {
-        if (q == 3 && (qin || wsin)) {
-            // the block's 32 particles are one contiguous range of each
-            // record array: consecutive lanes read it, then each lane its own
-            const int i0 = blockIdx.x * 32, m = min(32, p.n - i0);
-            if (qin)
-                for (int e = l; e < 4 * m; e += 32) s_in[e & 3][e >> 2] = qin[(size_t)4 * i0 + e];
-            if (wsin)
-                for (int e = l; e < 3 * m; e += 32) {
-                    const int pq = e / 3;
-                    s_in[4 + e - 3 * pq][pq] = wsin[(size_t)3 * i0 + e];
+            if constexpr (FUSED) {
+                for (int wl = 0; tch; ++wl, tch >>= 1) {  // the touching walls, in order
+                    if (!(tch & 1)) continue;
+                    const double* wf = d.wforce + (size_t)(6 * wl + q) * p.wstride + i;
+                    Fq += wf[0];
+                    Mq += wf[(size_t)3 * p.wstride];
                 }
-            __syncwarp();
+            }
         }
     }
     // warp 3: the step's starting spin, for the walls now and the quaternion
@@ -2587,80 +3018,37 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
         wx = d.wx[i];
         wy = d.wy[i];
         wz = d.wz[i];
-        bool qhost = false;
-        if constexpr (!MULTI) {
-            if (qin) {
-                qw = s_in[0][l];
-                qx = s_in[1][l];
-                qy = s_in[2][l];
-                qz = s_in[3][l];
-                qhost = true;
-            }
-            if (wsin) {  // the first wall's shear history, for wall_force below
-                d.wsx[i] = s_in[4][l];
-                d.wsy[i] = s_in[5][l];
-                d.wsz[i] = s_in[6][l];
-            }
-        }
-        if (!qhost) {
-            qw = d.qw[i];  // loaded here: their latency hides behind the walls
-            qx = d.qx[i];
-            qy = d.qy[i];
-            qz = d.qz[i];
-        }
-        const double x = d.px[i], y = d.py[i], z = d.pz[i];
-        const double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-        const double r = d.r[i];
-        const float4 p32 = d.pos32[i];
-        const float r32 = d.rm32[i].z;
-        const double dt = S.dt;
+        qw = d.qw[i];  // loaded here: their latency hides behind the walls
+        qx = d.qx[i];
+        qy = d.qy[i];
+        qz = d.qz[i];
         // resolve_wall!: each wall's force and moment, added by the component
         // warps in wall order
-        for (int wl = 0; wl < nwall; ++wl) {
-            size_t o = i;
-            WallK K;
-            if constexpr (TAB) {
-                const MatTables& T = *d.mt;
-                const int a = d.mid[i];
-                const WallConst& W = T.wall[wl];
-                K = WallK{W.wn, W.wd, W.wR, W.wRinv, W.f_wn, W.f_wc0, W.mu[a], W.Ys[a], W.Gs[a],
-                          W.cgn[a], W.cgt[a]};
-                o = (size_t)wl * p.wstride + i;
-            } else {
-                K = WallK{S.wn, S.wd, S.wR, S.wRinv, S.f_wn, S.f_wc0, S.pw_mu, S.pw_Ys, S.pw_Gs,
-                          S.pw_cgn, S.pw_cgt};
-            }
-            double g[3], mw[3];
-            if (out && wl == 0) {  // the first wall's shear history before the step
-                s_out[19][l] = d.wsx[o];
-                s_out[20][l] = d.wsy[o];
-                s_out[21][l] = d.wsz[o];
-            }
-            const bool touch = wall_force(d, sc, K, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz,
-                                          r, d.m[i], d.wsx + o, d.wsy + o, d.wsz + o, g, mw, true);
-            s_touch[wl][l] = touch ? 1 : 0;
-            if (touch) {
+        if constexpr (!FUSED) {
+            for (int wl = 0; wl < nwall; ++wl) {
+                double g[3], mw[3];
+                const bool touch = particle_wall<TAB>(d, p, S, i, sc, wl, wx, wy, wz, g, mw);
+                sh.touch[wl][l] = touch ? 1 : 0;
+                if (touch) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s_wall[wl][c][l] = g[c];
-                    s_wall[wl][3 + c][l] = mw[c];
+                    for (int c = 0; c < 3; ++c) {
+                        sh.wall[wl][c][l] = g[c];
+                        sh.wall[wl][3 + c][l] = mw[c];
+                    }
                 }
             }
         }
-        if (out) {  // the first wall's shear history as this thread left it
+        if (out) {  // the first wall's shear history, and what wall_items changed of it
             const double* ws[3] = {d.wsx, d.wsy, d.wsz};
+            const unsigned chg = d.wchg[i];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double v = ws[c][i];
-                // without walls nothing changed it (the value before the
-                // step is not staged then)
-                s_chg[19 + c][l] = nwall > 0 && __double_as_longlong(v) !=
-                                                    __double_as_longlong(s_out[19 + c][l]);
-                s_out[19 + c][l] = v;
+                sh.chg[19 + c][l] = (chg >> c) & 1u;
+                sh.out[19 + c][l] = ws[c][i];
             }
         }
     }
-    __syncthreads();  // walls in shared memory; every component thread has read in_cnt
+    meet();  // walls in shared memory; every component thread has read in_cnt
     if (q == 3 && exists) d.in_cnt[i] = 0;
     // the quaternion (integrate_body's update, from the starting spin) runs
     // while the component warps update the position, velocity and spin
@@ -2690,29 +3078,26 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             d.qx[i] = ox;
             d.qy[i] = oy;
             d.qz[i] = oz;
-        } else if (qin) {  // read from the caller's: the columns still hold the old ones
-            d.qw[i] = ow;
-            d.qx[i] = ox;
-            d.qy[i] = oy;
-            d.qz[i] = oz;
         }
         if (out) {
-            s_out[9][l] = ow;
-            s_out[10][l] = ox;
-            s_out[11][l] = oy;
-            s_out[12][l] = oz;
-            s_chg[9][l] = __double_as_longlong(ow) != __double_as_longlong(qw);
-            s_chg[10][l] = __double_as_longlong(ox) != __double_as_longlong(qx);
-            s_chg[11][l] = __double_as_longlong(oy) != __double_as_longlong(qy);
-            s_chg[12][l] = __double_as_longlong(oz) != __double_as_longlong(qz);
+            sh.out[9][l] = ow;
+            sh.out[10][l] = ox;
+            sh.out[11][l] = oy;
+            sh.out[12][l] = oz;
+            sh.chg[9][l] = __double_as_longlong(ow) != __double_as_longlong(qw);
+            sh.chg[10][l] = __double_as_longlong(ox) != __double_as_longlong(qx);
+            sh.chg[11][l] = __double_as_longlong(oy) != __double_as_longlong(qy);
+            sh.chg[12][l] = __double_as_longlong(oz) != __double_as_longlong(qz);
         }
     }
     if (q < 3 && live) {
         const double dt = S.dt;
-        for (int wl = 0; wl < nwall; ++wl) {
-            if (s_touch[wl][l]) {
-                Fq += s_wall[wl][q][l];
-                Mq += s_wall[wl][3 + q][l];
+        if constexpr (!FUSED) {
+            for (int wl = 0; wl < nwall; ++wl) {
+                if (sh.touch[wl][l]) {
+                    Fq += sh.wall[wl][q][l];
+                    Mq += sh.wall[wl][3 + q][l];
+                }
             }
         }
         // apply_body_force!
@@ -2728,7 +3113,7 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
         const double hdt2 = S.hdt2;
         const double pq1 = xq + vq * dt + aq * hdt2;
         pick3(q, d.px, d.py, d.pz)[i] = pq1;
-        s_pos[q][l] = d2f(pq1 - S.dmin[q]);
+        sh.pos[q][l] = d2f(pq1 - S.dmin[q]);
         const double vq1 = vq + aq * dt;
         pick3(q, d.vx, d.vy, d.vz)[i] = vq1;
         // 𝛚 + 𝐌·I⁻¹dt; with Mq = +0, a finite I⁻¹dt and wq not -0 the sum
@@ -2738,22 +3123,24 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             wq1 = __fma_rn(Mq, ii * dt, wq);
             pick3(q, d.wx, d.wy, d.wz)[i] = wq1;
         }
-        pick3(q, d.fx, d.fy, d.fz)[i] = Fq;
-        pick3(q, d.tx, d.ty, d.tz)[i] = Mq;
+        if (report) {
+            pick3(q, d.fx, d.fy, d.fz)[i] = Fq;
+            pick3(q, d.tx, d.ty, d.tz)[i] = Mq;
+        }
         if (out) {
-            s_out[q][l] = pq1;
-            s_out[3 + q][l] = vq1;
-            s_out[6 + q][l] = wq1;
-            s_out[13 + q][l] = Fq;
-            s_out[16 + q][l] = Mq;
-            s_chg[q][l] = __double_as_longlong(pq1) != __double_as_longlong(xq);
-            s_chg[3 + q][l] = __double_as_longlong(vq1) != __double_as_longlong(vq);
-            s_chg[6 + q][l] = __double_as_longlong(wq1) != __double_as_longlong(wq);
+            sh.out[q][l] = pq1;
+            sh.out[3 + q][l] = vq1;
+            sh.out[6 + q][l] = wq1;
+            sh.out[13 + q][l] = Fq;
+            sh.out[16 + q][l] = Mq;
+            sh.chg[q][l] = __double_as_longlong(pq1) != __double_as_longlong(xq);
+            sh.chg[3 + q][l] = __double_as_longlong(vq1) != __double_as_longlong(vq);
+            sh.chg[6 + q][l] = __double_as_longlong(wq1) != __double_as_longlong(wq);
         }
     }
-    __syncthreads();  // the new position components (and an armed step's rows) in shared memory
+    meet();  // the new position components (and the output rows) in shared memory
     if (q == 3 && live) {
-        const float fx = s_pos[0][l], fy = s_pos[1][l], fz = s_pos[2][l];
+        const float fx = sh.pos[0][l], fy = sh.pos[1][l], fz = sh.pos[2][l];
         d.pos32[i] = make_float4(fx, fy, fz, reach32(fx, fy, fz, d.rm32[i].z));
         const bool moved = S.f_half_skin > 0.0f && left_skin(S, fx, fy, fz, d.xref[i]);
         const unsigned am = __activemask();
@@ -2761,62 +3148,240 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
         if (moved && lane_id() == (unsigned)(__ffs(peers) - 1) && d.sflags[nxt][sc] == 0u)
             atomicOr(&d.sflags[nxt][sc], 1u);
     }
-    if constexpr (!MULTI) {
-        if (left > 0) {
-            if (out) {
-                // the block's 32 particles are one contiguous range of each
-                // record array: k·32 values, written by consecutive threads
-                const int i0 = blockIdx.x * 32, m = min(32, p.n - i0);
-                const unsigned same = d.ctr->hout.same;
-                int row = 0;
+    if constexpr (FUSED) {
+        if (out) {
+            // the 32 particles are one contiguous range of each record array:
+            // k·32 values, written by consecutive threads
+            const int i0 = u * 32, m = min(32, p.n - i0);
+            const unsigned same = H->same;
+            int row = 0;
 #pragma unroll
-                for (int f = 0; f < kHostOutFields; ++f) {
-                    const int k = f == 3 ? 4 : 3;
-                    double* rec = d.ctr->hout.rec[f];
-                    const bool keep = (same >> f) & 1u;  // unchanged values are there already
-                    if (rec) {
-                        for (int e = threadIdx.x; e < k * 32; e += kSplitThreads) {
-                            const int pq = e / k, r = row + e - pq * k;
-                            if (pq < m && (!keep || s_chg[r][pq])) rec[(size_t)k * i0 + e] = s_out[r][pq];
-                        }
+            for (int f = 0; f < kHostOutFields; ++f) {
+                const int k = f == 3 ? 4 : 3;
+                double* rec = H->rec[f];
+                const bool keep = (same >> f) & 1u;  // unchanged values are there already
+                if (rec) {
+                    for (int e = tq; e < k * 32; e += kSplitThreads) {
+                        const int pq = e / k, r = row + e - pq * k;
+                        if (pq < m && (!keep || sh.chg[r][pq]))
+                            rec[(size_t)k * i0 + e] = sh.out[r][pq];
                     }
-                    row += k;
                 }
+                row += k;
             }
-            __syncthreads();
-            if (threadIdx.x == 0) host_out_count(d, left, out);
+            meet();  // the next round's staging waits for these reads
         }
     }
+}
+
+// One block of four warps per 32 particles.  The roles rotate with the block's
+// round over the SMs: warp w of a block runs on SM sub-partition w, and blocks
+// are placed one per SM in turn (blocks b, b + sms, b + 2·sms, ... share an
+// SM), so rotating by b / sms gives the blocks on one SM different
+// sub-partitions for their wall and quaternion warp, the one with the most
+// FP64 instructions (a rotation by b mod 4 would not: the SM count, 152, is a
+// multiple of 4)
+template <bool MULTI, bool F32, bool TAB>
+__device__ __forceinline__ void integrate_split_block(const DemDev& d, const DemParams& p, int cur) {
+    __shared__ SplitShared<TAB, false> sh;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) d.ctr->alloc[cur] = RowCounter{0u, 0u};  // the free buffer is next step's target
+    for (int s2 = t; s2 < p.ns; s2 += gridDim.x * blockDim.x) scene_flags_one<MULTI>(d, p, cur, s2);
+    const int q = ((int)(threadIdx.x >> 5) - (int)((blockIdx.x / (unsigned)max(p.sms, 1)) & 3u) -
+                   1) & 3;
+    integrate_split<MULTI, F32, TAB, false>(d, p, cur, (int)blockIdx.x, q, (int)threadIdx.x, 0, sh,
+                                            nullptr, true);
 }
 
 // The integrator with the compiler's register choice (FP64 force mode), and
 // in the FP32 force mode with a budget for three 256-thread blocks per SM:
 // its FP64 work per particle is small enough that more resident warps hide
 // the state loads better than the extra registers would.
-template <bool MULTI, bool F32>
+template <bool MULTI, bool QUAT>
 __global__ void __launch_bounds__(kThreads) k_integrate(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
-    integrate_body<MULTI, F32>(d, p, cur);
+    integrate_body<MULTI, false, false, QUAT>(d, p, cur);
 }
+template <bool QUAT>
 __global__ void __launch_bounds__(kThreads) k_integrate_tab(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
-    integrate_body<false, false, true>(d, p, cur);
+    integrate_body<false, false, true, QUAT>(d, p, cur);
 }
-template <bool MULTI>
+template <bool MULTI, bool QUAT>
 __global__ void __launch_bounds__(kThreads, 3) k_integrate3(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
-    integrate_body<MULTI, true>(d, p, cur);
+    integrate_body<MULTI, true, false, QUAT>(d, p, cur);
 }
 // four warps per 32 particles (integrate_split)
 template <bool MULTI, bool F32>
 __global__ void __launch_bounds__(kSplitThreads) k_integrate_split(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
-    integrate_split<MULTI, F32>(d, p, cur);
+    integrate_split_block<MULTI, F32, false>(d, p, cur);
 }
 __global__ void __launch_bounds__(kSplitThreads) k_integrate_split_tab(DemDev d, DemParams p,
                                                                        int cur) {
     dep_begin(p.dep == 2);
-    integrate_split<false, false, true>(d, p, cur);
+    integrate_split_block<false, false, true>(d, p, cur);
+}
+
+// ---------------------------------------------------------------------------
+// Whole steps of a small or medium scene in one cooperative launch (dem_step,
+// dem_step_exchange): contact update, forces and integration of `nsteps`
+// steps, each phase the device code of the separate kernels, with a grid
+// barrier between phases.
+//
+// What bounds such a scene is latency: each phase is a chain of dependent
+// loads and FP64 instructions (63 cycles each, whatever else the SM does) on
+// a few warps per SM sub-partition.  As three kernels per step each phase
+// also paid a launch (a three-kernel graph takes 4.1 us per step with nothing
+// in its kernels), cold instruction and parameter caches and a placement of
+// blocks that the hardware chooses; here a phase boundary is a 1.05 us
+// barrier, and work goes to the warps in rounds over the SMs: chunk k of 32
+// contacts to warp k / blocks of block k mod blocks, so that every SM
+// sub-partition gets its share of the FP64 chains.
+//
+// Block size: 128 threads (one warp per sub-partition) while four lanes per
+// particle need no more warps than that, then 256, then 512 with one block
+// per SM; a small scene so leaves SMs (and registers) to other streams.
+//
+// IO (dem_step_exchange): the first step reads the particle state from the
+// caller's arrays, the positions by all warps (the contact update waits for
+// them), the other fields by a quarter of the warps while the others update
+// the contacts; the last step's integrator writes the state into the
+// caller's arrays as each group of 32 particles is done.
+//
+// Only the last step's contact points, Hertz forces and particle totals are
+// stored (report_last): the caller of several steps cannot read the others'.
+constexpr int kStepThreads = 512;
+
+// positions: 32 particles per warp, through shared memory (96 values of it),
+// with the FP32 position and the skin test of k_refresh_pos32
+__device__ __forceinline__ void read_positions(const DemDev& d, const DemParams& p, int cur,
+                                               const double* src, double* buf) {
+    const int l = (int)lane_id();
+    const int w = (int)(threadIdx.x >> 5);
+    const SceneParams& S = p.s0;
+    for (int c = w * (int)gridDim.x + (int)blockIdx.x; c * 32 < p.n;
+         c += (int)gridDim.x * (int)(blockDim.x >> 5)) {
+        const int base = c * 32, m = min(32, p.n - base);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (l + 32 * k < 3 * m) buf[l + 32 * k] = src[(size_t)3 * base + l + 32 * k];
+        __syncwarp();
+        if (l < m) {
+            const int i = base + l;
+            const double x = buf[3 * l], y = buf[3 * l + 1], z = buf[3 * l + 2];
+            d.px[i] = x;
+            d.py[i] = y;
+            d.pz[i] = z;
+            const float fx = d2f(x - S.dmin[0]), fy = d2f(y - S.dmin[1]), fz = d2f(z - S.dmin[2]);
+            d.pos32[i] = make_float4(fx, fy, fz, reach32(fx, fy, fz, d.rm32[i].z));
+            if ((!(S.f_half_skin > 0.0f) || left_skin(S, fx, fy, fz, d.xref[i])) &&
+                __ldcg(&d.sflags[cur][0]) == 0u)
+                atomicOr(&d.sflags[cur][0], 1u);
+        }
+        __syncwarp();
+    }
+}
+// the other fields, by warps [w0, warps of the block): every load of 32
+// particles is issued before the first store
+__device__ __forceinline__ void read_rest(const DemDev& d, const DemParams& p, const StepIO& io,
+                                          int w0) {
+    const int l = (int)lane_id();
+    const int nw = (int)(blockDim.x >> 5) - w0;
+    double* const col[4][4] = {{d.vx, d.vy, d.vz, nullptr},
+                               {d.wx, d.wy, d.wz, nullptr},
+                               {d.qw, d.qx, d.qy, d.qz},
+                               {d.wsx, d.wsy, d.wsz, nullptr}};
+    for (int c = ((int)(threadIdx.x >> 5) - w0) * (int)gridDim.x + (int)blockIdx.x; c * 32 < p.n;
+         c += (int)gridDim.x * nw) {
+        const int base = c * 32, m = min(32, p.n - base);
+        double v[4][4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            constexpr int K[4] = {3, 3, 4, 3};
+#pragma unroll
+            for (int k = 0; k < K[f]; ++k) {
+                v[f][k] = 0.0;
+                if (io.in[1 + f] && l + 32 * k < K[f] * m)
+                    v[f][k] = io.in[1 + f][(size_t)K[f] * base + l + 32 * k];
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            constexpr int K[4] = {3, 3, 4, 3};
+            if (!io.in[1 + f]) continue;
+#pragma unroll
+            for (int k = 0; k < K[f]; ++k) {
+                const int e = l + 32 * k, q = e / K[f], comp = e - K[f] * q;
+                double* dst = comp == 0 ? col[f][0]
+                                        : (comp == 1 ? col[f][1] : (comp == 2 ? col[f][2] : col[f][3]));
+                if (e < K[f] * m) dst[base + q] = v[f][k];
+            }
+        }
+    }
+}
+
+template <typename T, bool TAB>
+__global__ void __launch_bounds__(kStepThreads, 1)
+    k_steps(const __grid_constant__ DemDev d, const __grid_constant__ DemParams p, int cur0,
+            int nsteps, int report_last, const __grid_constant__ StepIO io) {
+    using Split = SplitShared<TAB, true>;
+    extern __shared__ __align__(16) unsigned char raw[];
+    __shared__ int fail;
+    const int nt = (int)blockDim.x;
+    // the contact update's and the integration's shared memory take turns
+    unsigned long long* red = reinterpret_cast<unsigned long long*>(raw);
+    DetectShared* det = reinterpret_cast<DetectShared*>(red + nt / 32);
+    ListShared* lst = reinterpret_cast<ListShared*>(det + nt / kLanes);
+    Split* split = reinterpret_cast<Split*>(raw);
+    if (threadIdx.x == 0) fail = 0;  // the first barrier orders this before any read of it
+    if (__ldcg(&d.ctr->error) & kErrTimeout) return;  // an earlier launch's barrier gave up
+    const Team all{nt, 0, &fail};
+    const int w = (int)(threadIdx.x >> 5);
+    const int t0 = (w * (int)gridDim.x + (int)blockIdx.x) * 32 + (int)lane_id();
+    for (int s = 0; s < nsteps; ++s) {
+        const int cur = (cur0 + s) & 1, nxt = cur ^ 1;
+        Team team = all;
+        if (io.has_in && s == 0) {
+            read_positions(d, p, cur, io.in[0], reinterpret_cast<double*>(raw) + 96 * w);
+            if (!grid_sync(d.ctr, all)) return;
+            team.nt = nt - nt / 4;
+            team.bar = 1;
+            if ((int)threadIdx.x >= team.nt) read_rest(d, p, io, team.nt / 32);
+        }
+        if ((int)threadIdx.x < team.nt) {
+            if (__ldcg(&d.sflags[cur][0]) != 0u)
+                search_phases<false, false>(d, p, cur, 0, team, det, lst, red);
+            else
+                list_phase<false>(d, p, cur, lst, team.nt);
+        }
+        if (!grid_sync(d.ctr, all)) return;
+        const bool last = s == nsteps - 1, report = last && report_last;
+        {
+            const int total = force_body<T, false, TAB, true>(d, p, nxt, t0, (int)gridDim.x * nt,
+                                                              report);
+            // the walls go to the warps after those of the last contacts
+            const int W = (int)gridDim.x * (nt / 32), items = (total + 31) / 32;
+            int u = t0 / 32 - items % W;
+            for (u = u < 0 ? u + W : u; u * 32 < p.n; u += W) wall_items<TAB>(d, p, u);
+        }
+        if (!grid_sync(d.ctr, all)) return;
+        if (t0 == 0) {
+            d.ctr->alloc[cur] = RowCounter{0u, 0u};  // the free buffer is next step's target
+            scene_flags_one<false>(d, p, cur, 0);
+            // no integrator raises an error
+            if (io.has_out && last) *io.out.err = __ldcg(&d.ctr->error);
+        }
+        const int quad = w >> 2;
+        int round = 0;
+        for (int u = quad * (int)gridDim.x + (int)blockIdx.x; u * 32 < p.n;
+             u += (int)gridDim.x * (nt / kSplitThreads), ++round)
+            integrate_split<false, std::is_same<T, float>::value, TAB, true>(
+                d, p, cur, u, (w - quad - round) & 3, (int)threadIdx.x & (kSplitThreads - 1),
+                2 + quad, split[quad], io.has_out && last ? &io.out : nullptr, report);
+        if (!last && !grid_sync(d.ctr, all)) return;
+    }
 }
 
 // ---- inspection kernels (dem_debug_broadphase) -------------------------------
@@ -2982,15 +3547,82 @@ void launch_search_b(const DemDev& d, const DemParams& p, int cur, bool init, bo
 void launch_search(const DemDev& d, const DemParams& p, int cur, bool init, bool multi, bool all,
                    const LaunchShape& sh, cudaStream_t s) {
     if (p.n == 0) return;
+    if (!init && !multi && !all && narrow_list(p.n, p.sms, p.list_lanes))
+        launch(p.dep != 0, k_list1, blocks_for(p.n, kThreads), kThreads, s, d, p, cur,
+               split_integrator(sh, p.n, p.sms) ? 0 : 1);
     if (sh.detect_blocks_per_sm == 3) launch_search_b<3>(d, p, cur, init, multi, all, s);
     else launch_search_b<4>(d, p, cur, init, multi, all, s);
+}
+
+namespace {
+size_t steps_shared(int threads, bool tab) {
+    const size_t search = sizeof(unsigned long long) * (size_t)(threads / 32) +
+                          sizeof(DetectShared) * (size_t)(threads / kLanes) +
+                          sizeof(ListShared) * (size_t)(threads / kVLanes);
+    const size_t split = (size_t)(threads / kSplitThreads) *
+                         (tab ? sizeof(SplitShared<true, true>) : sizeof(SplitShared<false, true>));
+    return std::max(std::max(search, split), sizeof(double) * 96 * (size_t)(threads / 32));
+}
+using StepsKernel = void (*)(DemDev, DemParams, int, int, int, StepIO);
+StepsKernel steps_kernel(const DemParams& p) {
+    if (p.tab) return k_steps<double, true>;
+    return p.precision == 1 ? k_steps<float, false> : k_steps<double, false>;
+}
+// the block size for a scene of n particles (k_steps's comment)
+void steps_shape(int n, int sms, int* grid, int* threads) {
+    const int warps = max(1, blocks_for((long long)n * kVLanes, 32));
+    *threads = warps <= 4 * sms ? 128 : (warps <= 8 * sms ? 256 : kStepThreads);
+    *grid = *threads == 128 ? blocks_for(warps, 4) : sms;
+}
+}  // namespace
+
+bool steps_ready(const DemParams& p) {
+    int grid, threads;
+    steps_shape(p.n, p.sms, &grid, &threads);
+    for (StepsKernel k : {(StepsKernel)k_steps<double, true>, (StepsKernel)k_steps<double, false>,
+                          (StepsKernel)k_steps<float, false>}) {
+        const bool tab = k == (StepsKernel)k_steps<double, true>;
+        int nb = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)steps_shared(kStepThreads, tab)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads,
+                                                          steps_shared(threads, tab)) != cudaSuccess ||
+            nb < 1) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
+}
+
+cudaError_t launch_steps(const DemDev& d, const DemParams& p, int cur, int nsteps, bool report,
+                         const StepIO& io, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    int grid, threads;
+    steps_shape(p.n, p.sms, &grid, &threads);
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = steps_shared(threads, p.tab != 0);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, steps_kernel(p), d, p, cur, nsteps, report ? 1 : 0, io);
 }
 
 void launch_force(const DemDev& d, const DemParams& p, int nxt, bool multi, const LaunchShape& sh,
                   cudaStream_t s) {
     if (p.n == 0 || p.cap == 0) return;
     const int block = clamp_block(sh.force_block);
-    const int grid = min(blocks_for(p.cap, block), max(sh.force_grid, 1));
+    // at most the blocks that are resident together (the kernels' register
+    // budgets): a last wave of a few blocks would have the grid's stride run
+    // on mostly idle SMs (256 scenes, 1.3 M contacts, 768 threads per SM
+    // resident: 2,432 blocks of 256 216 us, 456 175 us)
+    const int per_sm = p.precision == 1 ? (sh.force_blocks_per_sm == 4 ? 1024 : 768) : 512;
+    const int grid = min(min(blocks_for(p.cap, block), max(sh.force_grid, 1)),
+                         p.sms * max(per_sm / block, 1));
     if (p.precision == 1) {
         // FP32 mode: register budget for 3 (default) or 4 blocks of 256 per SM
         if (sh.force_blocks_per_sm == 4)
@@ -3010,6 +3642,9 @@ void launch_force(const DemDev& d, const DemParams& p, int nxt, bool multi, cons
 void launch_integrate(const DemDev& d, const DemParams& p, int cur, bool multi,
                       const LaunchShape& sh, cudaStream_t s) {
     if (p.n == 0) return;
+    // k_list1 has updated the quaternions (the split layout's four-lane list
+    // update of a forced shape has not)
+    const bool quat = multi || !narrow_list(p.n, p.sms, p.list_lanes);
     const int block = clamp_block(sh.integrate_block);
     if (split_integrator(sh, p.n, p.sms)) {
         const int nb = blocks_for(p.n, 32);
@@ -3026,13 +3661,18 @@ void launch_integrate(const DemDev& d, const DemParams& p, int cur, bool multi,
     }
     const int nb = blocks_for(p.n, block);
     if (p.tab)
-        launch(p.dep != 0, k_integrate_tab, nb, block, s, d, p, cur);
+        launch(p.dep != 0, quat ? k_integrate_tab<true> : k_integrate_tab<false>, nb, block, s, d,
+               p, cur);
     else if (p.precision == 1)
-        launch(p.dep != 0, multi ? k_integrate3<true> : k_integrate3<false>, nb, block, s, d, p,
-               cur);
+        launch(p.dep != 0,
+               multi ? (quat ? k_integrate3<true, true> : k_integrate3<true, false>)
+                     : (quat ? k_integrate3<false, true> : k_integrate3<false, false>),
+               nb, block, s, d, p, cur);
     else
-        launch(p.dep != 0, multi ? k_integrate<true, false> : k_integrate<false, false>, nb, block,
-               s, d, p, cur);
+        launch(p.dep != 0,
+               multi ? (quat ? k_integrate<true, true> : k_integrate<true, false>)
+                     : (quat ? k_integrate<false, true> : k_integrate<false, false>),
+               nb, block, s, d, p, cur);
 }
 
 // Active entries of a slot's row (its contacts (i, j), j > i, sorted by j).
@@ -3230,8 +3870,10 @@ void launch_selftest_conv(long long n, unsigned long long seed, unsigned long lo
 // block 0's wait must give up after `spin_limit` polls (kErrTimeout) and
 // return.  Launched cooperatively, so both blocks are resident.
 __global__ void k_selftest_barrier(DevCounters* c, int missing, unsigned long long spin_limit) {
+    __shared__ int fail;
     if (missing && blockIdx.x == 1) return;
-    grid_sync(c, spin_limit);
+    if (threadIdx.x == 0) fail = 0;
+    grid_sync(c, Team{(int)blockDim.x, 0, &fail}, spin_limit);
 }
 
 cudaError_t launch_selftest_wait(int which, int missing, unsigned long long spin_limit,
@@ -3303,8 +3945,7 @@ void launch_refresh_pos32(const DemDev& d, const DemParams& p, bool multi, int f
 // Small blocks put a 17,576-particle scene on every SM.  REFRESH (an upload
 // to a single-scene handle, field `posf` the positions): the FP32 position
 // and the skin test of each slot, from the uploaded values, as
-// k_refresh_pos32 does; with x.arm, it also arms the fused download
-// (HostOut) of the exchanged step that follows.
+// k_refresh_pos32 does.
 constexpr int kXferBlock = 64;
 static_assert(4 * kXferBlock <= kThreads, "one record value per thread and field");
 template <bool REFRESH>
@@ -3329,8 +3970,6 @@ __global__ void __launch_bounds__(kThreads)
         }
         s_ncol = cc;
         if (x.err_dst && blockIdx.x == 0) *x.err_dst = __ldcg(x.err_src);
-        // the step's integrators run after this kernel (stream order)
-        if (REFRESH && x.arm && blockIdx.x == 0) d.ctr->hout = x.hout;
     }
     if (to_cols) {
         double v[kXferFields];
