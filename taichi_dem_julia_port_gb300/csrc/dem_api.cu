@@ -5,6 +5,7 @@
 // (`simulate!`, src/executor.jl:162-172), host<->device state exchange, and the
 // arena of independent scenes (slot and bucket-range allocation, scene modes).
 #include <algorithm>
+#include <chrono>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -1406,7 +1407,6 @@ int create_single(const DemConfigC* cfg, const DemParticlesIn* pin, const DemTab
     if (rc == DEM_OK && pin->n > 0 && pin->n <= kStepsPerSm * sms) {
         h->steps_ok = steps_ready(h->p);
         rc = dalloc(h, &h->d.wtouch, (size_t)pin->n);
-        if (rc == DEM_OK) rc = dalloc(h, &h->d.wchg, (size_t)pin->n);
         if (rc == DEM_OK) rc = dalloc(h, &h->d.wforce, 6 * (size_t)h->nwall * (size_t)pin->n);
     }
     if (rc == DEM_OK) rc = flag_search(h, 0);
@@ -1886,13 +1886,23 @@ int dem_step_exchange(DemHandle* h, const DemParticleState* in, int64_t nsteps,
     if (!h || nsteps < 0 || h->multi) return DEM_ERR_INVALID;
     StepIO io{};
     if (direct_exchange(h, in, nsteps, out, &io)) {
-        volatile int* word = h->err_host;
-        *word = kNoHostOut;
+        __atomic_store_n(h->err_host, kNoHostOut, __ATOMIC_RELEASE);
         TRY(ensure_encoding(h));
         TRY(run_steps(h, nsteps, io));
-        CU(cudaStreamSynchronize(h->stream));
         ++h->exchanges_direct;
-        if (*word != kNoHostOut) return error_code(*word);
+        // the launch's last block writes the word once every record is in
+        // place: watched for a while (the launch is retired, and the stream
+        // wait returns, some microseconds later), then the stream is awaited
+        const auto t0 = std::chrono::steady_clock::now();
+        for (int k = 0;; ++k) {
+            const int e = __atomic_load_n(h->err_host, __ATOMIC_ACQUIRE);
+            if (e != kNoHostOut) return error_code(e);
+            if ((k & 63) == 63 && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(500))
+                break;
+        }
+        CU(cudaStreamSynchronize(h->stream));
+        const int e = __atomic_load_n(h->err_host, __ATOMIC_ACQUIRE);
+        if (e != kNoHostOut) return error_code(e);
         return device_error(h);  // not expected: a barrier of the steps gave up
     }
     if (in) TRY(set_particles(h, in, false));

@@ -148,7 +148,6 @@ struct alignas(8) RowCounter {
 // order: pos, vel, omega, quat, force, moment, wall_shear; nullptr: not
 // written) with the device error word.
 constexpr int kHostOutFields = 7;
-constexpr int kHostOutRows = 22;  // 3+3+3+4+3+3+3 values per particle
 struct HostOut {
     double* rec[kHostOutFields];
     int* err;
@@ -170,7 +169,7 @@ struct DevCounters {
     unsigned int pad;
     RowCounter alloc[2];            // contacts placed in each contact buffer
     unsigned long long tickets[2];  // tile tickets of the scan sites (never reset)
-    unsigned int bar, bar_pad;        // grid barrier of the cooperative kernels (grid_sync)
+    unsigned int bar, done;           // grid barrier of the cooperative kernels (grid_sync)
     unsigned int hashed[2];           // particles hashed by the step reading buffer cur
     // inspection of the fused pair search (DemParams::debug_enum): candidate
     // pairs (i, j > i) it visited and the wrapping sum of enum_mix(i, j)
@@ -200,9 +199,8 @@ struct DemDev {
     double *wsx, *wsy, *wsz;              // wall shear history: wall w of slot i at
                                           // [w * DemParams::wstride + i]
     // k_steps: per slot, the touching walls (bit mask) with their forces and
-    // moments (row 6·wall + component, wstride slots per row), and which
-    // components of the first wall's shear history the step changed
-    uint8_t *wtouch, *wchg;
+    // moments (row 6·wall + component, wstride slots per row)
+    uint8_t* wtouch;
     double* wforce;
     const MatTables* mt;                  // tables of a dem_create_tables handle, else null
     const uint8_t* mid;                   // its grains' material indices, else null

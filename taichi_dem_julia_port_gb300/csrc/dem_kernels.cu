@@ -1553,9 +1553,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
 // keeps it: |𝐪|² = 1 exactly, rsqrt(1) = 1 (checked by
 // dem_selftest_conversions) and 𝐪·1 = 𝐪, so nothing is computed or stored
 // (false is returned).
-__device__ __forceinline__ bool update_quaternion(const DemDev& d, int i, double wx, double wy,
-                                                  double wz, double qw, double qx, double qy,
-                                                  double qz) {
+__device__ __forceinline__ bool turn(double wx, double wy, double wz, double (&q)[4]) {
+    const double qw = q[0], qx = q[1], qy = q[2], qz = q[3];
     double nw = qw, nx = qx, ny = qy, nz = qz;
     const bool spinless = (__double_as_longlong(wx) | __double_as_longlong(wy) |
                            __double_as_longlong(wz)) == 0ll;
@@ -1572,10 +1571,21 @@ __device__ __forceinline__ bool update_quaternion(const DemDev& d, int i, double
         nz = __fma_rn(-qy, hx, __fma_rn(qx, hy, __fma_rn(qw, hz, qz)));
     }
     const double inq = rsqrt(__fma_rn(nz, nz, __fma_rn(ny, ny, __fma_rn(nx, nx, nw * nw))));
-    d.qw[i] = nw * inq;
-    d.qx[i] = nx * inq;
-    d.qy[i] = ny * inq;
-    d.qz[i] = nz * inq;
+    q[0] = nw * inq;
+    q[1] = nx * inq;
+    q[2] = ny * inq;
+    q[3] = nz * inq;
+    return true;
+}
+__device__ __forceinline__ bool update_quaternion(const DemDev& d, int i, double wx, double wy,
+                                                  double wz, double qw, double qx, double qy,
+                                                  double qz) {
+    double q[4] = {qw, qx, qy, qz};
+    if (!turn(wx, wy, wz, q)) return false;
+    d.qw[i] = q[0];
+    d.qx[i] = q[1];
+    d.qy[i] = q[2];
+    d.qz[i] = q[3];
     return true;
 }
 // The quaternions of a warp's 32 particles (slot i on lane i mod 32), reading
@@ -1680,6 +1690,19 @@ __device__ __forceinline__ void scene_flags_one(const DemDev& d, const DemParams
 
 
 // ---------------------------------------------------------------------------
+// The FP64 laws spell out their fused multiply-adds: which product of an
+// a·b + c·d the compiler would fuse can differ between two kernels that
+// contain the same code, and the kernels must agree bit for bit.
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double dot_(Vec3<double> a, Vec3<double> b) {
+    return fma_(a.z, b.z, fma_(a.y, b.y, a.x * b.x));
+}
+__device__ __forceinline__ double det_(double a, double b, double c, double d) {  // a·b - c·d
+    return fma_(a, b, -(c * d));
+}
+__device__ __forceinline__ Vec3<double> crossd(Vec3<double> a, Vec3<double> b) {
+    return {det_(a.y, b.z, a.z, b.y), det_(a.z, b.x, a.x, b.z), det_(a.x, b.y, a.y, b.x)};
+}
 // Contact frame of src/kernels.jl:145-165: the rotation 𝐑 taking the unit
 // normal a = normalize(𝐤ⱼ - 𝐤ᵢ) to the local x axis.  For b = x̂ the
 // reference's I + [v]ₓ + [v]ₓ² (1-c)/s² has the rows
@@ -1745,10 +1768,10 @@ __device__ __forceinline__ Frame contact_frame(double dx, double dy, double dz, 
     // degenerate branch is far (s² well above 4·tolerance²) is seen in FP32.
     const float y = d2f(ay), z = d2f(az);
     if (y * y + z * z > S.f_tol8 && d2f(ax) > -0.5f) {
-        F.f = rcp_nr(1.0 + ax);  // in (0.5, 2]
+        F.f = rcp_nr(__dadd_rn(1.0, ax));  // in (0.5, 2]
         return F;
     }
-    const double s2 = ay * ay + az * az;
+    const double s2 = fma_(az, az, ay * ay);
     // s² >= +0 (a sum of squares) and the tolerances are positive: compared
     // as bit patterns, off the FP64 pipe
     if (less_nonneg(s2, S.tol2_lo)) return frame_degenerate(ax);
@@ -1756,21 +1779,17 @@ __device__ __forceinline__ Frame contact_frame(double dx, double dy, double dz, 
     F.f = (1.0 - ax) * rcp_range(s2);
     return F;
 }
-template <typename T>
-__device__ __forceinline__ Vec3<T> rot(const Frame& R, Vec3<T> v) {  // 𝐑 v
-    const T a1 = (T)R.a1, a2 = (T)R.a2, a3 = (T)R.a3, f = (T)R.f;
-    const T w = a2 * v.y + a3 * v.z;
-    const T t = v.x + f * w;
-    const T z = v.z - a3 * t;
-    return {a1 * v.x + w, v.y - a2 * t, R.neg3 ? -z : z};
+__device__ __forceinline__ Vec3<double> rot(const Frame& R, Vec3<double> v) {  // 𝐑 v
+    const double w = fma_(R.a2, v.y, R.a3 * v.z);
+    const double t = fma_(R.f, w, v.x);
+    const double z = fma_(-R.a3, t, v.z);
+    return {fma_(R.a1, v.x, w), fma_(-R.a2, t, v.y), R.neg3 ? -z : z};
 }
-template <typename T>
-__device__ __forceinline__ Vec3<T> rot_t(const Frame& R, Vec3<T> v) {  // 𝐑ᵀ v
-    const T a1 = (T)R.a1, a2 = (T)R.a2, a3 = (T)R.a3, f = (T)R.f;
-    const T w = a2 * v.y + a3 * v.z;
-    const T u = v.x - f * w;
-    const T z = v.z + a3 * u;
-    return {a1 * v.x - w, v.y + a2 * u, R.neg3 ? -z : z};
+__device__ __forceinline__ Vec3<double> rot_t(const Frame& R, Vec3<double> v) {  // 𝐑ᵀ v
+    const double w = fma_(R.a2, v.y, R.a3 * v.z);
+    const double u = fma_(-R.f, w, v.x);
+    const double z = fma_(R.a3, u, v.z);
+    return {fma_(R.a1, v.x, -w), fma_(R.a2, u, v.y), R.neg3 ? -z : z};
 }
 
 __device__ __forceinline__ Vec3<double> ld3(const double* const* f, int base, int c) {
@@ -1781,11 +1800,6 @@ __device__ __forceinline__ void st3(double* const* f, int base, int c, Vec3<doub
     f[base + 1][c] = v.y;
     f[base + 2][c] = v.z;
 }
-template <typename T>
-__device__ __forceinline__ Vec3<T> from_d(Vec3<double> v) {
-    return {(T)v.x, (T)v.y, (T)v.z};
-}
-
 // EBPM failure (src/kernels.jl:208-219):
 //   σcᵢ = -Fₓ/A - (r/I)·sqrt(τᵢ₂²+τᵢ₃²), σc = -min(σcᵢ, σcⱼ), σt = max(σcᵢ, σcⱼ),
 //   σs = |τᵢ₁|·r/2/I + 4/3/A·sqrt(F₂²+F₃²);  breaks if σc >= σc₀ or σt >= σt₀ or
@@ -2036,8 +2050,9 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
         const float4 rmi = d.rm32[i], rmj = d.rm32[j];  // (rb/I, m, r, 0)
         const double Rsum = ri + rj;
         const double num = (dxd * dxd + dyd * dyd + dzd * dzd) - Rsum * Rsum;
-        const float L = L2 * invL;
-        const float gap = d2f(num) / (L + d2f(Rsum));
+        // (rounded before the sum in every kernel, not fused into it)
+        const float L = __fmul_rn(L2, invL);
+        const float gap = d2f(num) / __fadd_rn(L, d2f(Rsum));
         if (num > 0.0) atomicAdd(&d.sctr[sc].warn_gap, 1ull);
         const float ext = rmi.z - fabsf(gap);
         const Vec3<float> kri{ax * ext, ay * ext, az * ext};
@@ -2119,7 +2134,8 @@ __device__ __forceinline__ void force32(const DemDev& d, const SceneParams& SP,
 // bond section of rb = ρ·min(rᵢ, rⱼ) is formed here from that surface.
 __device__ __forceinline__ Frame pair_frame(Vec3<double> D, double L2, double invL,
                                             const SceneParams& SP) {
-    return contact_frame(D.x, D.y, D.z, D.x * invL, D.y * invL, D.z * invL, SP);
+    return contact_frame(D.x, D.y, D.z, __dmul_rn(D.x, invL), __dmul_rn(D.y, invL),
+                         __dmul_rn(D.z, invL), SP);
 }
 __device__ __forceinline__ Vec3<double> sub3(Vec3<double> a, Vec3<double> b) {
     return {a.x - b.x, a.y - b.y, a.z - b.z};
@@ -2170,27 +2186,26 @@ __device__ __forceinline__ PairOut bond_one(const DemDev& d, const SceneParams& 
         f_invA = d.bk32[small].w;
         f_rbI = d.rm32[small].x;
     }
-    const double L2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
+    const double L2 = dot_(dk, dk);
     const double invL = rsqrt(L2);
     const Frame R = pair_frame(dk, L2, invL, SP);
-    const Vec3<double> D = rot<double>(R, dv);
-    const Vec3<double> Sv = rot<double>(R, {wi.x + wj.x, wi.y + wj.y, wi.z + wj.z});
-    const Vec3<double> Q = rot<double>(R, sub3(wi, wj));
+    const Vec3<double> D = rot(R, dv);
+    const Vec3<double> Sv = rot(R, {wi.x + wj.x, wi.y + wj.y, wi.z + wj.z});
+    const Vec3<double> Q = rot(R, sub3(wi, wj));
     // with ϕ = c/L² the factor 1/(L²(1 + ϕ)) is 1/(L² + c), so
     // k₃dt = 6EI·dt/(L² + c), k₂dt = 2k₃dt/L, k₊dt = k₃dt·L/2 and
     // k₋dt = EI·dt/L
-    const double idt = invL * SP.dt;
-    const double km = b_EI * idt;
-    const double k1 = b_EA * idt;
-    const double k3 = (b_EI * SP.dt6) * rcp_range(L2 + b_phic);
-    const double k2 = twice_exact(k3 * invL);
-    const double k4 = km * b_1pnu;
-    const double kp = half_exact(k3) * (L2 * invL);
-    const double ay_ = kp * Sv.y - k3 * D.z, az_ = kp * Sv.z + k3 * D.y;
-    const double dtix = k4 * Q.x;
-    Fi = {Fi.x + k1 * D.x, Fi.y + (k2 * D.y + k3 * Sv.z), Fi.z + (k2 * D.z - k3 * Sv.y)};
-    ti = {ti.x + dtix, ti.y + (ay_ + km * Q.y), ti.z + (az_ + km * Q.z)};
-    tj = {tj.x - dtix, tj.y + (ay_ - km * Q.y), tj.z + (az_ - km * Q.z)};
+    const double idt = __dmul_rn(invL, SP.dt);
+    const double km = __dmul_rn(b_EI, idt);
+    const double k1 = __dmul_rn(b_EA, idt);
+    const double k3 = __dmul_rn(__dmul_rn(b_EI, SP.dt6), rcp_range(__dadd_rn(L2, b_phic)));
+    const double k2 = twice_exact(__dmul_rn(k3, invL));
+    const double k4 = __dmul_rn(km, b_1pnu);
+    const double kp = __dmul_rn(half_exact(k3), __dmul_rn(L2, invL));
+    const double ay_ = det_(kp, Sv.y, k3, D.z), az_ = fma_(kp, Sv.z, k3 * D.y);
+    Fi = {fma_(k1, D.x, Fi.x), Fi.y + fma_(k2, D.y, k3 * Sv.z), Fi.z + det_(k2, D.z, k3, Sv.y)};
+    ti = {fma_(k4, Q.x, ti.x), ti.y + fma_(km, Q.y, ay_), ti.z + fma_(km, Q.z, az_)};
+    tj = {fma_(-k4, Q.x, tj.x), tj.y + fma_(-km, Q.y, ay_), tj.z + fma_(-km, Q.z, az_)};
     // breakage test, FP64 (src/kernels.jl:208-222)
     bool broken;
     if constexpr (TAB) broken = bond_breaks_tab(Fi, ti, tj, f_invA, f_rbI, b_A, b_I, b_rb, *pc);
@@ -2206,8 +2221,8 @@ __device__ __forceinline__ PairOut bond_one(const DemDev& d, const SceneParams& 
     if (report)
         st3(w.f, CK, c, {half_exact(d.px[i] + d.px[j]), half_exact(d.py[i] + d.py[j]),
                          half_exact(d.pz[i] + d.pz[j])});
-    return {rot_t<double>(R, {-Fi.x, -Fi.y, -Fi.z}), rot_t<double>(R, {-ti.x, -ti.y, -ti.z}),
-            rot_t<double>(R, {-tj.x, -tj.y, -tj.z})};
+    return {rot_t(R, {-Fi.x, -Fi.y, -Fi.z}), rot_t(R, {-ti.x, -ti.y, -ti.z}),
+            rot_t(R, {-tj.x, -tj.y, -tj.z})};
 }
 // |𝐅ₜ| >= μF1 as the reference compares it
 static __device__ __noinline__ bool slides_exact(double n2, double muF1) { return sqrt(n2) >= muF1; }
@@ -2220,7 +2235,7 @@ __device__ __forceinline__ void tangential(double sx, double& sy, double& sz, do
                                            double vcy, double vcz, double muF1, double& F2,
                                            double& F3) {
     const double Fx = -kt * sx, Fy = -kt * sy, Fz = -kt * sz;
-    const double n2 = Fx * Fx + Fy * Fy + Fz * Fz, m2 = muF1 * muF1;
+    const double n2 = fma_(Fz, Fz, fma_(Fy, Fy, Fx * Fx)), m2 = muF1 * muF1;
     // n2 and m2 are >= +0 or NaN; both ordinary (an exponent field in
     // [64, 0x7fe]): compared as bit patterns, off the FP64 pipe
     const unsigned en = (unsigned)__double2hiint(n2) - 0x04000000u;
@@ -2236,8 +2251,8 @@ __device__ __forceinline__ void tangential(double sx, double& sy, double& sz, do
         sy *= -ratio;
         sz *= -ratio;
     } else {
-        F2 = Fy - gt * vcy;
-        F3 = Fz - gt * vcz;
+        F2 = fma_(-gt, vcy, Fy);
+        F3 = fma_(-gt, vcz, Fz);
     }
 }
 // Hertz-Mindlin (src/kernels.jl:240-313)
@@ -2253,18 +2268,20 @@ __device__ __forceinline__ PairOut hertz_one(const DemDev& d, const SceneParams&
     Vec3<double> s{0.0, 0.0, 0.0};
     if (sidx >= 0) s = ld3(o.f, CS, sidx);
     const double mi = d.m[i], mj = d.m[j];
-    const double L2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
+    const double L2 = dot_(dk, dk);
     const double invL = rsqrt(L2);
-    const double L = L2 * invL;
+    const double L = __dmul_rn(L2, invL);
     const Frame R = pair_frame(dk, L2, invL, SP);
-    const double gap = L - ri - rj;
+    const double gap = __dsub_rn(__dsub_rn(L, ri), rj);
     if (positive_bits(gap)) atomicAdd(&d.sctr[sc].warn_gap, 1ull);
-    const double dn = fabs(gap), ext = (ri - dn) * invL;
-    const Vec3<double> kri{dk.x * ext, dk.y * ext, dk.z * ext};
-    if (report) st3(w.f, CK, c, {d.px[i] + kri.x, d.py[i] + kri.y, d.pz[i] + kri.z});
-    const Vec3<double> krj = sub3(kri, dk);
-    const Vec3<double> wci = cross3<double>(wi, kri), wcj = cross3<double>(wj, krj);
-    const Vec3<double> vc = rot<double>(R, {dv0.x + (wcj.x - wci.x), dv0.y + (wcj.y - wci.y),
+    const double dn = fabs(gap), ext = __dmul_rn(__dsub_rn(ri, dn), invL);
+    const Vec3<double> kri{__dmul_rn(dk.x, ext), __dmul_rn(dk.y, ext), __dmul_rn(dk.z, ext)};
+    if (report)
+        st3(w.f, CK, c, {__dadd_rn(d.px[i], kri.x), __dadd_rn(d.py[i], kri.y),
+                         __dadd_rn(d.pz[i], kri.z)});
+    const Vec3<double> krj{__dsub_rn(kri.x, dk.x), __dsub_rn(kri.y, dk.y), __dsub_rn(kri.z, dk.z)};
+    const Vec3<double> wci = crossd(wi, kri), wcj = crossd(wj, krj);
+    const Vec3<double> vc = rot(R, {dv0.x + (wcj.x - wci.x), dv0.y + (wcj.y - wci.y),
                                             dv0.z + (wcj.z - wci.z)});
     const double sq = sqrt(ri * rj * rcp_range(ri + rj) * dn);  // √(R*·|gap|)
     const double pYs = TAB ? pc->Ys : SP.pp_Ys, pGs = TAB ? pc->Gs : SP.pp_Gs;
@@ -2277,14 +2294,15 @@ __device__ __forceinline__ PairOut hertz_one(const DemDev& d, const SceneParams&
         if (neg) atomicAdd(&d.sctr[sc].warn_damp, (unsigned long long)neg);
     }
     // (0·vc.x adds nothing to the normal component unless it is not finite)
-    s = {(__double2hiint(vc.x) & 0x7ff00000) != 0x7ff00000 ? s.x : s.x + vc.x * 0.0, s.y + vc.y * SP.dt, s.z + vc.z * SP.dt};
-    const double F1 = -kn * gap - gn * vc.x;
+    s = {(__double2hiint(vc.x) & 0x7ff00000) != 0x7ff00000 ? s.x : s.x + vc.x * 0.0,
+         fma_(vc.y, SP.dt, s.y), fma_(vc.z, SP.dt, s.z)};
+    const double F1 = -fma_(kn, gap, gn * vc.x);
     double F2, F3;
     tangential(s.x, s.y, s.z, kt, gt, vc.y, vc.z, (TAB ? pc->mu : SP.pp_mu) * F1, F2, F3);
     st3(w.f, CS, c, s);
     if (report) st3(w.f, CF, c, {F1, F2, F3});
-    const Vec3<double> F = rot_t<double>(R, {-F1, -F2, -F3});
-    return {F, cross3<double>(kri, F), cross3<double>(krj, {-F.x, -F.y, -F.z})};
+    const Vec3<double> F = rot_t(R, {-F1, -F2, -F3});
+    return {F, crossd(kri, F), crossd(krj, {-F.x, -F.y, -F.z})};
 }
 template <typename T, bool TAB = false>
 __device__ __forceinline__ void contact_one(const DemDev& d, const SceneParams& SP,
@@ -2358,8 +2376,12 @@ __device__ __forceinline__ int force_body(const DemDev& d, const DemParams& p, i
             else raise_error(d.ctr, kErrCapacity);
         };
         if (!LATE) enlist();
+        // opaque in each iteration: two copies of the loop, one per value, could
+        // fuse different products of the FP32 laws into FMAs
+        int rp = report ? 1 : 0;
+        asm volatile("" : "+r"(rp));
         contact_one<T, TAB>(d, scene_rec<MULTI>(d, p, sc), w, o, sidx, c, fl, i, j, sc, cap,
-                            report);
+                            rp != 0);
         if (LATE) enlist();
     }
     return total;
@@ -2576,39 +2598,40 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
         // point -L/|L|·(|L| + |gap|/2)·n is -sign(L)·(|L| + r)/2·n
         const double gap = fabs(L) - r;
         const double dn = -gap;
-        const double h = 0.5 * (fabs(L) + r);
+        const double h = __dmul_rn(0.5, __dadd_rn(fabs(L), r));
         const double hs = L > 0.0 ? -h : (L < 0.0 ? h : CUDART_NAN);  // L/|L| of a centre on the wall
-        const double kix = hs * W.wn[0], kiy = hs * W.wn[1], kiz = hs * W.wn[2];
-        const double vcix = wy * kiz - wz * kiy + vx, vciy = wz * kix - wx * kiz + vy,
-                     vciz = wx * kiy - wy * kix + vz;
+        const Vec3<double> ki{__dmul_rn(hs, W.wn[0]), __dmul_rn(hs, W.wn[1]), __dmul_rn(hs, W.wn[2])};
+        const Vec3<double> vci{fma_(wy, ki.z, fma_(-wz, ki.y, vx)), fma_(wz, ki.x, fma_(-wx, ki.z, vy)),
+                               fma_(wx, ki.y, fma_(-wy, ki.x, vz))};
         const double* Rw = W.wR;
-        const double vcx = -(Rw[0] * vcix + Rw[1] * vciy + Rw[2] * vciz);
-        const double vcy = -(Rw[3] * vcix + Rw[4] * vciy + Rw[5] * vciz);
-        const double vcz = -(Rw[6] * vcix + Rw[7] * vciy + Rw[8] * vciz);
-        const double sq = sqrt(r * dn);
-        const double kn = 4.0 / 3.0 * W.Ys * sq;
-        const double kt = 8.0 * W.Gs * sq;
-        const double root = sqrt(m * sq);
-        const double gn = W.cgn * root;
-        const double gt = W.cgt * root;
+        const double vcx = -dot_({Rw[0], Rw[1], Rw[2]}, vci);
+        const double vcy = -dot_({Rw[3], Rw[4], Rw[5]}, vci);
+        const double vcz = -dot_({Rw[6], Rw[7], Rw[8]}, vci);
+        const double sq = sqrt(__dmul_rn(r, dn));
+        const double kn = __dmul_rn(4.0 / 3.0 * W.Ys, sq);
+        const double kt = __dmul_rn(8.0 * W.Gs, sq);
+        const double root = sqrt(__dmul_rn(m, sq));
+        const double gn = __dmul_rn(W.cgn, root);
+        const double gt = __dmul_rn(W.cgt, root);
         if (count && (__double2hiint(gn) < 0 || __double2hiint(gt) < 0)) {
             const int neg = (gn < 0.0) + (gt < 0.0);
             if (neg) atomicAdd(&d.sctr[sc].warn_damp, (unsigned long long)neg);
         }
-        double sx = *wsx + vcx * 0.0, sy = *wsy + vcy * dt, sz = *wsz + vcz * dt;
-        const double F1 = -kn * gap - gn * vcx;
+        double sx = fma_(vcx, 0.0, *wsx), sy = fma_(vcy, dt, *wsy), sz = fma_(vcz, dt, *wsz);
+        const double F1 = -fma_(kn, gap, __dmul_rn(gn, vcx));
         double F2, F3;
         tangential(sx, sy, sz, kt, gt, vcy, vcz, W.mu * F1, F2, F3);
         const double* Ri = W.wRinv;
-        const double gx = -(Ri[0] * F1 + Ri[1] * F2 + Ri[2] * F3);
-        const double gy = -(Ri[3] * F1 + Ri[4] * F2 + Ri[5] * F3);
-        const double gz = -(Ri[6] * F1 + Ri[7] * F2 + Ri[8] * F3);
-        g[0] = gx;
-        g[1] = gy;
-        g[2] = gz;
-        mw[0] = kiy * gz - kiz * gy;
-        mw[1] = kiz * gx - kix * gz;
-        mw[2] = kix * gy - kiy * gx;
+        const Vec3<double> F{F1, F2, F3};
+        const Vec3<double> G{-dot_({Ri[0], Ri[1], Ri[2]}, F), -dot_({Ri[3], Ri[4], Ri[5]}, F),
+                             -dot_({Ri[6], Ri[7], Ri[8]}, F)};
+        const Vec3<double> Mw = crossd(ki, G);
+        g[0] = G.x;
+        g[1] = G.y;
+        g[2] = G.z;
+        mw[0] = Mw.x;
+        mw[1] = Mw.y;
+        mw[2] = Mw.z;
         *wsx = sx;
         *wsy = sy;
         *wsz = sz;
@@ -2708,16 +2731,16 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     }
     // apply_body_force!  A zero gravity component adds nothing: the force sum
     // starts at +0 and never becomes -0, so F + 0·m is F.
-    if (nonzero_bits(S.grav[0])) F[0] += S.grav[0] * m;
-    if (nonzero_bits(S.grav[1])) F[1] += S.grav[1] * m;
-    if (nonzero_bits(S.grav[2])) F[2] += S.grav[2] * m;
+    if (nonzero_bits(S.grav[0])) F[0] = fma_(S.grav[0], m, F[0]);
+    if (nonzero_bits(S.grav[1])) F[1] = fma_(S.grav[1], m, F[1]);
+    if (nonzero_bits(S.grav[2])) F[2] = fma_(S.grav[2], m, F[2]);
     if (nonzero_bits(S.damping)) {
         const double v3[3] = {vx, vy, vz}, w3[3] = {wx, wy, wz};
         double dF[3], dM[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            dF[q] = -S.damping * fabs(F[q]) * jl_sign(v3[q]);
-            dM[q] = -S.damping * fabs(M[q]) * jl_sign(w3[q]);
+            dF[q] = __dmul_rn(__dmul_rn(-S.damping, fabs(F[q])), jl_sign(v3[q]));
+            dM[q] = __dmul_rn(__dmul_rn(-S.damping, fabs(M[q])), jl_sign(w3[q]));
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -2728,8 +2751,8 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     // update!
     const double ax = F[0] * invm, ay = F[1] * invm, az = F[2] * invm;
     const double hdt2 = S.hdt2;  // 0.5·(dt·dt)
-    const double px1 = x + vx * dt + ax * hdt2, py1 = y + vy * dt + ay * hdt2,
-                 pz1 = z + vz * dt + az * hdt2;
+    const double px1 = fma_(ax, hdt2, fma_(vx, dt, x)), py1 = fma_(ay, hdt2, fma_(vy, dt, y)),
+                 pz1 = fma_(az, hdt2, fma_(vz, dt, z));
     d.px[i] = px1;
     d.py[i] = py1;
     d.pz[i] = pz1;
@@ -2747,9 +2770,9 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
         if (moved && lane_id() == (unsigned)(__ffs(peers) - 1) && d.sflags[nxt][sc] == 0u)
             atomicOr(&d.sflags[nxt][sc], 1u);
     }
-    d.vx[i] = vx + ax * dt;
-    d.vy[i] = vy + ay * dt;
-    d.vz[i] = vz + az * dt;
+    d.vx[i] = fma_(ax, dt, vx);
+    d.vy[i] = fma_(ay, dt, vy);
+    d.vz[i] = fma_(az, dt, vz);
     bool spin = turned && update_quaternion(d, i, wx, wy, wz, q4[0], q4[1], q4[2], q4[3]);
     // 𝛚 + 𝐌·I⁻¹dt: with 𝐌 = (+0, +0, +0) and a finite I⁻¹dt, fma(+0, I⁻¹dt, w)
     // is w unless w is -0, so a torque-free particle keeps its stored spin
@@ -2905,42 +2928,142 @@ __device__ __forceinline__ bool particle_wall(const DemDev& d, const DemParams& 
                       d.wsz + o, g, mw, true);
 }
 
-// k_steps: the walls of the 32 particles [32u, 32u + 32) by one warp, in the
-// force phase (the walls depend on the step's starting state only, and the
-// warps that have no contacts to compute are free then; a wall contact's
-// chain, about 90 FP64 instructions, was the longest of the integration).
-// Leaves the touching walls as a bit mask, their forces and moments, and
-// which components of the first wall's shear history changed.
-template <bool TAB>
-__device__ __forceinline__ void wall_items(const DemDev& d, const DemParams& p, int u) {
-    const int i = u * 32 + (int)lane_id();
-    if (i >= p.n) return;
-    const SceneParams& S = p.s0;
-    const int nwall = TAB ? d.mt->nwall : (S.has_wall ? 1 : 0);
-    const double wx = d.wx[i], wy = d.wy[i], wz = d.wz[i];
-    unsigned touch = 0u, chg = 0u;
-    for (int wl = 0; wl < nwall; ++wl) {
-        const double before[3] = {d.wsx[i], d.wsy[i], d.wsz[i]};
-        double g[3], mw[3];
-        if (particle_wall<TAB>(d, p, S, i, 0, wl, wx, wy, wz, g, mw)) {
-            touch |= 1u << wl;
+// One warp's staging of 32 particles' records (k_steps).
+struct RecordStage {
+    double v[4 * 32];
+    uint8_t chg[4 * 32];
+};
+// 32 particles' k-component records src (page-locked host or device memory) to
+// this lane's particle: x[0..k)
+template <int K>
+__device__ __forceinline__ void read_records(const double* src, int base, int m, RecordStage& st,
+                                             double (&x)[K]) {
+    const int l = (int)lane_id();
+    __syncwarp();
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                d.wforce[(size_t)(6 * wl + c) * p.wstride + i] = g[c];
-                d.wforce[(size_t)(6 * wl + 3 + c) * p.wstride + i] = mw[c];
-            }
-        }
-        if (wl == 0) {
-            const double after[3] = {d.wsx[i], d.wsy[i], d.wsz[i]};
+    for (int k = 0; k < K; ++k)
+        if (l + 32 * k < K * m) st.v[l + 32 * k] = src[(size_t)K * base + l + 32 * k];
+    __syncwarp();
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                chg |= __double_as_longlong(after[c]) != __double_as_longlong(before[c]) ? 1u << c : 0u;
-        }
+    for (int c = 0; c < K; ++c) x[c] = l < m ? st.v[K * l + c] : 0.0;
+}
+// and back; with `keep`, only the values that differ from `old`
+template <int K>
+__device__ __forceinline__ void write_records(double* dst, int base, int m, RecordStage& st,
+                                              const double (&x)[K], const double (&old)[K],
+                                              bool keep) {
+    const int l = (int)lane_id();
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+        st.v[K * l + c] = x[c];
+        st.chg[K * l + c] = __double_as_longlong(x[c]) != __double_as_longlong(old[c]);
     }
-    d.wtouch[i] = (uint8_t)touch;
-    d.wchg[i] = (uint8_t)chg;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int e = l + 32 * k;
+        if (e < K * m && (!keep || st.chg[e])) dst[(size_t)K * base + e] = st.v[e];
+    }
 }
 
+// k_steps: the walls and the quaternions of the 32 particles [32u, 32u + 32) by
+// one warp, in the force phase: both depend on the step's starting state only,
+// and the warps without contacts are free then (in the integration a wall
+// contact's chain, about 90 FP64 instructions, and the quaternion's after it
+// were the longest).  Leaves the touching walls as a bit mask with their
+// forces and moments.  IN: the orientations and the first wall's shear
+// history come from the caller's records; OUT: they go there, so that this
+// part of an exchange runs beside the forces.
+template <bool TAB>
+__device__ __forceinline__ void particle_items(const DemDev& d, const DemParams& p, int u,
+                                               RecordStage& st, const StepIO& io, bool in,
+                                               bool out) {
+    const int base = u * 32, m = min(32, p.n - base), l = (int)lane_id();
+    const int i = base + l;
+    const bool exists = l < m;
+    const SceneParams& S = p.s0;
+    const int nwall = TAB ? d.mt->nwall : (S.has_wall ? 1 : 0);
+    double w3[3] = {0.0, 0.0, 0.0}, q[4] = {1.0, 0.0, 0.0, 0.0}, s0[3] = {0.0, 0.0, 0.0};
+    if (exists) {
+        w3[0] = d.wx[i];
+        w3[1] = d.wy[i];
+        w3[2] = d.wz[i];
+    }
+    const bool qin = in && io.in[3], sin = in && io.in[4];
+    if (qin) {
+        read_records<4>(io.in[3], base, m, st, q);
+    } else if (exists) {
+        q[0] = d.qw[i];
+        q[1] = d.qx[i];
+        q[2] = d.qy[i];
+        q[3] = d.qz[i];
+    }
+    if (sin) {
+        read_records<3>(io.in[4], base, m, st, s0);
+        if (exists) {
+            d.wsx[i] = s0[0];
+            d.wsy[i] = s0[1];
+            d.wsz[i] = s0[2];
+        }
+    } else if (out && exists) {
+        s0[0] = d.wsx[i];
+        s0[1] = d.wsy[i];
+        s0[2] = d.wsz[i];
+    }
+    if (exists) {
+        unsigned touch = 0u;
+        for (int wl = 0; wl < nwall; ++wl) {
+            double g[3], mw[3];
+            if (particle_wall<TAB>(d, p, S, i, 0, wl, w3[0], w3[1], w3[2], g, mw)) {
+                touch |= 1u << wl;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    d.wforce[(size_t)(6 * wl + c) * p.wstride + i] = g[c];
+                    d.wforce[(size_t)(6 * wl + 3 + c) * p.wstride + i] = mw[c];
+                }
+            }
+        }
+        d.wtouch[i] = (uint8_t)touch;
+    }
+    if (out && io.out.rec[6]) {
+        double s1[3] = {0.0, 0.0, 0.0};
+        if (exists) {
+            s1[0] = d.wsx[i];
+            s1[1] = d.wsy[i];
+            s1[2] = d.wsz[i];
+        }
+        write_records<3>(io.out.rec[6], base, m, st, s1, s0, (io.out.same >> 6) & 1u);
+    }
+    double n[4] = {q[0], q[1], q[2], q[3]};
+    if (exists && (turn(w3[0], w3[1], w3[2], n) || qin)) {
+        d.qw[i] = n[0];
+        d.qx[i] = n[1];
+        d.qy[i] = n[2];
+        d.qz[i] = n[3];
+    }
+    if (out && io.out.rec[3])
+        write_records<4>(io.out.rec[3], base, m, st, n, q, (io.out.same >> 3) & 1u);
+}
+// The place of warp w in the order in which a block's warps take particle
+// items, given the block's contact chunks: warps with one chunk fewer first,
+// and among them those on SM sub-partitions (warp mod 4) with fewer chunks,
+// so that the items fill the gaps that the contacts leave.
+__device__ __forceinline__ int item_rank(int w, int nw, int chunks) {
+    const int r = chunks % nw;
+    const int l = (int)lane_id();
+    const int cls = l < r ? 2 : ((l & 3) >= (r & 3) ? 0 : 1);
+    const unsigned c0 = __ballot_sync(0xffffffffu, l < nw && cls == 0);
+    const unsigned c1 = __ballot_sync(0xffffffffu, l < nw && cls == 1);
+    const unsigned c2 = __ballot_sync(0xffffffffu, l < nw && cls == 2);
+    const unsigned lt = (1u << w) - 1u, me = 1u << w;
+    if (c0 & me) return __popc(c0 & lt);
+    if (c1 & me) return __popc(c0) + __popc(c1 & lt);
+    return __popc(c0) + __popc(c1) + __popc(c2 & lt);
+}
+
+// rows staged by the integrator: position, velocity, spin, force, moment
+constexpr int kStageRows = 15;
 // Shared memory of one group of four warps.  FUSED (k_steps): with the staging
 // of the exchange's output, and without the walls' forces, which wall_items
 // has left in memory.
@@ -2948,10 +3071,10 @@ template <bool TAB, bool FUSED>
 struct SplitShared {
     static constexpr int NW = FUSED ? 1 : (TAB ? kMaxWalls : 1);
     double wall[FUSED ? 1 : NW][FUSED ? 1 : 6][32];  // each wall's force and moment on each particle
-    double out[FUSED ? kHostOutRows : 1][32];   // the new state, as rows of the output records
+    double out[FUSED ? kStageRows : 1][32];     // the new state, as rows of the output records
     float pos[3][32];                           // the new FP32 position components
     uint8_t touch[NW][32];
-    uint8_t chg[FUSED ? kHostOutRows : 1][32];  // value differs from the step's input
+    uint8_t chg[FUSED ? kStageRows : 1][32];    // value differs from the step's input
 };
 // The particles [32u, 32u + 32) by four warps: q is the calling warp's role
 // (0, 1, 2: component; 3: walls and quaternion), tq its thread's index among
@@ -3014,17 +3137,17 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
     // warp 3: the step's starting spin, for the walls now and the quaternion
     // after the first barrier (the component warps store the new spin after it)
     double wx = 0.0, wy = 0.0, wz = 0.0, qw = 1.0, qx = 0.0, qy = 0.0, qz = 0.0;
-    if (q == 3 && live) {
-        wx = d.wx[i];
-        wy = d.wy[i];
-        wz = d.wz[i];
-        qw = d.qw[i];  // loaded here: their latency hides behind the walls
-        qx = d.qx[i];
-        qy = d.qy[i];
-        qz = d.qz[i];
-        // resolve_wall!: each wall's force and moment, added by the component
-        // warps in wall order
-        if constexpr (!FUSED) {
+    if constexpr (!FUSED) {
+        if (q == 3 && live) {
+            wx = d.wx[i];
+            wy = d.wy[i];
+            wz = d.wz[i];
+            qw = d.qw[i];  // loaded here: their latency hides behind the walls
+            qx = d.qx[i];
+            qy = d.qy[i];
+            qz = d.qz[i];
+            // resolve_wall!: each wall's force and moment, added by the component
+            // warps in wall order
             for (int wl = 0; wl < nwall; ++wl) {
                 double g[3], mw[3];
                 const bool touch = particle_wall<TAB>(d, p, S, i, sc, wl, wx, wy, wz, g, mw);
@@ -3038,57 +3161,13 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
                 }
             }
         }
-        if (out) {  // the first wall's shear history, and what wall_items changed of it
-            const double* ws[3] = {d.wsx, d.wsy, d.wsz};
-            const unsigned chg = d.wchg[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                sh.chg[19 + c][l] = (chg >> c) & 1u;
-                sh.out[19 + c][l] = ws[c][i];
-            }
-        }
     }
     meet();  // walls in shared memory; every component thread has read in_cnt
     if (q == 3 && exists) d.in_cnt[i] = 0;
     // the quaternion (integrate_body's update, from the starting spin) runs
     // while the component warps update the position, velocity and spin
-    if (q == 3 && live) {
-        const bool spinless = (__double_as_longlong(wx) | __double_as_longlong(wy) |
-                               __double_as_longlong(wz)) == 0ll;
-        const bool identity = spinless && __double_as_longlong(qw) == 0x3ff0000000000000ll &&
-                              (__double_as_longlong(qx) | __double_as_longlong(qy) |
-                               __double_as_longlong(qz)) == 0ll;
-        double ow = qw, ox = qx, oy = qy, oz = qz;
-        if (!identity) {
-            double nw = qw, nx = qx, ny = qy, nz = qz;
-            if (!(spinless && finite_not_negzero(qw) && finite_not_negzero(qx) &&
-                  finite_not_negzero(qy) && finite_not_negzero(qz))) {
-                const double hx = half_exact(wx), hy = half_exact(wy), hz = half_exact(wz);
-                nw = __fma_rn(-qz, hz, __fma_rn(-qy, hy, __fma_rn(-qx, hx, qw)));
-                nx = __fma_rn(-qz, hy, __fma_rn(qy, hz, __fma_rn(qw, hx, qx)));
-                ny = __fma_rn(qz, hx, __fma_rn(qx, hz, __fma_rn(qw, hy, qy)));
-                nz = __fma_rn(-qy, hx, __fma_rn(qx, hy, __fma_rn(qw, hz, qz)));
-            }
-            const double inq = rsqrt(__fma_rn(nz, nz, __fma_rn(ny, ny, __fma_rn(nx, nx, nw * nw))));
-            ow = nw * inq;
-            ox = nx * inq;
-            oy = ny * inq;
-            oz = nz * inq;
-            d.qw[i] = ow;
-            d.qx[i] = ox;
-            d.qy[i] = oy;
-            d.qz[i] = oz;
-        }
-        if (out) {
-            sh.out[9][l] = ow;
-            sh.out[10][l] = ox;
-            sh.out[11][l] = oy;
-            sh.out[12][l] = oz;
-            sh.chg[9][l] = __double_as_longlong(ow) != __double_as_longlong(qw);
-            sh.chg[10][l] = __double_as_longlong(ox) != __double_as_longlong(qx);
-            sh.chg[11][l] = __double_as_longlong(oy) != __double_as_longlong(qy);
-            sh.chg[12][l] = __double_as_longlong(oz) != __double_as_longlong(qz);
-        }
+    if constexpr (!FUSED) {
+        if (q == 3 && live) update_quaternion(d, i, wx, wy, wz, qw, qx, qy, qz);
     }
     if (q < 3 && live) {
         const double dt = S.dt;
@@ -3101,20 +3180,20 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             }
         }
         // apply_body_force!
-        if (nonzero_bits(S.grav[q])) Fq += S.grav[q] * m;
+        if (nonzero_bits(S.grav[q])) Fq = fma_(S.grav[q], m, Fq);
         if (nonzero_bits(S.damping)) {
-            const double dF = -S.damping * fabs(Fq) * jl_sign(vq);
-            const double dM = -S.damping * fabs(Mq) * jl_sign(wq);
+            const double dF = __dmul_rn(__dmul_rn(-S.damping, fabs(Fq)), jl_sign(vq));
+            const double dM = __dmul_rn(__dmul_rn(-S.damping, fabs(Mq)), jl_sign(wq));
             Fq += dF;
             Mq += dM;
         }
         // update!
         const double aq = Fq * invm;
         const double hdt2 = S.hdt2;
-        const double pq1 = xq + vq * dt + aq * hdt2;
+        const double pq1 = fma_(aq, hdt2, fma_(vq, dt, xq));
         pick3(q, d.px, d.py, d.pz)[i] = pq1;
         sh.pos[q][l] = d2f(pq1 - S.dmin[q]);
-        const double vq1 = vq + aq * dt;
+        const double vq1 = fma_(aq, dt, vq);
         pick3(q, d.vx, d.vy, d.vz)[i] = vq1;
         // 𝛚 + 𝐌·I⁻¹dt; with Mq = +0, a finite I⁻¹dt and wq not -0 the sum
         // is wq and the stored spin stays
@@ -3131,8 +3210,8 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
             sh.out[q][l] = pq1;
             sh.out[3 + q][l] = vq1;
             sh.out[6 + q][l] = wq1;
-            sh.out[13 + q][l] = Fq;
-            sh.out[16 + q][l] = Mq;
+            sh.out[9 + q][l] = Fq;
+            sh.out[12 + q][l] = Mq;
             sh.chg[q][l] = __double_as_longlong(pq1) != __double_as_longlong(xq);
             sh.chg[3 + q][l] = __double_as_longlong(vq1) != __double_as_longlong(vq);
             sh.chg[6 + q][l] = __double_as_longlong(wq1) != __double_as_longlong(wq);
@@ -3151,23 +3230,19 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
     if constexpr (FUSED) {
         if (out) {
             // the 32 particles are one contiguous range of each record array:
-            // k·32 values, written by consecutive threads
+            // 96 values, written by consecutive threads
             const int i0 = u * 32, m = min(32, p.n - i0);
             const unsigned same = H->same;
-            int row = 0;
+            constexpr int kField[5] = {0, 1, 2, 4, 5};  // (3, 6: particle_items wrote them)
 #pragma unroll
-            for (int f = 0; f < kHostOutFields; ++f) {
-                const int k = f == 3 ? 4 : 3;
-                double* rec = H->rec[f];
-                const bool keep = (same >> f) & 1u;  // unchanged values are there already
-                if (rec) {
-                    for (int e = tq; e < k * 32; e += kSplitThreads) {
-                        const int pq = e / k, r = row + e - pq * k;
-                        if (pq < m && (!keep || sh.chg[r][pq]))
-                            rec[(size_t)k * i0 + e] = sh.out[r][pq];
-                    }
+            for (int f = 0; f < 5; ++f) {
+                double* rec = H->rec[kField[f]];
+                const bool keep = (same >> kField[f]) & 1u;  // unchanged values are there already
+                if (rec && tq < 96) {
+                    const int pq = tq / 3, r = 3 * f + tq - pq * 3;
+                    if (pq < m && (!keep || sh.chg[r][pq]))
+                        rec[(size_t)3 * i0 + tq] = sh.out[r][pq];
                 }
-                row += k;
             }
             meet();  // the next round's staging waits for these reads
         }
@@ -3246,9 +3321,10 @@ __global__ void __launch_bounds__(kSplitThreads) k_integrate_split_tab(DemDev d,
 //
 // IO (dem_step_exchange): the first step reads the particle state from the
 // caller's arrays, the positions by all warps (the contact update waits for
-// them), the other fields by a quarter of the warps while the others update
-// the contacts; the last step's integrator writes the state into the
-// caller's arrays as each group of 32 particles is done.
+// them), velocities and spins by a quarter of the warps while the others
+// update the contacts, orientations and the first wall's shear history in the
+// force phase (particle_items); the last step writes those two there and the
+// rest in the integration, as each group of 32 particles is done.
 //
 // Only the last step's contact points, Hertz forces and particle totals are
 // stored (report_last): the caller of several steps cannot read the others'.
@@ -3283,42 +3359,31 @@ __device__ __forceinline__ void read_positions(const DemDev& d, const DemParams&
         __syncwarp();
     }
 }
-// the other fields, by warps [w0, warps of the block): every load of 32
+// velocities and spins, by warps [w0, warps of the block): every load of 32
 // particles is issued before the first store
-__device__ __forceinline__ void read_rest(const DemDev& d, const DemParams& p, const StepIO& io,
-                                          int w0) {
+__device__ __forceinline__ void read_motion(const DemDev& d, const DemParams& p, const StepIO& io,
+                                            int w0) {
     const int l = (int)lane_id();
     const int nw = (int)(blockDim.x >> 5) - w0;
-    double* const col[4][4] = {{d.vx, d.vy, d.vz, nullptr},
-                               {d.wx, d.wy, d.wz, nullptr},
-                               {d.qw, d.qx, d.qy, d.qz},
-                               {d.wsx, d.wsy, d.wsz, nullptr}};
     for (int c = ((int)(threadIdx.x >> 5) - w0) * (int)gridDim.x + (int)blockIdx.x; c * 32 < p.n;
          c += (int)gridDim.x * nw) {
         const int base = c * 32, m = min(32, p.n - base);
-        double v[4][4];
+        double v[2][3];
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            constexpr int K[4] = {3, 3, 4, 3};
+        for (int f = 0; f < 2; ++f)
 #pragma unroll
-            for (int k = 0; k < K[f]; ++k) {
-                v[f][k] = 0.0;
-                if (io.in[1 + f] && l + 32 * k < K[f] * m)
-                    v[f][k] = io.in[1 + f][(size_t)K[f] * base + l + 32 * k];
+            for (int k = 0; k < 3; ++k)
+                if (io.in[1 + f] && l + 32 * k < 3 * m)
+                    v[f][k] = io.in[1 + f][(size_t)3 * base + l + 32 * k];
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int e = l + 32 * k, q = e / 3, comp = e - 3 * q;
+                if (io.in[1 + f] && e < 3 * m)
+                    (f == 0 ? pick3(comp, d.vx, d.vy, d.vz) : pick3(comp, d.wx, d.wy, d.wz))[base + q] =
+                        v[f][k];
             }
-        }
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            constexpr int K[4] = {3, 3, 4, 3};
-            if (!io.in[1 + f]) continue;
-#pragma unroll
-            for (int k = 0; k < K[f]; ++k) {
-                const int e = l + 32 * k, q = e / K[f], comp = e - K[f] * q;
-                double* dst = comp == 0 ? col[f][0]
-                                        : (comp == 1 ? col[f][1] : (comp == 2 ? col[f][2] : col[f][3]));
-                if (e < K[f] * m) dst[base + q] = v[f][k];
-            }
-        }
     }
 }
 
@@ -3348,7 +3413,7 @@ __global__ void __launch_bounds__(kStepThreads, 1)
             if (!grid_sync(d.ctr, all)) return;
             team.nt = nt - nt / 4;
             team.bar = 1;
-            if ((int)threadIdx.x >= team.nt) read_rest(d, p, io, team.nt / 32);
+            if ((int)threadIdx.x >= team.nt) read_motion(d, p, io, team.nt / 32);
         }
         if ((int)threadIdx.x < team.nt) {
             if (__ldcg(&d.sflags[cur][0]) != 0u)
@@ -3361,17 +3426,18 @@ __global__ void __launch_bounds__(kStepThreads, 1)
         {
             const int total = force_body<T, false, TAB, true>(d, p, nxt, t0, (int)gridDim.x * nt,
                                                               report);
-            // the walls go to the warps after those of the last contacts
-            const int W = (int)gridDim.x * (nt / 32), items = (total + 31) / 32;
-            int u = t0 / 32 - items % W;
-            for (u = u < 0 ? u + W : u; u * 32 < p.n; u += W) wall_items<TAB>(d, p, u);
+            // particle items: unit u to block u mod blocks
+            const int G = (int)gridDim.x, nw = nt / 32, items = (total + 31) / 32;
+            const int chunks = (items - (int)blockIdx.x + G - 1) / G;  // of this block (>= 0)
+            RecordStage& st = reinterpret_cast<RecordStage*>(raw)[w];
+            for (int u = item_rank(w, nw, max(chunks, 0)) * G + (int)blockIdx.x; u * 32 < p.n;
+                 u += nw * G)
+                particle_items<TAB>(d, p, u, st, io, io.has_in && s == 0, io.has_out && last);
         }
         if (!grid_sync(d.ctr, all)) return;
         if (t0 == 0) {
             d.ctr->alloc[cur] = RowCounter{0u, 0u};  // the free buffer is next step's target
             scene_flags_one<false>(d, p, cur, 0);
-            // no integrator raises an error
-            if (io.has_out && last) *io.out.err = __ldcg(&d.ctr->error);
         }
         const int quad = w >> 2;
         int round = 0;
@@ -3381,6 +3447,21 @@ __global__ void __launch_bounds__(kStepThreads, 1)
                 d, p, cur, u, (w - quad - round) & 3, (int)threadIdx.x & (kSplitThreads - 1),
                 2 + quad, split[quad], io.has_out && last ? &io.out : nullptr, report);
         if (!last && !grid_sync(d.ctr, all)) return;
+    }
+    if (io.has_out) {
+        // the last block whose records are written (seen by the host before the
+        // word: system fences) tells the host, with the device error word (no
+        // integrator raises an error); the host need not wait for the launch
+        // to be retired
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence_system();
+            if (atomicAdd(&d.ctr->done, 1u) == gridDim.x - 1) {
+                d.ctr->done = 0u;
+                __threadfence_system();
+                *(volatile int*)io.out.err = __ldcg(&d.ctr->error);
+            }
+        }
     }
 }
 
@@ -3561,7 +3642,7 @@ size_t steps_shared(int threads, bool tab) {
                           sizeof(ListShared) * (size_t)(threads / kVLanes);
     const size_t split = (size_t)(threads / kSplitThreads) *
                          (tab ? sizeof(SplitShared<true, true>) : sizeof(SplitShared<false, true>));
-    return std::max(std::max(search, split), sizeof(double) * 96 * (size_t)(threads / 32));
+    return std::max(std::max(search, split), sizeof(RecordStage) * (size_t)(threads / 32));
 }
 using StepsKernel = void (*)(DemDev, DemParams, int, int, int, StepIO);
 StepsKernel steps_kernel(const DemParams& p) {
