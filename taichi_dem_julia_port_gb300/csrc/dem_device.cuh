@@ -232,6 +232,16 @@ __device__ __forceinline__ int32_t cell_index(double num, double cell, double in
 // the exact octant side follow from q' alone; otherwise (and for NaN or huge
 // values, which fail the test) the exact FP64 computation decides.  (The centre
 // test only matters where the side is wanted.)
+// The screen for the cell index alone, from num = pos - dmin: false where it
+// does not decide.
+__device__ __forceinline__ bool cell_screen(double num, float inv_cell32, float dmin_cells, int* k) {
+    const float q = d2f(num) * inv_cell32;
+    const float fl = floorf(q);
+    const float frac = q - fl;
+    const float m = (fabsf(q) + dmin_cells + 1.0f) * 0x1p-20f;
+    *k = (int)fl + 1;
+    return frac > m && frac < 1.0f - m;
+}
 // One coordinate: the cell index and, with want_side, whether the coordinate
 // lies above the cell's centre (*above; not computed otherwise).
 __device__ __forceinline__ int cell_component(double x, double dmin, double cell,

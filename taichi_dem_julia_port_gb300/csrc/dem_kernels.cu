@@ -1424,19 +1424,30 @@ __device__ __forceinline__ unsigned long long team_sum(unsigned long long v, con
 // buckets up to this step's largest, as the standalone scan), in tiles of
 // kScanTile: tile sums, a barrier, then each tile's prefix from the sums.
 // Ends with a barrier.
+// Lanes take four consecutive buckets each (16-byte loads and stores, a warp's
+// 512 bytes together).
 __device__ bool scan_phase(const DemDev& d, const DemParams& p, const Team& tm,
                            unsigned long long* red) {
     // (values written by other blocks earlier in this launch are read past L1)
     const long long lim = (long long)__ldcg(&d.ctr->bmax) + 1;
     const long long count = lim < (long long)p.T ? lim : (long long)p.T;
     const int ntiles = (int)((count + kScanTile - 1) / kScanTile);
-    const int items = (kScanTile + tm.nt - 1) / tm.nt;
+    auto four = [&](long long k) {  // buckets k .. k+3, zero past the range
+        if (k + 3 < count) return __ldcg(reinterpret_cast<const uint4*>(d.cell_count + k));
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (k < count) v.x = __ldcg(d.cell_count + k);
+        if (k + 1 < count) v.y = __ldcg(d.cell_count + k + 1);
+        if (k + 2 < count) v.z = __ldcg(d.cell_count + k + 2);
+        return v;
+    };
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * items;
-        const long long end = min(min(base + items, (long long)(t + 1) * kScanTile), count);
-        unsigned long long v = 0;
-#pragma unroll 8
-        for (long long k = base; k < end; ++k) v += d.cell_count[k];
+        const long long base = (long long)t * kScanTile;
+        unsigned v = 0;
+#pragma unroll 4
+        for (int k = 4 * (int)threadIdx.x; k < kScanTile; k += 4 * tm.nt) {
+            const uint4 x = four(base + k);
+            v += x.x + x.y + x.z + x.w;
+        }
         const unsigned long long tot = team_sum(v, tm, red);
         if (threadIdx.x == 0) d.tile_sums[t] = (uint32_t)tot;
     }
@@ -1444,31 +1455,50 @@ __device__ bool scan_phase(const DemDev& d, const DemParams& p, const Team& tm,
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         unsigned long long pre = 0;
         for (int u = threadIdx.x; u < t; u += tm.nt) pre += __ldcg(&d.tile_sums[u]);
-        pre = team_sum(pre, tm, red);
-        const long long base = (long long)t * kScanTile + (long long)threadIdx.x * items;
-        const long long end = min(min(base + items, (long long)(t + 1) * kScanTile), count);
-        unsigned long long mine = 0;
-#pragma unroll 8
-        for (long long k = base; k < end; ++k) mine += d.cell_count[k];
-        // exclusive prefix of `mine` across the team
-        unsigned long long x = mine;
+        unsigned run = (unsigned)team_sum(pre, tm, red);  // the particles in the buckets before
+        const long long base = (long long)t * kScanTile;
+        auto mine_of = [&](int k) {
+            return k < kScanTile ? four(base + k) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        uint4 next = mine_of(4 * (int)threadIdx.x);  // loaded a round ahead
+        for (int k0 = 0; k0 < kScanTile && base + k0 < count; k0 += 4 * tm.nt) {
+            const int k = k0 + 4 * (int)threadIdx.x;
+            const uint4 v = next;
+            next = mine_of(k + 4 * tm.nt);
+            const unsigned mine = v.x + v.y + v.z + v.w;
+            unsigned x = mine;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane_id() >= (unsigned)o) x += y;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane_id() >= (unsigned)o) x += y;
+            }
+            if (lane_id() == 31) red[threadIdx.x >> 5] = x;
+            tm.sync();
+            unsigned before = 0, all = 0;
+            for (int w = 0; w < tm.nt / 32; ++w) {
+                const unsigned r = (unsigned)red[w];
+                before += w < (int)(threadIdx.x >> 5) ? r : 0u;
+                all += r;
+            }
+            tm.sync();
+            if (k < kScanTile && base + k < count) {
+                uint4 o;
+                o.x = run + before + x - mine;
+                o.y = o.x + v.x;
+                o.z = o.y + v.y;
+                o.w = o.z + v.z;
+                // (the array has an entry past the last bucket, written below)
+                if (base + k + 3 < count) {
+                    *reinterpret_cast<uint4*>(d.cell_start + base + k) = o;
+                } else {
+                    d.cell_start[base + k] = o.x;
+                    if (base + k + 1 < count) d.cell_start[base + k + 1] = o.y;
+                    if (base + k + 2 < count) d.cell_start[base + k + 2] = o.z;
+                }
+            }
+            run += all;
         }
-        if (lane_id() == 31) red[threadIdx.x >> 5] = x;
-        tm.sync();
-        unsigned long long wpre = 0;
-        for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) wpre += red[w];
-        tm.sync();
-        unsigned long long run = pre + wpre + x - mine;
-#pragma unroll 8
-        for (long long k = base; k < end; ++k) {
-            d.cell_start[k] = (uint32_t)run;
-            run += d.cell_count[k];
-        }
-        if (t == ntiles - 1 && (int)threadIdx.x == tm.nt - 1) d.cell_start[count] = (uint32_t)run;
+        if (t == ntiles - 1 && threadIdx.x == 0) d.cell_start[count] = run;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr->cell_limit = (unsigned int)count;
     return grid_sync(d.ctr, tm);

@@ -52,8 +52,8 @@ constexpr size_t kWords = kTotalsOff + kBins;
 constexpr int kMaxDevices = 64;
 
 // The scratch: the first pass's output keys (0-based buckets) and particle
-// indices, the digit counts of every chunk (digit-major, scanned in place over
-// the chunks) and the digits' totals.
+// indices, the digit counts of every chunk (scanned in place over the chunks)
+// and the digits' totals.
 // Every word a call reads is written earlier in the same call, so nothing
 // needs clearing between calls.  Host code must not take this name as a
 // device address; it uses the address from cudaGetSymbolAddress (see
@@ -62,8 +62,8 @@ static __device__ __align__(256) uint32_t g_scratch[kWords];
 
 struct Geometry {
     double dmin[3];
-    double cell, inv_cell;
-    float inv_cell32, dmin_cells;  // the FP32 screen of the cell (cell_component)
+    double cell;
+    float inv_cell32, dmin_cells;  // the FP32 screen of the cell (cell_screen)
     int screen;                    // 0: the cell size is beyond the screen's range
     uint32_t H;
     uint32_t mask;
@@ -73,45 +73,57 @@ __device__ __forceinline__ uint32_t na_bucket(int x, int y, int z, const Geometr
     const uint32_t m = dem::morton1(x, y, z);
     return g.mask ? (m & g.mask) : (m % g.H);
 }
+// What the screen leaves open, out of line: eight particles' cells unrolled
+// with the exact divisions inline waited for instructions a third of the time
+// (1,000,000 particles: 23 us).
+static __device__ __noinline__ int na_cell_exact(double num, double cell) {
+    return dem::ceil_i32(__ddiv_rn(num, cell));
+}
 __device__ __forceinline__ int na_cell(double x, int c, const Geometry& g) {
-    if (g.screen)
-        return dem::cell_component(x, g.dmin[c], g.cell, g.inv_cell, g.inv_cell32, g.dmin_cells,
-                                   false, nullptr);
-    return dem::ceil_i32(__ddiv_rn(__dsub_rn(x, g.dmin[c]), g.cell));
+    const double num = __dsub_rn(x, g.dmin[c]);
+    int k;
+    if (g.screen && dem::cell_screen(num, g.inv_cell32, g.dmin_cells, &k)) return k;
+    return na_cell_exact(num, g.cell);
 }
 
 // cell + hashcode (src/utils.jl:1-2) of one chunk, the reference's 1-based
-// buckets, with the first pass's digit counts (digit-major: hist[digit · nblk
-// + chunk]).  The three quotients per particle were the whole sort's largest
-// cost as FP64 divisions (1,000,000 particles: 74 us of 166 us; GB300 retires
-// one FP64 warp-instruction per 64 cycles and SM sub-partition); the FP32
-// screen of cell_component decides all but the cells' edges (9 us with the
-// counts).
+// buckets, with the first pass's digit counts (hist[chunk · kBins + digit]).
+// The three quotients per particle were the whole sort's largest cost as FP64
+// divisions (1,000,000 particles: 74 us of 166 us; GB300 retires one FP64
+// warp-instruction per 64 cycles and SM sub-partition); the FP32 screen decides all but the cells' edges.
 __global__ void __launch_bounds__(kBlock)
     k_na_hash(const double* __restrict__ px, const double* __restrict__ py,
-              const double* __restrict__ pz, int n, Geometry g, int nblk, uint32_t* bucket_out,
+              const double* __restrict__ pz, int n, Geometry g, uint32_t* bucket_out,
               uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kBins];
+    const int base = blockIdx.x * kChunk + (int)threadIdx.x;
+    double x[kItems], y[kItems], z[kItems];
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int i = base + q * kBlock;
+        x[q] = i < n ? px[i] : 0.0;
+        y[q] = i < n ? py[i] : 0.0;
+        z[q] = i < n ? pz[i] : 0.0;
+    }
     for (int b = threadIdx.x; b < kBins; b += kBlock) h[b] = 0u;
     __syncthreads();
-    const int base = blockIdx.x * kChunk + (int)threadIdx.x;
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
         const int i = base + q * kBlock;
         if (i < n) {
-            const int cx = na_cell(px[i], 0, g), cy = na_cell(py[i], 1, g), cz = na_cell(pz[i], 2, g);
-            const uint32_t b = na_bucket(cx, cy, cz, g);
+            const uint32_t b = na_bucket(na_cell(x[q], 0, g), na_cell(y[q], 1, g),
+                                         na_cell(z[q], 2, g), g);
             bucket_out[i] = b + 1u;
             atomicAdd(&h[b & (kBins - 1)], 1u);
         }
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)b * nblk + blockIdx.x] = h[b];
+    for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)blockIdx.x * kBins + b] = h[b];
 }
 
 // Digit counts of one chunk's keys for a later pass.
 __global__ void __launch_bounds__(kBlock)
-    k_na_digit_count(const uint32_t* __restrict__ keys, int n, int shift, int nblk,
+    k_na_digit_count(const uint32_t* __restrict__ keys, int n, int shift,
                      uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kBins];
     for (int b = threadIdx.x; b < kBins; b += kBlock) h[b] = 0u;
@@ -128,30 +140,41 @@ __global__ void __launch_bounds__(kBlock)
             atomicAdd(&h[d], (uint32_t)__popc(peers));
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)b * nblk + blockIdx.x] = h[b];
+    for (int b = threadIdx.x; b < kBins; b += kBlock) hist[(size_t)blockIdx.x * kBins + b] = h[b];
 }
 
-// One warp per digit: its counts over the chunks become running sums, in
-// place, and its total.
-__global__ void k_na_digit_rows(uint32_t* hist, int nblk, uint32_t* totals) {
-    const unsigned lane = threadIdx.x & 31u;
-    const int d = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    if (d >= kBins) return;
-    uint32_t* row = hist + (size_t)d * nblk;
-    uint32_t carry = 0;
-    for (int b0 = 0; b0 < nblk; b0 += 32) {
-        const int b = b0 + (int)lane;
-        const uint32_t v = b < nblk ? row[b] : 0u;
-        uint32_t x = v;
+// Every digit's counts over the chunks become running sums, in place, and its
+// total: 32 digits per block, one per lane (128-byte rows), the chunks split
+// over the block's warps.
+constexpr int kRowWarps = 16;
+constexpr int kRowItems = (int)(kMaxBlocks / kRowWarps);
+__global__ void __launch_bounds__(32 * kRowWarps)
+    k_na_digit_rows(uint32_t* hist, int nblk, uint32_t* totals) {
+    __shared__ uint32_t sums[kRowWarps][32];
+    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+    const int d = blockIdx.x * 32 + lane;
+    const int per = (nblk + kRowWarps - 1) / kRowWarps, b0 = warp * per;
+    uint32_t v[kRowItems];
+    uint32_t sum = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= (unsigned)o) x += y;
-        }
-        if (b < nblk) row[b] = carry + x - v;
-        carry += __shfl_sync(0xffffffffu, x, 31);
+    for (int k = 0; k < kRowItems; ++k) {
+        v[k] = k < per && b0 + k < nblk ? hist[(size_t)(b0 + k) * kBins + d] : 0u;
+        sum += v[k];
     }
-    if (lane == 0) totals[d] = carry;
+    sums[warp][lane] = sum;
+    __syncthreads();
+    uint32_t run = 0, all = 0;
+    for (int w = 0; w < kRowWarps; ++w) {
+        const uint32_t t = sums[w][lane];
+        run += w < warp ? t : 0u;
+        all += t;
+    }
+#pragma unroll
+    for (int k = 0; k < kRowItems; ++k) {
+        if (k < per && b0 + k < nblk) hist[(size_t)(b0 + k) * kBins + d] = run;
+        run += v[k];
+    }
+    if (warp == 0) totals[d] = all;
 }
 
 // Exclusive scan of kBins values, two per thread (v: this thread's pair).
@@ -175,7 +198,8 @@ __device__ __forceinline__ uint2 block_scan_bins(uint2 v, uint32_t* warp_sums) {
 
 // Stable scatter of one chunk's (key, index) pairs by the digit at `shift`.
 // Each warp ranks its own 256 consecutive elements, 32 per round
-// (__match_any_sync groups equal digits), in a digit table of its own; the
+// (same_digit groups equal digits by one ballot per bit, 63 -> 59 us for the
+// whole sort of 1,000,000 against __match_any_sync), in a digit table of its own; the
 // tables' running sums over the warps, in order, then place every element
 // after the earlier elements of its digit, so the order inside a digit is the
 // input order.  The chunk is put in digit order in shared memory and written
@@ -183,6 +207,16 @@ __device__ __forceinline__ uint2 block_scan_bins(uint2 v, uint32_t* warp_sums) {
 // elements and every element written from its own thread the two scatters of
 // 1,000,000 particles took 26 and 13 us.)  idx_in == nullptr: the indices
 // are the positions.
+__device__ __forceinline__ unsigned same_digit(uint32_t d, bool valid) {
+    unsigned m = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < kDigitBits; ++b) {
+        const bool one = (d >> b) & 1u;
+        const unsigned v = __ballot_sync(0xffffffffu, one);
+        m &= one ? v : ~v;
+    }
+    return m;
+}
 struct ScatterShared {
     uint16_t cnt[kWarps][kBins];
     uint32_t key[kChunk], idx[kChunk];
@@ -191,7 +225,7 @@ struct ScatterShared {
 };
 __global__ void __launch_bounds__(kBlock)
     k_na_digit_scatter(const uint32_t* __restrict__ keys, uint32_t bias,
-                       const uint32_t* __restrict__ idx_in, int n, int shift, int nblk,
+                       const uint32_t* __restrict__ idx_in, int n, int shift,
                        const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals,
                        uint32_t* __restrict__ keys_out, uint32_t* __restrict__ idx_out) {
     extern __shared__ unsigned char raw[];
@@ -209,8 +243,7 @@ __global__ void __launch_bounds__(kBlock)
     }
     const int d0 = 2 * (int)threadIdx.x;
     const uint2 tot = make_uint2(totals[d0], totals[d0 + 1]);
-    const uint2 row = make_uint2(hist[(size_t)d0 * nblk + blockIdx.x],
-                                 hist[(size_t)(d0 + 1) * nblk + blockIdx.x]);
+    const uint2 row = *reinterpret_cast<const uint2*>(hist + (size_t)blockIdx.x * kBins + d0);
     uint32_t* zero = reinterpret_cast<uint32_t*>(&sh.cnt[0][0]);
     for (int b = threadIdx.x; b < kWarps * kBins / 2; b += kBlock) zero[b] = 0u;
     __syncthreads();
@@ -218,8 +251,8 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
         const bool valid = e0 + r * 32 < m;
-        const uint32_t d = valid ? (key[r] >> shift) & (kBins - 1) : (uint32_t)kBins;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t d = (key[r] >> shift) & (kBins - 1);
+        const unsigned peers = same_digit(d, valid);
         uint32_t before = 0;
         if (valid) before = sh.cnt[warp][d];
         __syncwarp();
@@ -330,9 +363,8 @@ extern "C" int dem_bucket_sort_noalloc(const double* px, const double* py, const
         dm = std::fmax(dm, std::fabs(g.dmin[c]));
     }
     g.cell = cell_size;
-    g.inv_cell = 1.0 / cell_size;
-    g.inv_cell32 = (float)g.inv_cell;
-    g.dmin_cells = (float)(dm * g.inv_cell * 1.001);
+    g.inv_cell32 = (float)(1.0 / cell_size);
+    g.dmin_cells = (float)(dm / cell_size * 1.001);
     g.screen = cell_size > 0x1p-100 && cell_size < 0x1p100;
     g.H = (uint32_t)hash_table_size;
     g.mask = (g.H & (g.H - 1)) == 0 ? g.H - 1 : 0u;
@@ -340,7 +372,7 @@ extern "C" int dem_bucket_sort_noalloc(const double* px, const double* py, const
     // buckets are 0 .. H-1 < 2^20: one 10-bit pass for H <= 1,024, else two
     const int passes = hash_table_size <= kBins ? 1 : 2;
     const int nblk = (nn + kChunk - 1) / kChunk;
-    k_na_hash<<<nblk, kBlock, 0, s>>>(px, py, pz, nn, g, nblk, bucket, hist);
+    k_na_hash<<<nblk, kBlock, 0, s>>>(px, py, pz, nn, g, bucket, hist);
     if (!launched()) return DEM_ERR_CUDA;
     for (int pass = 0; pass < passes; ++pass) {
         const int shift = pass * kDigitBits;
@@ -349,13 +381,13 @@ extern "C" int dem_bucket_sort_noalloc(const double* px, const double* py, const
         const uint32_t bias = pass == 0 ? 1u : 0u;  // the outputs' buckets are 1-based
         const uint32_t* iin = pass == 0 ? nullptr : idx_tmp;
         if (pass > 0) {
-            k_na_digit_count<<<nblk, kBlock, 0, s>>>(kin, nn, shift, nblk, hist);
+            k_na_digit_count<<<nblk, kBlock, 0, s>>>(kin, nn, shift, hist);
             if (!launched()) return DEM_ERR_CUDA;
         }
-        k_na_digit_rows<<<kBins / 8, 256, 0, s>>>(hist, nblk, totals);
+        k_na_digit_rows<<<kBins / 32, 32 * kRowWarps, 0, s>>>(hist, nblk, totals);
         if (!launched()) return DEM_ERR_CUDA;
         k_na_digit_scatter<<<nblk, kBlock, sizeof(ScatterShared), s>>>(
-            kin, bias, iin, nn, shift, nblk, hist, totals, last ? nullptr : keys_tmp,
+            kin, bias, iin, nn, shift, hist, totals, last ? nullptr : keys_tmp,
             last ? sorted : idx_tmp);
         if (!launched()) return DEM_ERR_CUDA;
     }
