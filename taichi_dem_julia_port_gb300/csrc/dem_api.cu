@@ -532,7 +532,9 @@ int allocate(DemHandle* h) {
         TRY(dalloc(h, &d.row_len[b], n));
     }
     TRY(dalloc(h, &d.qmask, (n + 31) / 32));
-    CU(cudaMemsetAsync(d.qmask, 0xff, (n + 31) / 32 * sizeof(uint32_t), h->stream));
+    TRY(dalloc(h, &d.smask, (n + 31) / 32));
+    for (uint32_t* m : {d.qmask, d.smask})
+        CU(cudaMemsetAsync(m, 0xff, (n + 31) / 32 * sizeof(uint32_t), h->stream));
     TRY(dalloc(h, &d.stash, n * (size_t)h->p.kstash));
     TRY(dalloc(h, &d.keep, cap));
     TRY(dalloc(h, &d.tlist, cap));
@@ -792,11 +794,13 @@ void record_step(DemHandle* h, int cur, bool report) {
     launch_force(h->d, p, nxt, h->multi, h->shape, h->stream);
     launch_integrate(h->d, p, cur, h->multi, h->shape, h->stream);
 }
-// Every quaternion bit of slots [p0, p0 + n) set (DemDev::qmask).
+// Every quaternion and wall-shear bit of slots [p0, p0 + n) set (DemDev::qmask,
+// smask).
 int mark_turned(DemHandle* h, int64_t p0, int64_t n) {
     if (n <= 0) return DEM_OK;
     const size_t w0 = (size_t)p0 / 32, w1 = (size_t)(p0 + n - 1) / 32;
-    CU(cudaMemsetAsync(h->d.qmask + w0, 0xff, (w1 - w0 + 1) * sizeof(uint32_t), h->stream));
+    for (uint32_t* m : {h->d.qmask, h->d.smask})
+        CU(cudaMemsetAsync(m + w0, 0xff, (w1 - w0 + 1) * sizeof(uint32_t), h->stream));
     return DEM_OK;
 }
 
@@ -1619,7 +1623,7 @@ int dem_set_launch_shape(DemHandle* h, const DemLaunchShape* sh) {
     h->p.dep = h->shape.dependent_launch;
     h->p.list_lanes = h->shape.list_lanes;
     drop_graphs(h);
-    // layouts other than the one-thread integrator's keep no quaternion bits
+    // layouts other than the one-thread integrator's keep no such bits
     return mark_turned(h, 0, h->n_cap);
 }
 

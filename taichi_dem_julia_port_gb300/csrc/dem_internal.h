@@ -190,6 +190,9 @@ struct DemDev {
     // they are).  Set by the integrator where a spin appears, and for every
     // slot by whatever else writes spins or orientations.
     uint32_t* qmask;
+    // the same for the wall-shear columns: a clear bit means that they hold
+    // zeros (the one-thread integrator then leaves them unwritten)
+    uint32_t* smask;
     double *m, *inv_m, *r, *r0, *inv_inertia;
     double *b_invA, *b_rbI;        // bond section constants for rb = ρ·r (1/A, rb/I)
     double *b_EA, *b_EI, *b_phic;  // E·A, E·I and 20/3·(1+ν)·rb² for rb = ρ·r
@@ -205,7 +208,8 @@ struct DemDev {
     const MatTables* mt;                  // tables of a dem_create_tables handle, else null
     const uint8_t* mid;                   // its grains' material indices, else null
     int32_t* scene_of;                    // arena: scene of each slot (-1 free); null otherwise
-    // neighbour lists: kvl partners per slot, their count, the position at the
+    // neighbour lists: kvl partners per slot (entry v of slot i at
+    // [v * wstride + i]: consecutive slots' entries together), their count, the position at the
     // last full search and the current position (FP32, relative to the
     // scene's domain_min, .w = reach32); rebuild flags per scene and buffer
     int32_t* vl;
@@ -239,7 +243,8 @@ struct DemDev {
                           // bonds at [0, bonds), the others at cap-1-k, k in
                           // [0, rows - bonds)
     int32_t* in_cnt;      // zero between steps
-    int2* in_list;        // n * kin: (contact slot, owner i) of contacts where the particle is j
+    int2* in_list;        // kin * n: entry u of slot j at [u * wstride + j], (contact slot, owner i)
+                          // of the contacts where the particle is j
     // Contact columns 𝐅ᵢ, 𝛕ᵢ, 𝛕ⱼ hold FP64 values in the FP64 force mode and
     // FP32 (hi, lo) pairs in the FP32 force mode.
     double* contrib;      // 9 * cap, [field][contact]
@@ -265,7 +270,7 @@ struct DemParams {
     int debug_enum; // 1: the pair search counts its candidate pairs (never in a graph)
     int tab;        // 1: a single scene with material / wall tables (DemDev::mt, mid)
     int list_lanes; // neighbour-list update: 0 auto, 1 or 4 lanes per particle
-    int wstride;    // slots per wall-shear column
+    int wstride;    // slots per wall-shear column and per row of vl and in_list
     int report;     // 1: a step stores what only its caller reads (contact points, Hertz
                     // forces, force and moment totals); 0: a later step of the call does
     SceneParams s0; // the scene of a single-scene handle

@@ -652,7 +652,7 @@ __device__ __forceinline__ void detect_group(const DemDev& d, const DemParams& p
     int seg = 0, segoff = sh.seg[0].x, nextb = sh.seg[1].y;
     // the neighbour list is rebuilt with this search (not for held scenes)
     const bool build = !frozen;
-    int32_t* vl = d.vl + (size_t)i * p.kvl;
+    int32_t* vl = d.vl + i;
     const float skin = S.f_skin;
     unsigned long long en = 0, eh = 0;  // inspection: pairs visited, their checksum
     for (int c0 = 0; c0 < total; c0 += kLanes * kBatch) {
@@ -689,7 +689,7 @@ __device__ __forceinline__ void detect_group(const DemDev& d, const DemParams& p
             const bool near = maybe_touching32(P32, qq[u], skin);
             if (build && near) {
                 const int vs = atomicAdd(&sh.nvl, 1);
-                if (vs < p.kvl) vl[vs] = j;
+                if (vs < p.kvl) vl[(size_t)vs * p.wstride] = j;
             }
             // a touching pair is near and passes the FP32 pre-filter; bond
             // initialisation tests r₀, with the pre-filter's reaches scaled
@@ -908,9 +908,9 @@ __device__ __forceinline__ void list_particle(const DemDev& d, const DemParams& 
     int32_t* stash = d.stash + (size_t)i * p.kstash;
     if (!frozen) {
         const float4 Pi = d.pos32[i];
-        const int32_t* vl = d.vl + (size_t)i * p.kvl;
+        const int32_t* vl = d.vl + i;
         for (int v = lane; v < nv; v += kVLanes) {
-            const int j = vl[v];
+            const int j = vl[(size_t)v * p.wstride];
             // a partner already in the row (a bond, a Hertz contact)
             // needs no position: the row is checked first
             bool found = false;
@@ -995,7 +995,7 @@ __device__ __forceinline__ void list_particle1(const DemDev& d, const DemParams&
                                                int e0, int e1, int nv, bool frozen, RowJob& job,
                                                unsigned long long& keepm) {
     const ContactSoA o = d.c[cur];
-    const int32_t* vl = d.vl + (size_t)i * p.kvl;
+    const int32_t* vl = d.vl + i;
     // the first entry, the first list partner and the particle's own FP32
     // position are loaded together (most rows and lists hold one)
     uint32_t fl0 = e0 < e1 ? o.fl[e0] : 0u;
@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void list_particle1(const DemDev& d, const DemParams&
     int nnew = 0;
     if (!frozen) {
         for (int v = 0; v < nv; ++v) {
-            const int j = v == 0 ? v0 : vl[v];
+            const int j = v == 0 ? v0 : vl[(size_t)v * p.wstride];
             bool found = (fl0 & kActive) && j == j0;
             for (int e = e0 + 1; e < e1 && !found; ++e)
                 found = (o.cj[e] == j) && (o.fl[e] & kActive);
@@ -1186,7 +1186,7 @@ __device__ __forceinline__ void list_quads(const DemDev& d, const DemParams& p, 
     const bool has = gl < len;
     const uint32_t fl = has ? o.fl[e] : 0u;
     const int cj = has ? o.cj[e] : -1;
-    const int vj = gl < nv ? d.vl[(size_t)i * p.kvl + gl] : -1;
+    const int vj = gl < nv ? d.vl[(size_t)gl * p.wstride + i] : -1;
     const bool alive = (fl & kActive) != 0u, bond = alive && (fl & kBonded);
     const int row = alive ? cj : -1;
     bool found = vj < 0;  // a partner already in the row (a bond, a Hertz contact)
@@ -2402,7 +2402,7 @@ __device__ __forceinline__ int force_body(const DemDev& d, const DemParams& p, i
         // sorts the list by owner, so the order of registration is free)
         const int slot = atomicAdd(&d.in_cnt[j], 1);
         auto enlist = [&]() {
-            if (slot < p.kin) d.in_list[(size_t)j * p.kin + slot] = make_int2(c, i);
+            if (slot < p.kin) d.in_list[(size_t)slot * p.wstride + j] = make_int2(c, i);
             else raise_error(d.ctr, kErrCapacity);
         };
         if (!LATE) enlist();
@@ -2511,10 +2511,10 @@ __device__ __forceinline__ void gather(const DemDev& d, const DemParams& p, int 
     const T* cb = contrib_of<T>(d);
     nin = nin < p.kin ? nin : p.kin;
     nin = nin < kMaxIncoming ? nin : kMaxIncoming;
-    const int2* il = d.in_list + (size_t)i * p.kin;
+    const int2* il = d.in_list + i;  // entry u at u * wstride
     int2 v4[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v4[u] = u < nin ? il[u] : make_int2(0, 0x7fffffff);
+    for (int u = 0; u < 4; ++u) v4[u] = u < nin ? il[(size_t)u * p.wstride] : make_int2(0, 0x7fffffff);
     const int c1 = min(c0 + len, p.cap);
     int c = c0;
     for (; c + 1 < c1; c += 2) {
@@ -2547,12 +2547,12 @@ __device__ __forceinline__ void gather(const DemDev& d, const DemParams& p, int 
     } else if (nin <= 8) {
         int2 v8[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v8[u] = u < 4 ? v4[u] : (u < nin ? il[u] : make_int2(0, 0x7fffffff));
+        for (int u = 0; u < 8; ++u) v8[u] = u < 4 ? v4[u] : (u < nin ? il[(size_t)u * p.wstride] : make_int2(0, 0x7fffffff));
         add_incoming<T, 8>(d, cap, v8, nin, F, M);
     } else {
         int2 inc[kMaxIncoming];
         for (int u = 0; u < nin; ++u) {
-            const int2 v = il[u];
+            const int2 v = il[(size_t)u * p.wstride];
             int b = u - 1;
             while (b >= 0 && inc[b].y > v.y) {
                 inc[b + 1] = inc[b];
@@ -2596,8 +2596,8 @@ struct WallK {
 // resolve_wall! for one particle and one wall (src/kernels.jl:317-426):
 // whether the wall touches the particle and, if so, the wall's force g and
 // moment mw on it; updates the wall contact's shear history (*wsx, *wsy,
-// *wsz; zero when not touching); `count`: this thread adds to the scene's
-// warning counters.  An FP32 screen on the
+// *wsz; zero when not touching, written unless `clear` says that it is zero
+// already); `count`: this thread adds to the scene's warning counters.  An FP32 screen on the
 // step's starting position (pos32, within 2^-24 of the FP64 one per
 // coordinate) skips the exact test when |n·x - d| exceeds r by a margin that
 // covers its rounding.
@@ -2605,7 +2605,8 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
                                            float4 p32, float r32, double x, double y, double z,
                                            double vx, double vy, double vz, double wx, double wy,
                                            double wz, double r, double m, double* wsx, double* wsy,
-                                           double* wsz, double g[3], double mw[3], bool count) {
+                                           double* wsz, double g[3], double mw[3], bool count,
+                                           bool clear = true) {
     bool wall_near;
     {
         const float4 q = p32;
@@ -2615,9 +2616,11 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
         wall_near = !(fabsf(Lf) > rf + mg);
     }
     if (!wall_near) {
-        *wsx = 0.0;
-        *wsy = 0.0;
-        *wsz = 0.0;
+        if (clear) {
+            *wsx = 0.0;
+            *wsy = 0.0;
+            *wsz = 0.0;
+        }
         return false;
     }
     const double dotkn = __dadd_rn(__dadd_rn(__dmul_rn(x, W.wn[0]), __dmul_rn(y, W.wn[1])),
@@ -2667,20 +2670,25 @@ __device__ __forceinline__ bool wall_force(const DemDev& d, int sc, const WallK&
         *wsz = sz;
         return true;
     }
-    *wsx = 0.0;
-    *wsy = 0.0;
-    *wsz = 0.0;
+    if (clear) {
+        *wsx = 0.0;
+        *wsy = 0.0;
+        *wsz = 0.0;
+    }
     return false;
 }
-// resolve_wall! adding the wall's force and moment to F, M
-__device__ __forceinline__ void wall_contact(const DemDev& d, int sc, const WallK& W, double dt,
+// resolve_wall! adding the wall's force and moment to F, M; returns whether it
+// touches
+__device__ __forceinline__ bool wall_contact(const DemDev& d, int sc, const WallK& W, double dt,
                                              float4 p32, float r32, double x, double y, double z,
                                              double vx, double vy, double vz, double wx, double wy,
                                              double wz, double r, double m, double* wsx,
-                                             double* wsy, double* wsz, double F[3], double M[3]) {
+                                             double* wsy, double* wsz, bool clear, double F[3],
+                                             double M[3]) {
     double g[3], mw[3];
-    if (wall_force(d, sc, W, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m, wsx, wsy, wsz, g,
-                   mw, true)) {
+    const bool touch = wall_force(d, sc, W, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m,
+                                  wsx, wsy, wsz, g, mw, true, clear);
+    if (touch) {
         F[0] += g[0];
         F[1] += g[1];
         F[2] += g[2];
@@ -2688,6 +2696,7 @@ __device__ __forceinline__ void wall_contact(const DemDev& d, int sc, const Wall
         M[1] += mw[1];
         M[2] += mw[2];
     }
+    return touch;
 }
 
 // QUAT: with the quaternions (otherwise k_list1 has updated them)
@@ -2711,11 +2720,18 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     const int row0 = d.row_start[nxt][i], rlen = d.row_len[nxt][i], nin = d.in_cnt[i];
     const double x = d.px[i], y = d.py[i], z = d.pz[i];
     const double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-    const double wx = d.wx[i], wy = d.wy[i], wz = d.wz[i];
+    // a clear quaternion bit: no spin (and the identity orientation)
+    const uint32_t qword = d.qmask[i >> 5];
+    const bool bit = (qword >> lane_id()) & 1u;
+    double wx = 0.0, wy = 0.0, wz = 0.0;
+    if (bit) {
+        wx = d.wx[i];
+        wy = d.wy[i];
+        wz = d.wz[i];
+    }
     const double r = d.r[i], m = d.m[i];
     const double invm = d.inv_m[i], ii = d.inv_inertia[i];
-    const uint32_t qword = d.qmask[i >> 5];
-    const bool turned = QUAT && ((qword >> lane_id()) & 1u);
+    const bool turned = QUAT && bit;
     double q4[4] = {0.0, 0.0, 0.0, 0.0};
     if (turned) {
         q4[0] = d.qw[i];
@@ -2724,7 +2740,9 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
         q4[3] = d.qz[i];
     }
     const float4 p32 = d.pos32[i], xr = d.xref[i];
-    const float r32 = d.rm32[i].z;
+    const float r32 = d2f(r);  // the FP32 record's radius, without its 16 bytes
+    const uint32_t sword = d.smask[i >> 5];
+    bool shear = (sword >> lane_id()) & 1u;  // the slot's wall shear may be nonzero
     double F[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
     if constexpr (F32) {
         float Ff[3] = {0.0f, 0.0f, 0.0f}, Mf[3] = {0.0f, 0.0f, 0.0f};
@@ -2737,27 +2755,31 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     } else {
         gather<double>(d, p, i, row0, rlen, nin, F, M);
     }
-    d.in_cnt[i] = 0;
+    if (nin) d.in_cnt[i] = 0;
     const double dt = S.dt;
     // resolve_wall! (src/kernels.jl:317-426): the scene's one wall, or every
     // wall of a table scene in order (wall j's force and moment are added
     // after wall j-1's, as the reference's per-particle loop over j does)
+    bool touched = false;
     if constexpr (TAB) {
         const MatTables& T = *d.mt;
         const int a = d.mid[i];
+        touched = shear && T.nwall == 0;
         for (int wl = 0; wl < T.nwall; ++wl) {
             const WallConst& W = T.wall[wl];
             const WallK K{W.wn, W.wd, W.wR, W.wRinv, W.f_wn, W.f_wc0, W.mu[a], W.Ys[a], W.Gs[a],
                           W.cgn[a], W.cgt[a]};
             const size_t o = (size_t)wl * p.wstride + i;
-            wall_contact(d, sc, K, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m, d.wsx + o,
-                         d.wsy + o, d.wsz + o, F, M);
+            touched |= wall_contact(d, sc, K, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m,
+                                    d.wsx + o, d.wsy + o, d.wsz + o, shear, F, M);
         }
     } else if (S.has_wall) {
         const WallK K{S.wn, S.wd, S.wR, S.wRinv, S.f_wn, S.f_wc0, S.pw_mu, S.pw_Ys, S.pw_Gs,
                       S.pw_cgn, S.pw_cgt};
-        wall_contact(d, sc, K, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m, d.wsx + i,
-                     d.wsy + i, d.wsz + i, F, M);
+        touched = wall_contact(d, sc, K, dt, p32, r32, x, y, z, vx, vy, vz, wx, wy, wz, r, m,
+                               d.wsx + i, d.wsy + i, d.wsz + i, shear, F, M);
+    } else {
+        touched = shear;  // no wall: nothing is written
     }
     // apply_body_force!  A zero gravity component adds nothing: the force sum
     // starts at +0 and never becomes -0, so F + 0·m is F.
@@ -2825,8 +2847,12 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
         // updated (QUAT), set where a spin will turn the particle
         const unsigned am = __activemask();
         const unsigned on = __ballot_sync(am, spin), looked = __ballot_sync(am, QUAT);
-        const uint32_t next = (qword & ~looked) | on;
-        if (lane_id() == (unsigned)(__ffs(am) - 1) && next != qword) d.qmask[i >> 5] = next;
+        const unsigned held = __ballot_sync(am, touched);
+        const uint32_t next = (qword & ~looked) | on, hold = (sword & ~am) | held;
+        if (lane_id() == (unsigned)(__ffs(am) - 1)) {
+            if (next != qword) d.qmask[i >> 5] = next;
+            if (hold != sword) d.smask[i >> 5] = hold;
+        }
     }
     if (p.report) {  // nobody can read the totals of a step inside a call
         d.fx[i] = F[0];
@@ -2889,10 +2915,10 @@ __device__ __forceinline__ void gather_component(const DemDev& d, const DemParam
     const T* cmj = cb + (size_t)(6 + qc) * cap;  // the partner's moment
     nin = nin < p.kin ? nin : p.kin;
     nin = nin < kMaxIncoming ? nin : kMaxIncoming;
-    const int2* il = d.in_list + (size_t)i * p.kin;
+    const int2* il = d.in_list + i;  // entry u at u * wstride
     int2 v4[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v4[u] = u < nin ? il[u] : make_int2(0, 0x7fffffff);
+    for (int u = 0; u < 4; ++u) v4[u] = u < nin ? il[(size_t)u * p.wstride] : make_int2(0, 0x7fffffff);
     const int c1 = min(c0 + len, p.cap);
     for (int c = c0; c < c1; c += 4) {  // four entries' loads at a time
         T a[4], m[4];
@@ -2914,12 +2940,12 @@ __device__ __forceinline__ void gather_component(const DemDev& d, const DemParam
     } else if (nin <= 8) {
         int2 v8[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v8[u] = u < 4 ? v4[u] : (u < nin ? il[u] : make_int2(0, 0x7fffffff));
+        for (int u = 0; u < 8; ++u) v8[u] = u < 4 ? v4[u] : (u < nin ? il[(size_t)u * p.wstride] : make_int2(0, 0x7fffffff));
         add_incoming_component<T, 8>(cf, cmj, v8, nin, F, M);
     } else {
         int2 inc[kMaxIncoming];
         for (int u = 0; u < nin; ++u) {
-            const int2 v = il[u];
+            const int2 v = il[(size_t)u * p.wstride];
             int b = u - 1;
             while (b >= 0 && inc[b].y > v.y) {
                 inc[b + 1] = inc[b];
@@ -3303,12 +3329,12 @@ __device__ __forceinline__ void integrate_split_block(const DemDev& d, const Dem
 // its FP64 work per particle is small enough that more resident warps hide
 // the state loads better than the extra registers would.
 template <bool MULTI, bool QUAT>
-__global__ void __launch_bounds__(kThreads) k_integrate(DemDev d, DemParams p, int cur) {
+__global__ void __launch_bounds__(kThreads, 2) k_integrate(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
     integrate_body<MULTI, false, false, QUAT>(d, p, cur);
 }
 template <bool QUAT>
-__global__ void __launch_bounds__(kThreads) k_integrate_tab(DemDev d, DemParams p, int cur) {
+__global__ void __launch_bounds__(kThreads, 2) k_integrate_tab(DemDev d, DemParams p, int cur) {
     dep_begin(p.dep == 2);
     integrate_body<false, false, true, QUAT>(d, p, cur);
 }
