@@ -1796,8 +1796,8 @@ __device__ __forceinline__ Frame contact_frame(double dx, double dy, double dz, 
     // f = (1 - a₁)/s² = 1/(1 + a₁), since s² = 1 - a₁²: three FP64
     // instructions fewer, and well conditioned away from a₁ = -1.  That the
     // degenerate branch is far (s² well above 4·tolerance²) is seen in FP32.
-    const float y = d2f(ay), z = d2f(az);
-    if (y * y + z * z > S.f_tol8 && d2f(ax) > -0.5f) {
+    const float y = d2f_coarse(ay), z = d2f_coarse(az);
+    if (y * y + z * z > S.f_tol8 && d2f_coarse(ax) > -0.5f) {
         F.f = rcp_nr(__dadd_rn(1.0, ax));  // in (0.5, 2]
         return F;
     }
@@ -1862,11 +1862,12 @@ __device__ __forceinline__ bool bond_breaks(const Vec3<double>& F, const Vec3<do
 // Breakage decision of bond_breaks behind an FP32 screen.  The three stresses
 // σc = fa + rb/I·sqrt(amax), σt = -fa - rb/I·sqrt(amin) and
 // σs = |τᵢ₁|·rb/2/I + 4/3/A·sqrt(F₂²+F₃²) are evaluated in FP32 from the FP64
-// values; each FP32 result lies within 2^-20 (|terms| + |threshold|) of the
-// exact one, so when every stress is below its threshold by 2^-16 of that
-// scale the bond cannot break and the FP64 test is skipped.  Otherwise (and for
-// NaN or out-of-range values, which fail every comparison) the FP64 test
-// decides, so the outcome is always that of bond_breaks.
+// values; each FP32 result lies within 2^-18 (|terms| + |threshold|) of the
+// exact one (the FP64 mode's coarse conversions are off by up to 2^-20, what
+// else is rounded by far less), so when every stress is below its threshold
+// by 2^-16 of that scale the bond cannot break and the FP64 test is skipped.
+// Otherwise (and for NaN or out-of-range values, which fail every comparison)
+// the FP64 test decides, so the outcome is always that of bond_breaks.
 __device__ __forceinline__ double pair_value(float2 v) { return (double)v.x + (double)v.y; }
 
 // bond_breaks on FP32 hi/lo pairs (out of line: the FP32 screen settles
@@ -1911,9 +1912,9 @@ __device__ __forceinline__ bool bond_breaks_fp64(const Vec3<double>& F, const Ve
                                                  const Vec3<double>& tj, float iA, float rb,
                                                  const DemDev& d, int small,
                                                  const SceneParams& p) {
-    const Vec3<float> Ff{d2f(F.x), d2f(F.y), d2f(F.z)};
-    const Vec3<float> tif{d2f(ti.x), d2f(ti.y), d2f(ti.z)};
-    const Vec3<float> tjf{d2f(tj.x), d2f(tj.y), d2f(tj.z)};
+    const Vec3<float> Ff{d2f_coarse(F.x), d2f_coarse(F.y), d2f_coarse(F.z)};
+    const Vec3<float> tif{d2f_coarse(ti.x), d2f_coarse(ti.y), d2f_coarse(ti.z)};
+    const Vec3<float> tjf{d2f_coarse(tj.x), d2f_coarse(tj.y), d2f_coarse(tj.z)};
     if (stress_clear(Ff, tif, tjf, iA, rb, p.f_sc, p.f_st, p.f_ss)) return false;
     return bond_breaks_d(F, ti, tj, d.b_invA[small], d.b_rbI[small], p);
 }
@@ -1930,9 +1931,9 @@ __device__ __forceinline__ bool bond_breaks_tab(const Vec3<double>& F, const Vec
                                                 const Vec3<double>& tj, float iA, float rbI,
                                                 double A, double I, double rb,
                                                 const PairConst& pc) {
-    const Vec3<float> Ff{d2f(F.x), d2f(F.y), d2f(F.z)};
-    const Vec3<float> tif{d2f(ti.x), d2f(ti.y), d2f(ti.z)};
-    const Vec3<float> tjf{d2f(tj.x), d2f(tj.y), d2f(tj.z)};
+    const Vec3<float> Ff{d2f_coarse(F.x), d2f_coarse(F.y), d2f_coarse(F.z)};
+    const Vec3<float> tif{d2f_coarse(ti.x), d2f_coarse(ti.y), d2f_coarse(ti.z)};
+    const Vec3<float> tjf{d2f_coarse(tj.x), d2f_coarse(tj.y), d2f_coarse(tj.z)};
     if (stress_clear(Ff, tif, tjf, iA, rbI, pc.f_sc, pc.f_st, pc.f_ss)) return false;
     return bond_breaks_tab_d(F, ti, tj, A, I, rb, pc);
 }
@@ -3946,6 +3947,13 @@ __global__ void k_selftest_conv(long long n, unsigned long long seed, unsigned l
     const unsigned long long c = (unsigned long long)__double_as_longlong(f2d(f));
     const unsigned long long e = (unsigned long long)__double_as_longlong((double)f);
     if (a != b) atomicAdd(bad, 1ull);
+    // d2f_coarse: within 2^-20 of x (and not above it) where binary32 is
+    // normal, below that range under it, infinite above it
+    const double ax = fabs(x), ac = fabs((double)d2f_coarse(x));
+    const bool coarse = ax < 0x1p-126 ? ac < 0x1p-126
+                        : ax < 0x1p128 ? ac <= ax && ax - ac < ax * 0x1p-20
+                                       : isinf(ac);
+    if (!coarse || signbit(d2f_coarse(x)) != signbit(x)) atomicAdd(bad, 1ull);
     if (c != e && !isnan(f)) atomicAdd(bad + 1, 1ull);
     // rcp_nr on positive values across the normal FP32 range: within 2 ulp of
     // the correctly rounded reciprocal
