@@ -595,13 +595,14 @@ void free_all(DemHandle* h) {
 // and its expected ~3 contacts per particle at least eight.  Force blocks have
 // at most 64 threads: the FP64 force pass of a 103,823-sphere body takes
 // 82 us in blocks of 256, 70 us in blocks of 64, because the hardware spreads
-// small blocks more evenly over the SMs (the FP32 pass does not change).  An
-// arena's integrator, whose scenes differ in work per particle, takes blocks
-// of 128 (256 scenes: 151 -> 143 us).  Both kinds of handles default to the
-// FP32 force kernel with the register budget for four 256-thread blocks per
-// SM (64 registers, a few bytes of spills): with the compiler's choice (three
-// blocks) the 2,000,000-sphere bed's force pass measured 180 us instead of
-// 156 us, the 256 scenes' 186 us instead of 174 us.
+// small blocks more evenly over the SMs (the FP32 pass does not change).
+// Integrator blocks too: 2,000,000 spheres in a bed take 159 us in blocks of
+// 256, 155 us in 128, 153 us in 64; 256 scenes 151, 141 and 139 us.  The FP32
+// force kernel of a single scene has the register budget for four 256-thread
+// blocks per SM (64 registers): the 2,000,000-sphere bed's force pass takes
+// 109 us with it, 121 us with three blocks' (80 registers).  An arena, whose
+// scenes are mostly bonded bodies, takes the latter: 256 scenes 157 us, 165 us
+// with four; a single cracked body of 800,000 would take 271 us, 294 us.
 LaunchShape default_shape(const DemHandle* h) {
     auto block_for = [&](int64_t units, int per_sm) {
         int b = 256;
@@ -609,9 +610,9 @@ LaunchShape default_shape(const DemHandle* h) {
         return b;
     };
     const int64_t n = h->multi ? INT64_MAX / 16 : h->n_cap;
-    const int ib = h->multi ? 128 : block_for(n, 4), fb = std::min(block_for(3 * n, 8), 64);
+    const int ib = std::min(block_for(n, 4), 64), fb = std::min(block_for(3 * n, 8), 64);
     const int cb = block_for(4 * n, 4);
-    return LaunchShape{fb, h->sm_count * 32, cb, h->sm_count * 16, ib, 4, 4, 0, 0, 0};
+    return LaunchShape{fb, h->sm_count * 32, cb, h->sm_count * 16, ib, 4, h->multi ? 0 : 4, 0, 0, 0};
 }
 
 int init_handle(DemHandle* h) {

@@ -109,19 +109,23 @@ __device__ __forceinline__ bool surely_touching32(float4 a, float ra, float4 b, 
 // unconditionally (on the FP64 pipe) and select.
 static __device__ __noinline__ float d2f_hw(double x) { return __double2float_rn(x); }
 static __device__ __noinline__ double f2d_hw(float f) { return (double)f; }
+__device__ __forceinline__ bool d2f_normal(unsigned h) {  // h: high word without its sign
+    return h - 0x38100000u < 0x0fe00000u;                 // 2^-126 <= |x| < 2^128
+}
+__device__ __forceinline__ float d2f_bits(unsigned hi, unsigned lo) {
+    // exponent rebiased (modulo 2^32) and the top 23 significand bits; the 29
+    // bits rounded off stand at the top of lo << 3
+    unsigned r = __funnelshift_l(lo, hi & 0x7fffffffu, 3) - ((1023u - 127u) << 23);
+    if (((lo << 3) | (r & 1u)) > 0x80000000u) ++r;  // above half, or half and odd
+    return __uint_as_float(r | (hi & 0x80000000u));
+}
 __device__ __forceinline__ float d2f(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-    const int e = (int)((hi >> 20) & 0x7ffu) - (1023 - 127);  // binary32 exponent field
-    if ((unsigned)(e - 1) >= 254u) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    if (!d2f_normal(hi & 0x7fffffffu)) {
         if (((hi << 1) | lo) == 0u) return __uint_as_float(hi);  // ±0
         return d2f_hw(x);
     }
-    const unsigned sig = ((hi & 0xfffffu) << 3) | (lo >> 29);  // top 23 significand bits
-    const unsigned rest = lo & 0x1fffffffu;                    // the 29 bits rounded off
-    unsigned r = (hi & 0x80000000u) | ((unsigned)e << 23) | sig;
-    r += (rest > 0x10000000u || (rest == 0x10000000u && (sig & 1u))) ? 1u : 0u;
-    return __uint_as_float(r);
+    return d2f_bits(hi, lo);
 }
 __device__ __forceinline__ double f2d(float f) {
     const unsigned u = __float_as_uint(f);
@@ -195,6 +199,9 @@ __device__ __forceinline__ double twice_exact(double x) {
 // largest one).
 __device__ __forceinline__ bool not_negzero(double v) {
     return __double_as_longlong(v) != (long long)0x8000000000000000ull;
+}
+__device__ __forceinline__ bool finite_bits(double v) {
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
 }
 __device__ __forceinline__ bool finite_not_negzero(double v) {
     const long long b = __double_as_longlong(v);
