@@ -98,6 +98,11 @@ INTEGRATE_BYTES_PER_CONTACT = 80
 # the identity orientation, so the integrator writes neither its spin (24 B)
 # nor its quaternion (32 B)
 INTEGRATE_BYTES_SETTLING = INTEGRATE_BYTES_PER_PARTICLE - 3 * 8 - 4 * 8
+# and what such a step's integrator still moves: it reads position, velocity,
+# r, m, 1/m, 1/I, two FP32 positions, row bounds and count (124 B), and writes
+# the position and velocity component along gravity, the FP32 position and the
+# force and moment totals (80 B)
+INTEGRATE_BYTES_FREE = 124 + 80
 # k_search on a neighbour-list step, per particle: path byte, current row
 # bounds, list length, FP32 position, next row bounds written, four list
 # partner indices (53 B; the partners' FP32 positions are re-reads); per
@@ -117,27 +122,35 @@ def algorithmic_bytes(n: int, contacts: int, bonds: int, settling: bool = False)
             "contacts": n * DETECT_BYTES_PER_PARTICLE + contacts * ROW_BYTES_PER_CONTACT}
 
 
-# k_search (contact update: full search or lists, next rows), k_force, k_integrate
-KERNELS_PER_STEP = 3
+def kernels_per_step(n: int, arena: bool = False) -> int:
+    """The library's launches per timed step at the default launch shape: one
+    cooperative step kernel for a single scene of up to 256 particles per SM;
+    else k_search, k_force and k_integrate, with k_list1 before them for a
+    single scene of more than 512 particles per SM."""
+    if arena:
+        return 3
+    return 1 if n <= 256 * SM_COUNT else 3 if n <= 512 * SM_COUNT else 4
+
+
 # FP64-pipe instructions per unit, from ncu (sm__thread_inst_executed_pipe_fp64_pred_on.sum
 # of one launch over the units it processed).  Force kernel, FP64 mode: per
-# Hertz contact 151.0 (a 100,000-sphere compacted bed, every contact a Hertz
-# contact: 1.503e7 per launch), per bond 116.1 (the 17,576-sphere cube in its
-# fragmentation, 41,427 bonds and 6,670 Hertz contacts: 5.818e6 per launch,
-# less the Hertz share); FP32 mode per bond 15.0 (the same cube before its
-# impact).  Integrator per particle: 92.0 in FP64 mode (the cube in its
-# fragmentation, split over four warps per 32 particles: 1.616e6 per launch;
-# the one-thread form measured 84.1), 51.0 in the FP32 mode (64 scenes of the
-# batched workload).  Then GB300's FP64 pipe width.
-FP64_INST = {("force", "fp64", "bond"): 116.1, ("force", "fp64", "hertz"): 151.0,
-             ("force", "fp32", "bond"): 15.0,
-             ("integrate", "fp64"): 92.0, ("integrate", "fp32"): 51.0}
-# The integrator skips the quaternion increment of a particle with exactly zero
-# spin, the normalisation of a spinless identity orientation and the spin
-# update of a particle with exactly zero torque: in the pour's settling phase
-# (no contacts) that is every particle (ncu on a 400,000-sphere pour:
-# 7,200,000 FP64 thread instructions per launch)
-FP64_INST_WORKLOAD = {("c3", "integrate", "fp32"): 18.0}
+# Hertz contact 130.0 (a 103,823-sphere bed, every contact a Hertz contact:
+# 1.334e7 per launch), per bond 104.0 (a cracked lattice of 17,576, 40,535 bonds
+# and 5,101 Hertz contacts: 4.879e6 per launch, less the Hertz share); FP32
+# mode per bond 15.0 (64 batched scenes, 652,624 bonds: 9.789e6), per Hertz
+# contact 13.0 (the bed: 1.334e6).  Integrator per particle: 95.1 in FP64 mode
+# (the cracked lattice, split over four warps per 32 particles, with the
+# quaternions: 1.672e6 per launch), 32.1 in the FP32 mode (the 64 scenes, with
+# the quaternions: 1.188e7).  Then GB300's FP64 pipe width.
+FP64_INST = {("force", "fp64", "bond"): 104.0, ("force", "fp64", "hertz"): 130.0,
+             ("force", "fp32", "bond"): 15.0, ("force", "fp32", "hertz"): 13.0,
+             ("integrate", "fp64"): 95.1, ("integrate", "fp32"): 32.1}
+# The integrator leaves out the components without a force, the spin update of
+# a particle with exactly zero torque and the orientation of one that does not
+# spin: in the pour's settling phase (no contacts) that is every particle (ncu
+# on a 400,000-sphere pour: 3,200,000 FP64 thread instructions per launch)
+# (the bed's orientations are k_list1's: 2.394e6 for 103,823 spheres)
+FP64_INST_WORKLOAD = {("c3", "integrate", "fp32"): 8.0, ("c3bed", "integrate", "fp32"): 23.1}
 FP64_LANES_PER_SM = 2
 SM_COUNT = 152
 
@@ -181,22 +194,21 @@ L2_FLUSH_BYTES = 256 << 20
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
 # of each dominant kernel, from one ncu capture each, with the particles that
-# launch processed.  The batched captures ran on the first 64 scenes of the
-# batch (431,416 spheres); their traffic is scaled to a launch by particles
-# processed.  Keys: workload and timed window ("c2" the cube in its impact
-# window, "c3" the pour settling, "c3bed" the compacted bed), kernel.
+# launch processed.  The batched captures ran on 64 scenes (369,893 spheres);
+# their traffic is scaled to a launch by particles processed.  Keys: workload
+# and timed window ("c2" a cracked lattice of the cube's size, "c3" the pour
+# settling, "c3bed" the compacted bed), kernel.
 NCU_TRAFFIC = {
-    ("c2", "force"): (7.470848e6, 17576),          # k_force<double>, step 4,006
-    ("c2", "contacts"): (2.336768e6, 17576),       # k_search, list step, step 4,006
-    ("c2", "integrate"): (9.095680e6, 17576),      # k_integrate_split, step 4,006
-    ("c3bed", "force"): (94.237e6, 400000),        # k_force4<float>, 400,000-sphere bed
-    ("c3bed", "contacts"): (51.041e6, 400000),     # k_search, list step (one lane per particle)
-    ("c3bed", "integrate"): (181.203e6, 400000),   # k_integrate3 (FP32 gather)
-    ("c3", "integrate"): (628.523e6, 2000000),     # k_integrate3 (FP32 mode, no contacts)
-    ("c3", "contacts"): (43.036e6, 2000000),       # k_search, list step (wide pass)
-    ("c4", "force"): (186.237e6, 431416),          # k_force<float, 1>
-    ("c4", "integrate"): (176.134e6, 431416),      # k_integrate3<1> (FP32 gather)
-    ("c4", "contacts"): (35.621e6, 431416),        # k_search<0, 1>, list step
+    ("c2", "force"): (8.206e6, 17576),             # k_force<double>
+    ("c2", "contacts"): (1.570e6, 17576),          # k_search, list step
+    ("c2", "integrate"): (7.064e6, 17576),         # k_integrate_split
+    ("c3bed", "force"): (392.9e6, 2000000),        # k_force4<float>, inside a call
+    ("c3bed", "contacts"): (404.9e6, 2000000),     # k_list1, with the quaternions
+    ("c3bed", "integrate"): (528.6e6, 2000000),    # k_integrate3, inside a call
+    ("c3", "integrate"): (365.5e6, 2000000),       # k_integrate3 (no contacts)
+    ("c4", "force"): (147.5e6, 369893),            # k_force<float, 1>
+    ("c4", "integrate"): (99.5e6, 369893),         # k_integrate3<1>
+    ("c4", "contacts"): (20.3e6, 369893),          # k_search<0, 1>, list step
 }
 
 
@@ -492,7 +504,7 @@ def main_batched(args, lib, ws, rank, dist=None) -> None:
                        "l2": "inputs larger than L2 (no flush)",
                        "parallelism": f"replicas x{ws}" if ws > 1 else "one arena"},
             "roofline": r["roofline"], "cpu_baseline": cpu, "e2e": e2e, "clocks": r["clocks"],
-            "gpu_launches": KERNELS_PER_STEP * r["steps"],
+            "gpu_launches": kernels_per_step(0, arena=True) * r["steps"],
         }
         print(json.dumps(line), flush=True)
 
@@ -547,7 +559,7 @@ def main_served(args, lib, ws, rank, dist=None) -> None:
                     "d2h_bytes_per_step": 0,
                     "note": "the served loop is end to end: uploads at admission, device-side "
                             "completion, host bookkeeping; results are step counts and stats"},
-            "clocks": clk, "gpu_launches": KERNELS_PER_STEP * rep.launches,
+            "clocks": clk, "gpu_launches": kernels_per_step(0, arena=True) * rep.launches,
         }
         print(json.dumps(line), flush=True)
 
@@ -797,6 +809,8 @@ def measure_scene(args, lib, sc, precision: str, steps: int, warmup: int, advanc
     ph = {k: float(np.mean([q[k] for q in phases])) for k in phases[0]}
     c_mean, b_mean = window["contacts_mean"], window["bonds_mean"]
     alg = algorithmic_bytes(sc.n, int(round(c_mean)), int(round(b_mean)), settling)
+    if settling and not c_mean:
+        alg["integrate"] = sc.n * INTEGRATE_BYTES_FREE
     dom = max(ph, key=ph.get)
     peaks = load_peaks()
     roof = {"bound": "hbm", "kernel": dom, "unit": "GB/s", "peak": peaks["hbm_gbs"],
@@ -1053,7 +1067,7 @@ def main() -> None:
                        "l2": "flushed between timed steps (256 MiB write)",
                        "parallelism": f"replicas x{ws}" if ws > 1 else "single scene"},
             "roofline": r["roofline"], "cpu_baseline": cpu, "e2e": r.get("e2e"),
-            "clocks": r["clocks"], "gpu_launches": KERNELS_PER_STEP * args.steps,
+            "clocks": r["clocks"], "gpu_launches": kernels_per_step(sc.n) * args.steps,
         }
         if proxy:
             line["reference_gpu_proxy"] = proxy
