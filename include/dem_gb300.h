@@ -298,9 +298,13 @@ int dem_sync(DemHandle* h);
 int dem_set_precision(DemHandle* h, int mode);
 
 /* Launch shape of the grid-stride kernels (contact forces, integration):
- * block sizes (multiples of 32, at most 256) and grid upper bounds.  Results
- * are the same for every shape; the shape only changes speed (the
- * autotuner's knob).  No counterpart in the reference. */
+ * block sizes (multiples of 32, at most 256) and grid upper bounds (the force
+ * grid is at most the blocks resident at once).  Results are the same for
+ * every shape; the shape only changes speed (the autotuner's knob).  With
+ * list_lanes, integrate_lanes and dependent_launch all 0 a single scene of up
+ * to 256 particles per SM runs whole steps in one cooperative kernel, which
+ * the block and grid sizes do not concern; any of them set selects the
+ * separate kernels.  No counterpart in the reference. */
 typedef struct DemLaunchShape {
     int32_t force_block;
     int32_t force_grid;
@@ -366,14 +370,12 @@ int dem_set_particles_async(DemHandle* h, const DemParticleState* in);
  * dem_set_particles_async(in) (skipped for NULL), dem_step(nsteps), then
  * dem_get_particles(out) (skipped for NULL; returns when `out` holds the
  * state).  Single-scene handles.  With `in` and `out` in page-locked host (or
- * device) memory and the integrator split over four warps per 32 particles
- * (scenes of up to 256 particles per SM), the host-link traffic overlaps the
- * step: the positions are uploaded first, the other fields beside the
- * contact update (a one-step call replays one captured graph per set of
- * buffers; in a call of several steps the velocities and spins go with the
- * positions and the first step's integrator reads the orientations and the
- * first wall's shear history from `in`), and the last step's integrator
- * writes the state into `out` block by block as it finishes
+ * device) memory, a scene that runs whole steps in one cooperative kernel (up
+ * to 256 particles per SM, default launch shape) exchanges inside it: the
+ * positions are read first, velocities and spins beside the contact update,
+ * orientations and the walls' shear beside the forces, the last step's
+ * integrator writes the state into `out` block by block as it finishes, and
+ * the last block writes a word that the host waits for
  * (DemStats.exchanges_direct counts these calls).  `in` and `out` may be the
  * same buffers; a one-step exchange in place then leaves out the values the
  * step did not change (bit for bit), which the buffers hold already.
