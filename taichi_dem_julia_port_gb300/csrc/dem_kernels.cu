@@ -2794,12 +2794,32 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     // the end-of-step rebuild-flag work of every scene (see scene_flags_one):
     // it only ORs into the next flags, as the particles' skin test does
     for (int s = i; s < p.ns; s += gridDim.x * blockDim.x) scene_flags_one<MULTI>(d, p, cur, s);
-    if (i >= p.n) return;
-    const int sc = slot_scene<MULTI>(d, i);
-    if (MULTI && (sc < 0 || d.sp[sc].mode != kModeStep)) {
-        d.in_cnt[i] = 0;
-        return;
+    // the lanes that take part in the votes below, which decide stored bits: not
+    // __activemask(), which after the wall, position and quaternion code need
+    // not name all of them (two groups of lanes writing one word of bits would
+    // each undo the other's).  In an arena they are taken from the whole warp
+    // here; a single scene's are the slots below p.n, and are worked out where
+    // they are used (held in a register from here they cost the integrator of a
+    // pour of 2,000,000 four per cent).
+    int sc = 0;
+    unsigned stepping = 0u;
+    if constexpr (MULTI) {
+        const bool exists = i < p.n;
+        sc = exists ? slot_scene<MULTI>(d, i) : -1;
+        const bool live = sc >= 0 && d.sp[sc].mode == kModeStep;
+        stepping = __ballot_sync(0xffffffffu, live);
+        if (!live) {
+            if (exists) d.in_cnt[i] = 0;
+            return;
+        }
+    } else {
+        if (i >= p.n) return;
     }
+    auto lanes = [&]() {
+        if constexpr (MULTI) return stepping;
+        const int left = p.n - (i & ~31);
+        return left >= 32 ? 0xffffffffu : (1u << left) - 1u;
+    };
     const SceneParams& S = scene_rec<MULTI>(d, p, sc);
     // every load of the particle's own state is issued before the gather's
     // dependent loads (nothing here is stored before the gather completes)
@@ -2897,7 +2917,7 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
         // 82 us, 103 us without it.  Otherwise the three run as one straight
         // line: a branch per component makes them a chain (a bed of 2,000,000:
         // 160 us, straight 158 us, without the choice 153 us).
-        const unsigned am = __activemask();
+        const unsigned am = lanes();
         const bool fin = finite_bits(invm) && finite_bits(S.hdt2) && finite_bits(dt);
         const bool u0 = __all_sync(am, fin && __double_as_longlong(F[0]) == 0ll);
         const bool u1 = __all_sync(am, fin && __double_as_longlong(F[1]) == 0ll);
@@ -2949,10 +2969,9 @@ __device__ __forceinline__ void integrate_body(const DemDev& d, const DemParams&
     {
         // the quaternion bits of the warp's slots: cleared where nothing was
         // updated (QUAT), set where a spin will turn the particle
-        const unsigned am = __activemask();
-        const unsigned on = __ballot_sync(am, spin), looked = __ballot_sync(am, QUAT);
-        const unsigned held = __ballot_sync(am, touched);
-        const uint32_t next = (qword & ~looked) | on, hold = (sword & ~am) | held;
+        const unsigned am = lanes();
+        const unsigned on = __ballot_sync(am, spin), held = __ballot_sync(am, touched);
+        const uint32_t next = (QUAT ? qword & ~am : qword) | on, hold = (sword & ~am) | held;
         if (lane_id() == (unsigned)(__ffs(am) - 1)) {
             if (next != qword) d.qmask[i >> 5] = next;
             if (hold != sword) d.smask[i >> 5] = hold;
@@ -3379,11 +3398,11 @@ __device__ __forceinline__ void integrate_split(const DemDev& d, const DemParams
         }
     }
     meet();  // the new position components (and the output rows) in shared memory
+    const unsigned am = __ballot_sync(0xffffffffu, live);
     if (q == 3 && live) {
         const float fx = sh.pos[0][l], fy = sh.pos[1][l], fz = sh.pos[2][l];
         d.pos32[i] = make_float4(fx, fy, fz, reach32(fx, fy, fz, d.rm32[i].z));
         const bool moved = S.f_half_skin > 0.0f && left_skin(S, fx, fy, fz, d.xref[i]);
-        const unsigned am = __activemask();
         const unsigned peers = __match_any_sync(am, moved ? sc : -1);
         if (moved && lane_id() == (unsigned)(__ffs(peers) - 1) && d.sflags[nxt][sc] == 0u)
             atomicOr(&d.sflags[nxt][sc], 1u);

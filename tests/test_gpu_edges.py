@@ -205,6 +205,22 @@ def test_touched_bits_follow_the_layout(gpu):
         _same(run(shapes), want, f"{shapes}")
 
 
+@pytest.mark.parametrize("n", [31, 33, 320])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_lanes_of_a_warp_that_differ(gpu, n, precision):
+    """Warps whose lanes spin or not, touch the plane or not, have partners or
+    none and turn at different steps: each lane's bit survives the others'."""
+    cfg, p, omega = _columns(n, seed=5)
+    k = np.arange(n)
+    omega[k % 3 != 0] = 0.0
+    p.pos[k % 7 == 0, 2] += 0.5e-3  # off the plane and off their neighbours
+    one, four = (_run(cfg, p, omega, [1, 4, 25], dict(list_lanes=m, integrate_lanes=m), precision)
+                 for m in (1, 4))
+    still = np.all(four[0]["quat"] == [1.0, 0.0, 0.0, 0.0], axis=1)
+    assert 0 < still.sum() < n and np.any(four[0]["wall_shear"] != 0.0)
+    _same(one, four, f"n={n} {precision}")
+
+
 @pytest.mark.parametrize("small", [3, 4, 5, 20, 40])
 def test_rows_longer_than_a_group(gpu, small):
     """A sphere in contact with more partners than a particle has lanes, and
