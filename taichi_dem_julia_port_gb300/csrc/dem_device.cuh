@@ -81,6 +81,12 @@ __device__ __forceinline__ bool maybe_touching32(float4 a, float4 b, float extra
     return !(s * (1.0f - 0x1p-17f) > B * B);
 }
 
+// A NaN among the coordinates of an FP32 position (an infinite one, which a
+// finite FP64 coordinate may round to, is no NaN; the reach .w may hide one).
+__device__ __forceinline__ bool no_place(float4 a) {
+    return isnan(a.x) || isnan(a.y) || isnan(a.z);
+}
+
 // Conservative FP32 acceptance, the mirror of maybe_touching32: returns true
 // only when the FP64 test touching_rn is certain to succeed.  a, b are the
 // particles' FP32 positions (as for maybe_touching32), ra, rb their FP32

@@ -697,8 +697,14 @@ __device__ __forceinline__ void detect_group(const DemDev& d, const DemParams& p
                 ++en;
                 eh += enum_mix(i, j);
             }
-            // partners within rᵢ + rⱼ + skin join the neighbour list
-            const bool near = maybe_touching32(P32, qq[u], skin);
+            // partners within rᵢ + rⱼ + skin join the neighbour list.  NaN
+            // coordinates are near nothing: every distance to them is NaN,
+            // which the FP32 test cannot reject, all such spheres share one
+            // bucket, and as each other's partners they would overflow their
+            // lists and so ask for a full search in every step (a pour of
+            // 200,000 with 40 landed spheres: 129 us per step, 20 us without)
+            const bool near =
+                maybe_touching32(P32, qq[u], skin) && !no_place(P32) && !no_place(qq[u]);
             if (build && near) {
                 const int vs = atomicAdd(&sh.nvl, 1);
                 if (vs < p.kvl) vl[(size_t)vs * p.wstride] = j;

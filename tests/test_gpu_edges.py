@@ -280,3 +280,32 @@ def test_not_a_number_asks_for_no_search(gpu, n):
     _same(lists, full, f"n={n}")
     assert full[2]["full_searches"] == steps
     assert lists[2]["full_searches"] < steps // 4
+
+
+@pytest.mark.parametrize("n", [2000, 40_000, 80_000])
+def test_many_not_a_numbers_share_no_list(gpu, n):
+    """More spheres with NaN coordinates than a neighbour list holds: a full
+    search that finds them together in one bucket puts none on another's list,
+    so the others go on as with a search in every step, and search as often as
+    they do beside 40 spheres that have not landed."""
+    nan, k = np.arange(9, 409, 10), np.arange(40)
+
+    def run(gap, skin):
+        cfg, p, omega = _columns(n, seed=8)
+        r = np.cbrt(0.75 * p.volume[nan] / np.pi)
+        p.pos[nan] = np.stack([-0.045 + 5e-3 * (k % 8), -0.045 + 5e-3 * (k // 8), r + gap], axis=1)
+        p.vel[nan] = [0.0, 0.0, -0.01]
+        omega[nan] = 0.0
+        with GlobalData(cfg, p) as g:
+            g.set_skin_factor(skin)
+            g.set_particles(omega=omega)
+            g.simulate(200)
+            assert np.isnan(g.particles()["pos"][nan]).any(axis=1).all() == (gap < 1e-6)
+            g.set_skin_factor(skin)  # the lists are built again
+            before = g.stats()["full_searches"]
+            g.simulate(60)
+            return _result(g), g.stats()["full_searches"] - before
+
+    (full, every), (lists, few), (_, beside) = run(1e-9, 0.0), run(1e-9, 0.9), run(1e-3, 0.9)
+    _same(lists, full, f"n={n}")
+    assert every == 60 and few == beside < 60
