@@ -304,7 +304,8 @@ int dem_set_precision(DemHandle* h, int mode);
  * list_lanes, integrate_lanes and dependent_launch all 0 a single scene of up
  * to 256 particles per SM runs whole steps in one cooperative kernel, which
  * the block and grid sizes do not concern; any of them set selects the
- * separate kernels.  No counterpart in the reference. */
+ * separate kernels (dem_step_exchange takes the cooperative one all the same,
+ * see there).  No counterpart in the reference. */
 typedef struct DemLaunchShape {
     int32_t force_block;
     int32_t force_grid;
@@ -369,14 +370,17 @@ int dem_set_particles_async(DemHandle* h, const DemParticleState* in);
 /* One call of a host loop that exchanges the state every step:
  * dem_set_particles_async(in) (skipped for NULL), dem_step(nsteps), then
  * dem_get_particles(out) (skipped for NULL; returns when `out` holds the
- * state).  Single-scene handles.  With `in` and `out` in page-locked host (or
- * device) memory, a scene that runs whole steps in one cooperative kernel (up
- * to 256 particles per SM, default launch shape) exchanges inside it: the
- * positions are read first, velocities and spins beside the contact update,
- * orientations and the walls' shear beside the forces, the last step's
- * integrator writes the state into `out` block by block as it finishes, and
- * the last block writes a word that the host waits for
- * (DemStats.exchanges_direct counts these calls).  `in` and `out` may be the
+ * state).  Single-scene handles.  With `out` in page-locked host (or device)
+ * memory and `in` given with its positions, the steps of a scene of up to 256
+ * particles per SM run in one cooperative kernel that also exchanges the state
+ * (for every launch shape but integrate_lanes = 1; with integrate_lanes = 4
+ * above that size too, calls of one or two steps): the positions are read
+ * first, velocities and spins beside the contact update, orientations and the
+ * walls' shear beside the forces, the last step's integrator writes the state
+ * into `out` block by block as it finishes, and the last block writes a word
+ * that the host waits for (DemStats.exchanges_direct counts these calls).  If
+ * any field of `in` is pageable, `in` is uploaded before that kernel.  `in` and
+ * `out` may be the
  * same buffers; a one-step exchange in place then leaves out the values the
  * step did not change (bit for bit), which the buffers hold already.
  * Replaces `simulate!` (src/executor.jl:162-172) with the host copy of the

@@ -878,6 +878,20 @@ bool steps_fit(const DemHandle* h) {
     return h->steps_ok && h->p.n <= kStepsPerSm * h->sm_count && h->shape.list_lanes == 0 &&
            h->shape.integrate_lanes == 0 && h->shape.dependent_launch == 0;
 }
+// k_steps's own buffers, and whether its launch fits the device.  Handles of
+// scenes that run their steps in it have them from the start, others once an
+// exchange first needs them.
+int alloc_steps(DemHandle* h) {
+    TRY(dalloc(h, &h->d.wtouch, (size_t)h->p.n));
+    return dalloc(h, &h->d.wforce, 6 * (size_t)h->nwall * (size_t)h->p.wstride);
+}
+bool steps_buffers(DemHandle* h) {
+    if (!h->steps_ok && !h->d.wtouch) {
+        h->steps_ok = steps_ready(h->p) && alloc_steps(h) == DEM_OK;
+        if (!h->steps_ok) cudaGetLastError();  // the exchange goes the usual way
+    }
+    return h->steps_ok;
+}
 // nsteps steps by k_steps, at most kStepsPerLaunch in each launch (other
 // streams' work gets its turn between launches); the first reads io's input,
 // the last writes its output.
@@ -1411,8 +1425,7 @@ int create_single(const DemConfigC* cfg, const DemParticlesIn* pin, const DemTab
     if (rc == DEM_OK && h->tab) rc = upload_tables(h, M, mid);
     if (rc == DEM_OK && pin->n > 0 && pin->n <= kStepsPerSm * sms) {
         h->steps_ok = steps_ready(h->p);
-        rc = dalloc(h, &h->d.wtouch, (size_t)pin->n);
-        if (rc == DEM_OK) rc = dalloc(h, &h->d.wforce, 6 * (size_t)h->nwall * (size_t)pin->n);
+        rc = alloc_steps(h);
     }
     if (rc == DEM_OK) rc = flag_search(h, 0);
     if (rc == DEM_OK) {
@@ -1851,18 +1864,31 @@ int dem_set_particles_async(DemHandle* h, const DemParticleState* in) {
 }
 
 // The exchange of dem_step_exchange inside the steps' launch: the device
-// addresses of the caller's records (every given field must be
-// device-accessible: page-locked host or device memory, and the positions
-// must be given) and of the page-locked error word.
+// addresses of the caller's records (the positions must be given and every
+// output field be device-accessible: page-locked host or device memory) and of
+// the page-locked error word.  Input that is not device-accessible is uploaded
+// before the launch, which then only writes.
+//
+// All launch shapes whose integrator is the split one go this way: a shape
+// chooses among kernels with the same results, and k_steps is the one that can
+// exchange.  One step as upload, kernels and read-back against this, 17,576
+// spheres: 82 and 57 us with integrate_lanes, list_lanes or dependent_launch
+// set, 133 and 119 us with pageable input.  Above the scenes that run their
+// steps in k_steps anyway (integrate_lanes = 4) its steps are slower than the
+// separate kernels', and a call takes it for the exchange's sake while it has
+// few of them: 512,000 spheres, one step 1,306 and 1,052 us, two 1,808 and
+// 1,734, three 2,307 and 2,335; 103,823 one 316 and 243, two 428 and 380, five
+// 772 and 767.
+constexpr int64_t kLargeExchange = 2;
 constexpr int kNoHostOut = INT_MIN;  // the error word's sentinel: not written
 static bool direct_exchange(DemHandle* h, const DemParticleState* in, int64_t nsteps,
                             const DemParticleState* out, StepIO* io) {
-    if (!in || !in->pos || !out || nsteps <= 0 || !steps_fit(h)) return false;
-    const double* const fi[5] = {in->pos, in->vel, in->omega, in->quat, in->wall_shear};
+    if (!in || !in->pos || !out || nsteps <= 0 || h->p.n == 0 ||
+        !split_integrator(h->shape, h->p.n, h->p.sms) ||
+        (h->p.n > kStepsPerSm * h->sm_count && nsteps > kLargeExchange) || !steps_buffers(h))
+        return false;
     double* const fo[kHostOutFields] = {out->pos,   out->vel,    out->omega,     out->quat,
                                         out->force, out->moment, out->wall_shear};
-    for (int q = 0; q < 5; ++q)
-        if (fi[q] && !(io->in[q] = device_view(fi[q]))) return false;
     for (int q = 0; q < kHostOutFields; ++q)
         if (fo[q] && !(io->out.rec[q] = device_view(fo[q]))) return false;
     if (!h->err_host) {
@@ -1875,6 +1901,15 @@ static bool direct_exchange(DemHandle* h, const DemParticleState* in, int64_t ns
     }
     if (!h->err_dev) return false;
     io->out.err = h->err_dev;
+    io->has_out = 1;
+    const double* const fi[5] = {in->pos, in->vel, in->omega, in->quat, in->wall_shear};
+    for (int q = 0; q < 5; ++q) {
+        if (fi[q] && !(io->in[q] = device_view(fi[q]))) {
+            for (const double*& f : io->in) f = nullptr;
+            return true;
+        }
+    }
+    io->has_in = 1;
     // a one-step exchange in place: values the step leaves unchanged are in
     // `out` already (the step's input of that field came from there)
     const double* const same[kHostOutFields] = {io->in[0], io->in[1], io->in[2], io->in[3],
@@ -1882,7 +1917,6 @@ static bool direct_exchange(DemHandle* h, const DemParticleState* in, int64_t ns
     if (nsteps == 1)
         for (int q = 0; q < kHostOutFields; ++q)
             if (same[q] && same[q] == io->out.rec[q]) io->out.same |= 1u << q;
-    io->has_in = io->has_out = 1;
     return true;
 }
 
@@ -1891,6 +1925,7 @@ int dem_step_exchange(DemHandle* h, const DemParticleState* in, int64_t nsteps,
     if (!h || nsteps < 0 || h->multi) return DEM_ERR_INVALID;
     StepIO io{};
     if (direct_exchange(h, in, nsteps, out, &io)) {
+        if (!io.has_in) TRY(set_particles(h, in, false));
         __atomic_store_n(h->err_host, kNoHostOut, __ATOMIC_RELEASE);
         TRY(ensure_encoding(h));
         TRY(run_steps(h, nsteps, io));
