@@ -49,7 +49,9 @@ constexpr int kListBlocksFew = 4, kListBlocks = 6;
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
-constexpr unsigned long long kSpinLimit = 1ull << 22;
+// polls of a device wait before it gives up: about 4 s (grid barrier 234 ns a
+// poll, the scan's look-back 256 ns), far above any wait for blocks that work
+constexpr unsigned long long kSpinLimit = 1ull << 24;
 constexpr double kPi = 3.141592653589793;  // Julia's π rounded to binary64
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }

@@ -19,3 +19,13 @@ def test_no_vote_rests_on_the_active_mask():
     the whole warp instead."""
     for f in sorted(CSRC.glob("*.cu*")):
         assert "__activemask" not in code(f.name), f.name
+
+
+def test_device_waits_last_as_long_as_ever():
+    """A wait for blocks that still work must not give up on them: 2^24 polls
+    (about 4 s) for the grid barrier and the scan's look-back."""
+    src = code("dem_kernels.cu")
+    limit = re.search(r"kSpinLimit = 1ull << (\d+);", src)
+    assert limit and int(limit.group(1)) >= 24
+    assert len(re.findall(r"spin_limit = kSpinLimit", src)) == 1  # the grid barrier's default
+    assert len(re.findall(r"d\.ctr, kSpinLimit\)", src)) == 2  # both scan sites
