@@ -1590,6 +1590,9 @@ __global__ void __launch_bounds__(kThreads, MINB)
         if (!narrow_list(p.n, p.sms, p.list_lanes)) list_phase<false>(d, p, cur, lsh, kThreads);
         return;
     }
+    // a barrier that gave up left some arrivals in its word: the next launch's
+    // would let blocks through before the others, so there is none
+    if (__ldcg(&d.ctr->error) & kErrTimeout) return;
     if (threadIdx.x == 0) fail = 0;  // the first barrier orders this before any read of it
     search_phases<INIT, MULTI>(d, p, cur, all, Team{kThreads, 0, &fail}, sh, lsh, red);
 }

@@ -29,3 +29,27 @@ def test_device_waits_last_as_long_as_ever():
     assert limit and int(limit.group(1)) >= 24
     assert len(re.findall(r"spin_limit = kSpinLimit", src)) == 1  # the grid barrier's default
     assert len(re.findall(r"d\.ctr, kSpinLimit\)", src)) == 2  # both scan sites
+
+
+def kernels(src):
+    """Name and body of every __global__ function."""
+    for m in re.finditer(r"__global__[^{;]*?\b(k_\w+)\s*\([^{;]*\)\s*\{", src):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(src[at], 0)
+            at += 1
+        yield m.group(1), src[m.end():at]
+
+
+def test_no_barrier_after_one_that_gave_up():
+    """A grid barrier that gave up leaves arrivals in its word, which would
+    release the next one early: kernels that meet at one first look for a
+    pending timeout and return."""
+    meet = r"grid_sync\(|search_phases<"
+    found = {}
+    for name, body in kernels(code("dem_kernels.cu")):
+        first = re.search(meet, body)
+        if first and name != "k_selftest_barrier":  # which has a counter of its own
+            found[name] = "kErrTimeout) return;" in body[:first.start()]
+    assert set(found) == {"k_search", "k_steps"}
+    assert all(found.values()), found
