@@ -305,7 +305,9 @@ int dem_set_precision(DemHandle* h, int mode);
  * to 256 particles per SM runs whole steps in one cooperative kernel, which
  * the block and grid sizes do not concern; any of them set selects the
  * separate kernels (dem_step_exchange takes the cooperative one all the same,
- * see there).  No counterpart in the reference. */
+ * see there).  From 64 particles per SM on that kernel fills the GPU: work on
+ * other streams waits for up to 16 steps, with the separate kernels for
+ * hardly any.  No counterpart in the reference. */
 typedef struct DemLaunchShape {
     int32_t force_block;
     int32_t force_grid;

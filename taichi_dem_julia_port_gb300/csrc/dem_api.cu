@@ -892,13 +892,12 @@ bool steps_buffers(DemHandle* h) {
     }
     return h->steps_ok;
 }
-// nsteps steps by k_steps, at most kStepsPerLaunch in each launch (other
-// streams' work gets its turn between launches); the first reads io's input,
-// the last writes its output.
-constexpr int64_t kStepsPerLaunch = 64;
+// nsteps steps by k_steps, steps_per_launch in each launch (other streams' work
+// gets its turn between launches); the first reads io's input, the last writes
+// its output.
 int run_steps(DemHandle* h, int64_t nsteps, const StepIO& io) {
     for (int64_t done = 0; done < nsteps;) {
-        const int k = (int)std::min<int64_t>(nsteps - done, kStepsPerLaunch);
+        const int k = (int)std::min<int64_t>(nsteps - done, steps_per_launch(h->p));
         StepIO part = io;
         part.has_in = done == 0 ? io.has_in : 0;
         part.has_out = done + k == nsteps ? io.has_out : 0;

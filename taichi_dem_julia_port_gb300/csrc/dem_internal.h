@@ -325,6 +325,8 @@ void launch_search(const DemDev& d, const DemParams& p, int cur, bool init, bool
 // points, Hertz forces and particle totals that a caller can read; steps_ready sets the kernels up on the current
 // device and says whether that launch fits it
 bool steps_ready(const DemParams& p);
+// the most steps that one such launch may take (its other streams' wait)
+int steps_per_launch(const DemParams& p);
 cudaError_t launch_steps(const DemDev& d, const DemParams& p, int cur, int nsteps, bool report,
                          const StepIO& io, cudaStream_t s);
 void launch_force(const DemDev& d, const DemParams& p, int nxt, bool multi, const LaunchShape& sh,

@@ -25,7 +25,7 @@
 //   k_integrate  per particle: contact force gather in a fixed order,
 //                resolve_wall!, apply_body_force!, update!
 // A single scene of up to 256 particles per SM runs whole steps, up to 64 per
-// launch, in one cooperative kernel (k_steps) with the same phases.  Otherwise
+// launch (16 where it fills the SMs), in one cooperative kernel (k_steps) with the same phases.  Otherwise
 // a CUDA graph per contact-buffer parity holds a step's launches: these three,
 // and k_list1 before them for a single scene of more than 512 particles per SM
 // (its list update with one lane per particle, and the quaternions); a
@@ -3518,7 +3518,8 @@ __global__ void __launch_bounds__(kSplitThreads)
 //
 // Block size: 128 threads (one warp per sub-partition) while four lanes per
 // particle need no more warps than that, then 256, then 512 with one block
-// per SM; a small scene so leaves SMs (and registers) to other streams.
+// per SM; a small scene so leaves SMs (and registers) to other streams, a large
+// one ends its launches sooner (steps_per_launch).
 //
 // IO (dem_step_exchange): the first step reads the particle state from the
 // caller's arrays, the positions by all warps (the contact update waits for
@@ -3860,6 +3861,17 @@ void steps_shape(int n, int sms, int* grid, int* threads) {
     *grid = *threads == 128 ? blocks_for(warps, 4) : sms;
 }
 }  // namespace
+
+// Blocks of 512 threads take every SM's registers until the launch ends, and
+// whatever else the GPU has to do waits for that.  Steps per launch, what
+// another stream's small kernel beside 17,576 spheres waits, and a step's time:
+// 64, 1.78 ms, 28.0 us; 16, 0.45 ms, 28.2; 8, 0.23 ms, 28.4; 1, 0.03 ms, 31.1
+// (as the separate kernels, 41.8 us).  Smaller blocks leave it room.
+int steps_per_launch(const DemParams& p) {
+    int grid, threads;
+    steps_shape(p.n, p.sms, &grid, &threads);
+    return threads == kStepThreads ? 16 : 64;
+}
 
 bool steps_ready(const DemParams& p) {
     int grid, threads;

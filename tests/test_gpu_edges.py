@@ -309,3 +309,47 @@ def test_many_not_a_numbers_share_no_list(gpu, n):
     (full, every), (lists, few), (_, beside) = run(1e-9, 0.0), run(1e-9, 0.9), run(1e-3, 0.9)
     _same(lists, full, f"n={n}")
     assert every == 60 and few == beside < 60
+
+
+@pytest.mark.parametrize("n", [2000, 17_576])
+def test_other_streams_get_their_turn(gpu, n):
+    """A small kernel on a caller's own stream does not wait for dozens of
+    steps of a scene that fills the GPU."""
+    torch = pytest.importorskip("torch")
+    import time
+    cfg, p, omega = _columns(n, seed=10)
+    x, s = torch.zeros(4096, device="cuda"), torch.cuda.Stream()
+    with GlobalData(cfg, p) as g:
+        step = g.simulate_timed(512) / 512 * 1e-3
+        waits = []
+        for _ in range(5):
+            g.simulate(1000)
+            for _ in range(4):
+                t = time.perf_counter()
+                with torch.cuda.stream(s):
+                    x.add_(1.0)
+                s.synchronize()
+                waits.append(time.perf_counter() - t)
+            g.sync()
+    # the 16 steps of the launch in flight, as much again for the host's calls
+    assert np.median(waits) < 32 * step + 1e-4, (np.median(waits), step)
+
+
+@pytest.mark.parametrize("n", [2000, 7000, 17_576])
+def test_two_handles_step_at_once(gpu, n):
+    """Two threads, each stepping its own scene: as each alone."""
+    import threading
+    made = [_columns(n, seed=s) for s in (11, 12)]
+    want = [_run(*m, [40, 40, 40]) for m in made]
+    got = [None, None]
+
+    def work(k):
+        got[k] = _run(*made[k], [40, 40, 40])
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(got, want):
+        _same(a, b, f"n={n}")
