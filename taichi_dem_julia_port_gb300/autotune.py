@@ -15,7 +15,8 @@ dependent launches) and the pair search's register budget; each
 candidate is timed over `steps` steps after one untimed step.  The run moves
 on while candidates are timed, so the choice is confirmed at the end: the
 chosen and the starting settings are timed alternately (`confirm_rounds`
-times each) and the faster is kept.
+times each) and the faster is kept.  A single scene whose steps share
+cooperative launches has none of these knobs and keeps its settings.
 """
 from __future__ import annotations
 
@@ -62,6 +63,12 @@ def autotune(target, sm_count: int = 152, steps: int = 10, cell_factors=CELL_FAC
     start_shape = target.launch_shape()
     best = _time(target, steps)
     trials.append(({"baseline": True}, best))
+    if not is_arena and getattr(target, "steps_in_one_launch", lambda sms: False)(sm_count):
+        # no candidate but the launch mode changes anything, and that one by
+        # leaving the steps' kernel for the separate ones (us per step in it and
+        # outside: 1,000 spheres 16.3 and 18.3, 17,576 28.0 and 30.3, 38,000
+        # 50.1 and 49.0)
+        return TuneResult(None, start_shape, best, trials)
     if is_arena:
         best_cf = 1.0
         for cf in cell_factors:

@@ -226,6 +226,14 @@ class GlobalData:
     def set_launch_shape(self, **shape) -> None:
         set_launch_shape(self.lib, self.h, shape)
 
+    def steps_in_one_launch(self, sm_count: int) -> bool:
+        """Whether a call's steps share cooperative launches (up to 256
+        particles per SM and no layout of the separate kernels chosen), which
+        the launch shape's block and grid sizes do not concern."""
+        shape = self.launch_shape()
+        return 0 < self.n <= 256 * sm_count and not any(
+            shape[k] for k in ("list_lanes", "integrate_lanes", "dependent_launch"))
+
     def set_skin_factor(self, skin_factor: float) -> None:
         """Neighbour-list skin as a fraction of the largest the search allows
         (0 = full pair search every step); results do not change."""

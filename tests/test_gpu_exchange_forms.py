@@ -129,3 +129,18 @@ def test_calls_longer_than_a_launch(gpu, steps):
         same(buf, want, f"{steps}")
         assert g.stats()["exchanges_direct"] == 1
         buf.close()
+
+
+def test_autotuned_scene_keeps_its_exchange(gpu):
+    """The autotuner leaves a scene whose steps share a launch as it is; a
+    forced layout or a larger scene does have knobs."""
+    from taichi_dem_julia_port_gb300.autotune import autotune
+    sc = scenes.bonded_cube(8, speed=30.0, steps=0, seed=2)
+    with GlobalData(sc.cfg, sc.particles) as g:
+        g.initialize()
+        before = g.launch_shape()
+        assert g.steps_in_one_launch(152) and not g.steps_in_one_launch(1)
+        r = autotune(g, steps=2)
+        assert r.shape == before == g.launch_shape() and r.ms_per_step > 0.0
+        g.set_launch_shape(dependent_launch=1)
+        assert not g.steps_in_one_launch(152)

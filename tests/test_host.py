@@ -222,6 +222,39 @@ def test_autotune_confirms_its_choice():
     assert chosen, "the descent timed candidates"
 
 
+class _OneLaunchHandle:
+    """A single scene whose steps share cooperative launches: any timing of a
+    candidate is noise (each call a little faster than the one before)."""
+
+    def __init__(self):
+        self.shapes, self.t = [], 1.0
+
+    def steps_in_one_launch(self, sm_count):
+        return True
+
+    def launch_shape(self):
+        return dict(force_block=64, dependent_launch=0)
+
+    def set_launch_shape(self, **shape):
+        self.shapes.append(shape)
+
+    def simulate(self, n):
+        pass
+
+    def simulate_timed(self, n):
+        self.t *= 0.999
+        return n * self.t
+
+
+def test_autotune_leaves_steps_in_one_launch_alone():
+    """None of the knobs reaches such a scene's kernel, and the launch mode
+    would take it out of it: nothing is tried and nothing changed."""
+    from taichi_dem_julia_port_gb300.autotune import autotune
+    h = _OneLaunchHandle()
+    r = autotune(h, steps=2)
+    assert h.shapes == [] and r.shape == h.launch_shape() and len(r.trials) == 1
+
+
 def test_corrupt_p4p_is_rejected_with_its_line(tmp_path):
     """Malformed p4p input raises ValueError naming the file and line, before
     anything reaches the library."""
