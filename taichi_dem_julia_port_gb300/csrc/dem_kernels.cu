@@ -86,7 +86,8 @@ struct Team {
 };
 
 // Grid barrier over the teams of all blocks of a cooperative launch (every
-// block is resident, so it cannot wait on one that has not started).  Block 0
+// block is resident, so it cannot wait on one that has not started).  The
+// arrivals are counted as CUDA's cooperative groups count theirs: block 0
 // arrives with 2^31 - (blocks - 1), the others with 1: each full round of
 // arrivals flips the word's top bit and leaves the others as they were, so
 // the word needs no reset and any grid size can use it next.  The wait is
@@ -1145,9 +1146,9 @@ __device__ __forceinline__ void emit_row1(const DemDev& d, const DemParams& p, i
     const int start = place_rows<1>(d, p, cur ^ 1, len, active ? r.nb : 0, &bstart);
     if (active) write_row1(d, p, cur, r, keepm, start, bstart, len, tl);
 }
-// The neighbour-list update with one lane per particle: in large scenes with
-// few contacts and list partners per particle (a compacted bed, a pour) four
-// lanes per particle leave most lanes idle and too few particles in flight
+// The neighbour-list update of an arena with one lane per particle: where there
+// are few contacts and list partners per particle (beds, pours) four lanes per
+// particle leave most lanes idle and too few particles in flight
 // to cover the chain of dependent loads; one lane per particle puts four
 // times as many particles in flight.  A warp's rows are placed together
 // (one atomic per warp).
@@ -1155,7 +1156,6 @@ __device__ __forceinline__ void emit_row1(const DemDev& d, const DemParams& p, i
 // block b is the grid's warp w·gridDim + b): a cooperative launch places
 // consecutive blocks on the same SM, so chunks by block would leave SMs idle
 // whenever the particles do not fill the grid.
-template <bool MULTI>
 __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemParams& p, int cur,
                                                   int nt, bool tl) {
     const int wslot = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
@@ -1163,7 +1163,7 @@ __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemPara
         const int i0 = (int)(t0 + 32LL * wslot);
         const int i = i0 + (int)lane_id();
         bool act = i < p.n, frz = false;
-        if (MULTI && act) {
+        if (act) {
             const uint8_t path = d.path[i];
             act = (path & 3) == 2;
             frz = (path >> 2) == kModeFrozen;
@@ -1179,7 +1179,7 @@ __device__ __forceinline__ void list_phase_narrow(const DemDev& d, const DemPara
                 d.row_len[cur ^ 1][i] = 0;
                 act = false;
             } else {
-                list_particle1<MULTI>(d, p, cur, i, e0, e1, nv, frz, job, keepm);
+                list_particle1<true>(d, p, cur, i, e0, e1, nv, frz, job, keepm);
             }
         }
         emit_row1(d, p, cur, act, job, keepm, tl);
@@ -1317,11 +1317,11 @@ __device__ __forceinline__ void list_phase(const DemDev& d, const DemParams& p, 
     // come from the bond initialisation), and the force pass of one type of
     // contacts reads no type-ordered list
     const bool tl = MULTI || __ldcg(&d.ctr->alloc[cur].bonds) != 0u;
-    // one lane per particle when chosen, or by default when the particles
-    // outnumber half the launch's threads
+    // an arena's: one lane per particle when chosen, or by default when the
+    // particles outnumber half the launch's threads (a single scene's: k_list1)
     if (MULTI && (p.list_lanes == 1 ||
                   (p.list_lanes == 0 && 2LL * p.n > (long long)gridDim.x * nt))) {
-        list_phase_narrow<MULTI>(d, p, cur, nt, tl);
+        list_phase_narrow(d, p, cur, nt, tl);
         return;
     }
     const int lane = threadIdx.x & (kVLanes - 1);
@@ -3256,7 +3256,7 @@ __device__ __forceinline__ int item_rank(int w, int nw, int chunks) {
 // rows staged by the integrator: position, velocity, spin, force, moment
 constexpr int kStageRows = 15;
 // Shared memory of one group of four warps.  FUSED (k_steps): with the staging
-// of the exchange's output, and without the walls' forces, which wall_items
+// of the exchange's output, and without the walls' forces, which particle_items
 // has left in memory.
 template <bool TAB, bool FUSED>
 struct SplitShared {
@@ -3270,7 +3270,7 @@ struct SplitShared {
 // The particles [32u, 32u + 32) by four warps: q is the calling warp's role
 // (0, 1, 2: component; 3: walls and quaternion), tq its thread's index among
 // the four warps, which meet at block barrier `bar`.  FUSED: the walls' forces
-// come from wall_items; H (may be null): this step also writes the new state
+// come from particle_items; H (may be null): this step also writes the new state
 // into the caller's records; `report`: the force and moment totals are stored
 // (a step whose totals nobody can read before the next one leaves them out).
 template <bool MULTI, bool F32, bool TAB, bool FUSED>
@@ -3939,9 +3939,9 @@ void launch_force(const DemDev& d, const DemParams& p, int nxt, bool multi, cons
 void launch_integrate(const DemDev& d, const DemParams& p, int cur, bool multi,
                       const LaunchShape& sh, cudaStream_t s) {
     if (p.n == 0) return;
-    // k_list1 has updated the quaternions (the split layout's four-lane list
-    // update of a forced shape has not)
-    const bool quat = multi || !narrow_list(p.n, p.sms, p.list_lanes);
+    // a single scene's quaternions: k_list1 has updated them (the split layout's
+    // four-lane list update of a forced shape has not)
+    const bool quat = !narrow_list(p.n, p.sms, p.list_lanes);
     const int block = clamp_block(sh.integrate_block);
     if (split_integrator(sh, p.n, p.sms)) {
         const int nb = blocks_for(p.n, 32);
@@ -3962,13 +3962,15 @@ void launch_integrate(const DemDev& d, const DemParams& p, int cur, bool multi,
                p, cur);
     else if (p.precision == 1)
         launch(p.dep != 0,
-               multi ? (quat ? k_integrate3<true, true> : k_integrate3<true, false>)
-                     : (quat ? k_integrate3<false, true> : k_integrate3<false, false>),
+               multi  ? k_integrate3<true, true>
+               : quat ? k_integrate3<false, true>
+                      : k_integrate3<false, false>,
                nb, block, s, d, p, cur);
     else
         launch(p.dep != 0,
-               multi ? (quat ? k_integrate<true, true> : k_integrate<true, false>)
-                     : (quat ? k_integrate<false, true> : k_integrate<false, false>),
+               multi  ? k_integrate<true, true>
+               : quat ? k_integrate<false, true>
+                      : k_integrate<false, false>,
                nb, block, s, d, p, cur);
 }
 

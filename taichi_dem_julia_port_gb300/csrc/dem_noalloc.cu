@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kBlock)
     const uint2 local = block_scan_bins(c, sh.warp_sums);    // first place in the chunk
     const uint2 global = block_scan_bins(tot, sh.warp_sums);  // first place of the digit
     // the chunk's first place of each digit joins the warps' running sums
-    // (at most kChunk - 1, so 16 bits hold it)
+    // (at most kChunk, of a digit after all of them, so 16 bits hold it)
 #pragma unroll
     for (int w = 0; w < kWarps; ++w)
         reinterpret_cast<uint32_t*>(sh.cnt[w])[threadIdx.x] += local.x | (local.y << 16);
