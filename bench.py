@@ -23,7 +23,9 @@ arrays, steps, and reads it back into them (one dem_step_exchange call per
 step, through GlobalData.state_buffers).  `roofline` reports the dominant
 kernel from per-phase CUDA events (dem_step_profiled) over the same window,
 against its algorithmic bytes (every field once per unit; re-reads from L2
-are `gather_bytes`).  `cpu_baseline` times the CPU oracle (OpenMP, all host
+are `gather_bytes`); a scene whose step is one launch (k_steps) has that
+launch's figures under `roofline.step`, and its phases are of the separate
+kernels.  `cpu_baseline` times the CPU oracle (OpenMP, all host
 threads) from the window's first state.  The clock sampler polls every 20 ms;
 a window shorter than five samples is followed by untimed steps of the same
 load until five are in (`clocks.padding_steps`).
@@ -138,12 +140,14 @@ def kernels_per_step(n: int, arena: bool = False) -> int:
 # 1.334e7 per launch), per bond 104.0 (a cracked lattice of 17,576, 40,535 bonds
 # and 5,101 Hertz contacts: 4.879e6 per launch, less the Hertz share); FP32
 # mode per bond 15.0 (64 batched scenes, 652,624 bonds: 9.789e6), per Hertz
-# contact 13.0 (the bed: 1.334e6).  Integrator per particle: 95.1 in FP64 mode
+# contact 16.0 (a bed of 400,000, 398,236 contacts: 6.372e6 in a step that
+# reports, as each timed one-step call does; 13.0 without the contact point).
+# Integrator per particle: 95.1 in FP64 mode
 # (the cracked lattice, split over four warps per 32 particles, with the
 # quaternions: 1.672e6 per launch), 32.1 in the FP32 mode (the 64 scenes, with
 # the quaternions: 1.188e7).  Then GB300's FP64 pipe width.
 FP64_INST = {("force", "fp64", "bond"): 104.0, ("force", "fp64", "hertz"): 130.0,
-             ("force", "fp32", "bond"): 15.0, ("force", "fp32", "hertz"): 13.0,
+             ("force", "fp32", "bond"): 15.0, ("force", "fp32", "hertz"): 16.0,
              ("integrate", "fp64"): 95.1, ("integrate", "fp32"): 32.1}
 # The integrator leaves out the components without a force, the spin update of
 # a particle with exactly zero torque and the orientation of one that does not
@@ -210,6 +214,25 @@ NCU_TRAFFIC = {
     ("c4", "integrate"): (99.5e6, 369893),         # k_integrate3<1>
     ("c4", "contacts"): (20.3e6, 369893),          # k_search<0, 1>, list step
 }
+
+
+# The same of one whole step in k_steps (a scene of up to 256 particles per SM)
+# at the first step of each timed window, L2 flushed before it, with its
+# FP64-pipe thread instructions (sm__thread_inst_executed_pipe_fp64_pred_on.sum)
+NCU_STEP = {"c1": (0.803e6, 0.3914e6), "c2": (12.49e6, 7.938e6)}
+
+
+def step_roofline(workload: str, alg: dict, ms: float, sm_mhz: float, peak_gbs: float) -> dict:
+    """The roofline of a whole step in one launch: the bytes of its phases and,
+    where counted, its FP64 instructions over the timed step."""
+    traffic, inst = NCU_STEP.get(workload, (None, None))
+    total = sum(alg.values())
+    out = {"kernel": "k_steps", "ms": ms, "algorithmic_bytes": total, "traffic": traffic,
+           "achieved_gbs": total / (ms * 1e-3) / 1e9}
+    out["frac_hbm"] = out["achieved_gbs"] / peak_gbs
+    if inst:
+        out["fp64_frac"] = inst / (ms * 1e-3) / (FP64_LANES_PER_SM * SM_COUNT * sm_mhz * 1e6)
+    return out
 
 
 def ncu_traffic(workload: str, kernel: str, n: int):
@@ -825,6 +848,10 @@ def measure_scene(args, lib, sc, precision: str, steps: int, warmup: int, advanc
                        "c3" if settling else None, n_hertz=int(round(c_mean - b_mean)))
     if fr:
         roof["fp64_pipe"] = fr
+    if kernels_per_step(sc.n) == 1:  # the timed steps are one launch each; the phases are not
+        roof["step"] = step_roofline(traffic_key, alg, ms_per_step, clk.get("sm_mhz") or 2070.0,
+                                     peaks["hbm_gbs"])
+        roof["phases_of"] = "the separate kernels (dem_step_profiled), not of the timed step"
     # every phase's figures (the phases of a step are close in length, so the
     # dominant one alone does not describe the step)
     roof["phases"] = {}
